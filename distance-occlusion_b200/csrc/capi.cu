@@ -146,6 +146,23 @@ dol_status get_workspace(Workspace& ws, void* user, size_t user_bytes, size_t ne
     return DOL_OK;
 }
 
+// The same with a size that is enough (`least`) below the size asked for
+// (`need`): a caller's workspace or the cap on the library's own may lie in
+// between.  *bytes: what there is.
+dol_status get_workspace_between(Workspace& ws, void* user, size_t user_bytes, size_t need, size_t least,
+                                 size_t* bytes, cudaStream_t st)
+{
+    size_t want = need;
+    if (user) {
+        if (user_bytes < need) want = least;
+    } else {
+        const size_t cap = g_workspace_limit.load(std::memory_order_relaxed);
+        if (cap && need > cap) want = least;
+    }
+    *bytes = want;
+    return get_workspace(ws, user, user_bytes, want, st);
+}
+
 inline cudaStream_t S(void* s) { return static_cast<cudaStream_t>(s); }
 
 // widest row the single-CTA sweeps handle (8 cells per thread, 512 threads),
@@ -575,8 +592,10 @@ static dol_status edt_common(int dim, int w, int h, int d, const uint32_t* mask,
     DOL_TRY(check_dev_ptr(mask, "mask"));
     DOL_TRY(check_dev_ptr(out, "out"));
     Workspace ws;
-    DOL_TRY(get_workspace(ws, workspace, workspace_bytes, edt_workspace_bytes(dim, w, h, d), S(stream)));
-    launch_edt_mask(dim, mask, out, w, h, d, form, ws.ptr, ds->err_dev, S(stream));
+    size_t got;
+    DOL_TRY(get_workspace_between(ws, workspace, workspace_bytes, edt_workspace_bytes(dim, w, h, d),
+                                  edt_workspace_bytes_min(dim, w, h, d), &got, S(stream)));
+    launch_edt_mask(dim, mask, out, w, h, d, form, ws.ptr, got, ds->err_dev, S(stream));
     return launched("edt_mask");
 }
 
@@ -745,12 +764,15 @@ static dol_status sdf_common(int dim, int w, int h, int d, const uint32_t* mask,
         return fail(DOL_ERR_UNSUPPORTED, "JumpFlood volumes are limited to 65535 slices");
     cudaStream_t st = S(stream);
     Workspace ws;
-    DOL_TRY(get_workspace(ws, workspace, workspace_bytes, dol_sdf_workspace_size(w, h, dim == 3 ? d : 1, method), st));
-
     if (method == DOL_FELZENSZWALB) {
-        launch_edt_mask(dim, mask, dist, w, h, d, DOL_EDT_SIGNED, ws.ptr, ds->err_dev, st);
+        const int ed = d > 1 ? dim : 2;   // a one-slice volume is an image, as dol_sdf_workspace_size counts it
+        size_t got;
+        DOL_TRY(get_workspace_between(ws, workspace, workspace_bytes, edt_workspace_bytes(ed, w, h, d),
+                                      edt_workspace_bytes_min(ed, w, h, d), &got, st));
+        launch_edt_mask(ed, mask, dist, w, h, d, DOL_EDT_SIGNED, ws.ptr, got, ds->err_dev, st);
         return launched("sdf (felzenszwalb)");
     }
+    DOL_TRY(get_workspace(ws, workspace, workspace_bytes, dol_sdf_workspace_size(w, h, dim == 3 ? d : 1, method), st));
     const size_t cells = (size_t)w * h * (dim == 3 ? d : 1);
     const size_t cb = dim == 3 ? sizeof(dol_delta3) : sizeof(dol_delta2);
     char* p = static_cast<char*>(ws.ptr);
@@ -1221,7 +1243,7 @@ dol_status dol_edt_mask_3d_host(int w, int h, int d, const uint32_t* mask, float
     const int slabs = d >= 2 * kHostSlabs ? kHostSlabs : 1;
     const int chunks = h >= 8 * kHostChunks ? kHostChunks : (h >= 64 ? 8 : 1);
     launch_edt_mask_3d_chunked(static_cast<uint32_t*>(dm.p), static_cast<float*>(df.p), w, h, d, form, dw.p,
-                               ds->err_dev, os.st, slabs, slab_ready, chunks, chunk_done, &hc);
+                               edt_workspace_bytes(3, w, h, d), ds->err_dev, os.st, slabs, slab_ready, chunks, chunk_done, &hc);
     const cudaError_t le = cudaGetLastError();
     // the copies back must finish before the device buffers are released (the
     // DevBuf destructors free on the compute stream)

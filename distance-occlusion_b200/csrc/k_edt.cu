@@ -105,8 +105,15 @@ __device__ __forceinline__ void store_half(uint16_t* o, const uint32_t pk[8], bo
     }
 }
 
+// Rows of the x-pass field are padded to whole 16-byte units (8 cells), so that
+// every width takes the vector stores here and the TMA line passes: unpadded,
+// a width that is no multiple of 8 went to the plain line kernel (1501 x 1013
+// signed: y pass 582 us there).  The padding cells hold 0 (a clear cell at
+// distance 0: its walk ends at once).
+static inline int padded_pitch(int w) { return (w + 7) & ~7; }
+
 __global__ void __launch_bounds__(256) k_edt_x(const uint32_t* __restrict__ mask, uint16_t* __restrict__ out, int w,
-                                               long long rows)
+                                               int pitch, long long rows)
 {
     __shared__ int right_carry[8][kMaxChunks][2];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -115,7 +122,7 @@ __global__ void __launch_bounds__(256) k_edt_x(const uint32_t* __restrict__ mask
     const int seg = lane / SW, sl = lane % SW, rpw = 32 / SW;
     const int nchunks = (ws + 31) >> 5;
     const int NEG = -(1 << 30), POS = 1 << 30;
-    const bool vec_ok = (w & 7) == 0;   // 16-byte aligned word outputs
+    const bool vec_ok = (pitch & 7) == 0 && ((uintptr_t)out & 15) == 0;   // 16-byte aligned word outputs
     long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
 
@@ -123,7 +130,7 @@ __global__ void __launch_bounds__(256) k_edt_x(const uint32_t* __restrict__ mask
         const long long row = row0 + seg;
         const bool rowok = row < rows;
         const uint32_t* mrow = mask + (rowok ? row : 0) * ws;
-        uint16_t* orow = out + (rowok ? row : 0) * (long long)w;
+        uint16_t* orow = out + (rowok ? row : 0) * (long long)pitch;
 
         // long rows: first clear / set cell right of each chunk (segments are whole warps here)
         if (nchunks > 1) {
@@ -201,6 +208,7 @@ __global__ void __launch_bounds__(256) k_edt_x(const uint32_t* __restrict__ mask
             store_half(o + 16, pk, whole, nlive - 16);
             x_half<0>(me, tl, tr, xb, carry_l, runB, pk);
             store_half(o, pk, whole, nlive);
+            for (int t = nlive; t < 32 && xb + t < pitch; t++) o[t] = 0;
         }
     }
 }
@@ -362,27 +370,33 @@ __device__ __forceinline__ void put_walk_value(void* out, long long o, uint32_t 
 
 // Plain-load form: 32 adjacent x per CTA, the line staged in shared memory when
 // it fits (kStaged) or read from global memory otherwise.
+// in: position stride and outer stride of the input; out likewise.
+struct LineStrides {
+    long long in, in_outer, out, out_outer;
+};
+
 template <typename TIn, bool kFinal, bool kStaged>
 __global__ void __launch_bounds__(256) k_edt_line(const TIn* __restrict__ in, void* __restrict__ out, int w, int n,
-                                                  long long stride, long long outer_stride, int form, int outer0)
+                                                  LineStrides ls, int form, int outer0)
 {
     extern __shared__ unsigned char smem_raw[];
     TIn* tile = reinterpret_cast<TIn*>(smem_raw);   // [n][32]
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int x = blockIdx.x * 32 + lane;
-    const long long base = (long long)(blockIdx.y + outer0) * outer_stride + x;
+    const long long base = (long long)(blockIdx.y + outer0) * ls.in_outer + x;
+    const long long obase = (long long)(blockIdx.y + outer0) * ls.out_outer + x;
     const bool live = x < w;
 
     if (kStaged) {
-        for (int q = wib; q < n; q += nw) tile[q * 32 + lane] = live ? in[base + q * stride] : (TIn)0;
+        for (int q = wib; q < n; q += nw) tile[q * 32 + lane] = live ? in[base + q * ls.in] : (TIn)0;
         __syncthreads();
     }
-    auto at = [&](int q) -> TIn { return kStaged ? tile[q * 32 + lane] : in[base + q * stride]; };
+    auto at = [&](int q) -> TIn { return kStaged ? tile[q * 32 + lane] : in[base + q * ls.in]; };
     for (int q = wib; q < n; q += nw) {
         if (!live) continue;
         uint32_t s;
         uint32_t best = search_line<TIn>(at, q, n, &s);
-        put_line_value<kFinal>(out, base + q * stride, s, best, form);
+        put_line_value<kFinal>(out, obase + q * ls.out, s, best, form);
     }
 }
 
@@ -612,7 +626,7 @@ __global__ void __launch_bounds__(512) k_edt_line_tma(const __grid_constant__ CU
     int x0, outer, line = 0;
     if (kMode == 2) {
         // one block per (y, 8-column group) of the [y][x/8][z][8] array
-        const int wb = w >> 3;
+        const int wb = (w + 7) >> 3;
         line = blockIdx.x + outer0 * wb;
         outer = line / wb;
         x0 = (line - outer * wb) * 8;
@@ -694,11 +708,17 @@ __global__ void __launch_bounds__(512) k_edt_line_tma(const __grid_constant__ CU
     const uint32_t n_none = sizeof(TIn) == 2 ? s_score : (s_score & 0xFFFFu), n_far = s_score >> 16;
     const bool use_hull = hull_pct <= 100u && 100LL * n_none >= (long long)hull_pct * sampled;
 
+    // kMode 0: a tile whose grid leaves SMs idle is searched by gridDim.z CTAs,
+    // each taking every gridDim.z-th block of positions (all of them stage the
+    // tile); the other two paths run in the first
+    const int part = kMode == 0 ? blockIdx.z : 0, parts = kMode == 0 ? gridDim.z : 1;
     if (use_hull) {
+        if (part) return;
         edt_tile_envelope<TIn, kFinal, TX, kMode>(F0, F1, rows, n, w, x0, outer, out, stride, outer_stride, form);
         return;
     }
     if (sizeof(TIn) == 4 && far_pct <= 100u && 100LL * n_far >= (long long)far_pct * sampled) {
+        if (part) return;
         edt_tile_pruned<TIn, kFinal, TX, kMode>(F0, F1, rows, n, w, x0, outer, out, stride, outer_stride, form);
         return;
     }
@@ -711,14 +731,14 @@ __global__ void __launch_bounds__(512) k_edt_line_tma(const __grid_constant__ CU
     constexpr int kGroups = TX / 8;
     const int lane = threadIdx.x & 31, nw = blockDim.x >> 5, wi = threadIdx.x >> 5;
     const int col = (wi % kGroups) * 8 + (lane & 7), sub = lane >> 3;
-    const int qstep = 8 * (nw / kGroups);
+    const int qpart = 8 * (nw / kGroups), qstep = qpart * parts;
     const int x = x0 + col;
     if (x >= w) return;
     const long long base = kMode == 1 ? ((long long)(x >> 3) * outer_stride + outer) * 8 + (x & 7)
                                       : (long long)outer * outer_stride + x;
     // "no cell of the other state reachable": INF (0x7FFF) squared for u16 input, 0x7FFFFFFF for u32
     const uint32_t kNone = sizeof(TIn) == 2 ? kInf16 * kInf16 : kInf32;
-    const int q0 = 8 * (wi / kGroups) + sub;
+    const int q0 = 8 * (wi / kGroups) + sub + part * qpart;
     long long o = base + (long long)q0 * stride;   // output index of the lane's first cell
     const long long ostep = (long long)qstep * stride, o4 = 4 * stride;
     for (int qa = q0; qa < n; qa += qstep, o += ostep) {
@@ -783,12 +803,13 @@ __global__ void __launch_bounds__(512) k_edt_line_tma(const __grid_constant__ CU
 }
 
 constexpr size_t kStageLimit = 200 * 1024;   // largest staged line tile of the plain form
+constexpr size_t kTileLimit = 200 * 1024;    // largest tile of the TMA form
 
 // set_attr = false: the caller raised the staged kernel's shared-memory limit
 // to kStageLimit beforehand (prepare_edt_mask_2d_plain)
 template <typename TIn, bool kFinal>
-static void line_pass_plain(const TIn* in, void* out, int w, int n, long long stride, long long outer,
-                            long long outer_stride, int form, cudaStream_t st, int outer0 = 0, bool set_attr = true)
+static void line_pass_plain(const TIn* in, void* out, int w, int n, long long outer, const LineStrides& ls, int form,
+                            cudaStream_t st, int outer0 = 0, bool set_attr = true)
 {
     size_t bytes = (size_t)n * 32 * sizeof(TIn);
     dim3 grid((w + 31) / 32, (unsigned)outer);
@@ -796,9 +817,9 @@ static void line_pass_plain(const TIn* in, void* out, int w, int n, long long st
         auto kern = k_edt_line<TIn, kFinal, true>;
         if (set_attr && bytes > 48 * 1024)
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        kern<<<grid, 256, bytes, st>>>(in, out, w, n, stride, outer_stride, form, outer0);
+        kern<<<grid, 256, bytes, st>>>(in, out, w, n, ls, form, outer0);
     } else {
-        k_edt_line<TIn, kFinal, false><<<grid, 256, 0, st>>>(in, out, w, n, stride, outer_stride, form, outer0);
+        k_edt_line<TIn, kFinal, false><<<grid, 256, 0, st>>>(in, out, w, n, ls, form, outer0);
     }
 }
 
@@ -827,15 +848,15 @@ static bool line_map(CUtensorMap* map, const TIn* in, int w, int h, int d, int a
 }
 
 // True when a volume's y pass can write, and its z pass read, the
-// [y][x/8][z][8] array: 8 | w, both line tiles fit, both maps encode.
-static bool blocked_layout_ok(const uint16_t* vx, const uint32_t* ey, int w, int h, int d)
+// [y][pitch/8][z][8] array: 8 | pitch, both line tiles fit, both maps encode.
+static bool blocked_layout_ok(const uint16_t* vx, const uint32_t* ey, int pitch, int h, int d)
 {
-    if (w % 8 != 0 || d > 65535) return false;
-    if (tma_tile_bytes<uint16_t, 16>(h) > 200 * 1024 || tma_tile_bytes<uint32_t, 8>(d) > 200 * 1024) return false;
-    if ((long long)(w / 8) * h > 0x7FFFFFFFLL) return false;
+    if (pitch % 8 != 0 || d > 65535) return false;
+    if (tma_tile_bytes<uint16_t, 16>(h) > kTileLimit || tma_tile_bytes<uint32_t, 8>(d) > kTileLimit) return false;
+    if ((long long)(pitch / 8) * h > 0x7FFFFFFFLL) return false;
     if (((uintptr_t)vx % 16) != 0 || ((uintptr_t)ey % 16) != 0) return false;
     CUtensorMap m;
-    return line_map<uint16_t, 16>(&m, vx, w, h, d, 0, 1) && line_map<uint32_t, 8>(&m, ey, w, h, d, 1, 2);
+    return line_map<uint16_t, 16>(&m, vx, pitch, h, d, 0, 1) && line_map<uint32_t, 8>(&m, ey, pitch, h, d, 1, 2);
 }
 
 // Share of "none" cells (percent) at which a line-pass tile takes the
@@ -864,63 +885,87 @@ static uint32_t edt_far_share(int n)
     return 50u;
 }
 
+// One launch of the TMA form with TX columns per tile
+template <typename TIn, bool kFinal, int TX, int kMode>
+static void launch_line_tma(const CUtensorMap& map, void* out, int w, int n, long long stride, long long outer_stride,
+                            int along_z, int form, int* err, dim3 grid, int threads, int outer0, cudaStream_t st)
+{
+    auto kern = k_edt_line_tma<TIn, kFinal, TX, kMode>;
+    const size_t tile_bytes = tma_tile_bytes<TIn, TX>(n);
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_bytes);
+    cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    kern<<<grid, threads, tile_bytes, st>>>(map, out, w, n, stride, outer_stride, along_z, form, err, outer0,
+                                            edt_hull_share(n), edt_far_share(n));
+}
+
 // Lines along y (along_z = 0, outer index = z) or z (along_z = 1, outer = y)
-// of a w x h x d array; outer indices outer0 .. outer0 + nouter - 1 (nouter < 0:
-// all).  TMA needs 16-byte row pitches and a tile that fits in shared memory;
+// of a w x h x d array whose input rows are `pitch` cells apart (w, or w
+// rounded up to 8; intermediate outputs have the same pitch, the final field
+// is packed); outer indices outer0 .. outer0 + nouter - 1 (nouter < 0: all).
+// TMA needs 16-byte row pitches and a tile that fits in shared memory;
 // otherwise the plain form runs.  mode 1 / 2 (blocked y-pass output / z-pass
 // input) only after blocked_layout_ok.
 template <typename TIn, bool kFinal>
-static void line_pass(const TIn* in, void* out, int w, int h, int d, int along_z, int form, int* err, cudaStream_t st,
-                      int outer0 = 0, int nouter = -1, int mode = 0)
+static void line_pass(const TIn* in, void* out, int w, int pitch, int h, int d, int along_z, int form, int* err,
+                      cudaStream_t st, int outer0 = 0, int nouter = -1, int mode = 0)
 {
     const int n = along_z ? d : h;
-    const long long plane = (long long)w * h;
-    const long long stride = along_z ? plane : w;
+    const int wo = kFinal ? w : pitch;   // an intermediate field is written whole, padding included
+    const long long in_plane = (long long)pitch * h, out_plane = (long long)wo * h;
+    const long long stride = along_z ? out_plane : wo;
     const long long outer = nouter >= 0 ? nouter : (along_z ? h : d);
-    const long long outer_stride = along_z ? w : plane;
+    const long long outer_stride = along_z ? wo : out_plane;
     constexpr int TX = sizeof(TIn) == 2 ? 16 : 8;   // 32-byte box rows either way
-    const size_t tile_bytes = tma_tile_bytes<TIn, TX>(n);
-    const bool aligned = ((size_t)w * sizeof(TIn)) % 16 == 0 && ((uintptr_t)in % 16) == 0;
+    const bool aligned = ((size_t)pitch * sizeof(TIn)) % 16 == 0 && ((uintptr_t)in % 16) == 0;
     const int tv = tune_get(kTuneEdt, w);
     const int threads = tv == 256 ? 256 : 512;
-    const uint32_t hthr = edt_hull_share(n), fthr = edt_far_share(n);
     CUtensorMap map;
     if (mode == 1) {
-        if (!line_map<TIn, TX>(&map, in, w, h, d, along_z, 0)) return;   // blocked_layout_ok encoded it already
-        auto kern = k_edt_line_tma<TIn, kFinal, TX, 1>;
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_bytes);
-        cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        dim3 grid((w + TX - 1) / TX, (unsigned)outer);
-        kern<<<grid, threads, tile_bytes, st>>>(map, out, w, n, (long long)w * d, d, along_z, form, err, outer0, hthr,
-                                                fthr);
+        if (!line_map<TIn, TX>(&map, in, pitch, h, d, along_z, 0)) return;   // blocked_layout_ok encoded it already
+        const dim3 grid((pitch + TX - 1) / TX, (unsigned)outer);
+        launch_line_tma<TIn, kFinal, TX, 1>(map, out, pitch, n, (long long)pitch * d, d, along_z, form, err, grid,
+                                            threads, outer0, st);
         return;
     }
     if (mode == 2) {
-        if (!line_map<TIn, TX>(&map, in, w, h, d, along_z, 2)) {
+        if (!line_map<TIn, TX>(&map, in, pitch, h, d, along_z, 2)) {
             // blocked_layout_ok encoded this map; should the driver refuse it
             // now, the call reports failure rather than leave the field unwritten
             k_flag_error<<<1, 1, 0, st>>>(err);
             return;
         }
-        auto kern = k_edt_line_tma<TIn, kFinal, 8, 2>;
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_bytes);
-        cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        const unsigned blocks = (unsigned)(outer * (w / 8));
-        kern<<<blocks, threads, tile_bytes, st>>>(map, out, w, n, plane, w, along_z, form, err, outer0, hthr, fthr);
+        const unsigned blocks = (unsigned)(outer * (pitch / 8));
+        launch_line_tma<TIn, kFinal, 8, 2>(map, out, w, n, out_plane, w, along_z, form, err, dim3(blocks), threads,
+                                           outer0, st);
         return;
     }
-    if (aligned && tile_bytes <= 200 * 1024 && outer <= 65535) {
-        if (line_map<TIn, TX>(&map, in, w, h, d, along_z, 0)) {
-            auto kern = k_edt_line_tma<TIn, kFinal, TX, 0>;
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_bytes);
-        cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-            dim3 grid((w + TX - 1) / TX, (unsigned)outer);
-            kern<<<grid, threads, tile_bytes, st>>>(map, out, w, n, stride, outer_stride, along_z, form, err, outer0,
-                                                    hthr, fthr);
-            return;
+    if (aligned && outer <= 65535) {
+        // grid.z CTAs search one tile while the tiles alone would leave SMs
+        // idle (an image: w / 16 tiles), each at least 64 positions
+        auto parts = [&](int tx) {
+            const long long tiles = (long long)((wo + tx - 1) / tx) * outer;
+            const long long want = (3LL * g_num_sms + tiles - 1) / tiles;
+            return (unsigned)max(1LL, min(want, (long long)(n + 63) / 64));
+        };
+        if (tma_tile_bytes<TIn, TX>(n) <= kTileLimit) {
+            if (line_map<TIn, TX>(&map, in, pitch, h, d, along_z, 0)) {
+                const dim3 grid((wo + TX - 1) / TX, (unsigned)outer, parts(TX));
+                launch_line_tma<TIn, kFinal, TX, 0>(map, out, wo, n, stride, outer_stride, along_z, form, err, grid,
+                                                    threads, outer0, st);
+                return;
+            }
+        } else if constexpr (sizeof(TIn) == 2) {
+            // lines too long for 16 columns: 8 columns (16-byte box rows)
+            if (tma_tile_bytes<TIn, 8>(n) <= kTileLimit && line_map<TIn, 8>(&map, in, pitch, h, d, along_z, 0)) {
+                const dim3 grid((wo + 7) / 8, (unsigned)outer, parts(8));
+                launch_line_tma<TIn, kFinal, 8, 0>(map, out, wo, n, stride, outer_stride, along_z, form, err, grid,
+                                                   threads, outer0, st);
+                return;
+            }
         }
     }
-    line_pass_plain<TIn, kFinal>(in, out, w, n, stride, outer, outer_stride, form, st, outer0);
+    const LineStrides ls{along_z ? in_plane : pitch, along_z ? pitch : in_plane, stride, outer_stride};
+    line_pass_plain<TIn, kFinal>(in, out, wo, n, outer, ls, form, st, outer0);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -948,40 +993,54 @@ bool encode_map_3d(CUtensorMap* map, const void* base, CUtensorMapDataType type,
     return r == CUDA_SUCCESS;
 }
 
-size_t edt_workspace_bytes(int dim, int w, int h, int d)
+// scratch of the mask EDT with rows `pitch` cells apart
+static size_t edt_bytes(int dim, int pitch, int h, int d)
 {
-    size_t cells = (size_t)w * h * (dim == 3 ? d : 1);
+    size_t cells = (size_t)pitch * h * (dim == 3 ? d : 1);
     size_t b = cells * sizeof(uint16_t);
     b = (b + 255) & ~(size_t)255;
     if (dim == 3) b += cells * sizeof(uint32_t);
     return b;
 }
 
-void launch_edt_mask(int dim, const uint32_t* mask, float* out, int w, int h, int d, int form, void* ws, int* err,
-                     cudaStream_t st)
+size_t edt_workspace_bytes(int dim, int w, int h, int d) { return edt_bytes(dim, padded_pitch(w), h, d); }
+size_t edt_workspace_bytes_min(int dim, int w, int h, int d) { return edt_bytes(dim, w, h, d); }
+
+// padded rows whenever the scratch holds them
+static int edt_pitch(int dim, int w, int h, int d, size_t ws_bytes)
+{
+    return ws_bytes >= edt_workspace_bytes(dim, w, h, d) ? padded_pitch(w) : w;
+}
+
+static void run_edt_x(const uint32_t* mask, uint16_t* vx, int w, int pitch, long long rows, int sms, cudaStream_t st)
+{
+    const long long blocks = (rows * 32 + 255) / 256, cap = (long long)sms * 16;
+    k_edt_x<<<(int)(blocks < cap ? blocks : cap), 256, 0, st>>>(mask, vx, w, pitch, rows);
+}
+
+void launch_edt_mask(int dim, const uint32_t* mask, float* out, int w, int h, int d, int form, void* ws,
+                     size_t ws_bytes, int* err, cudaStream_t st)
 {
     long long rows = (long long)h * (dim == 3 ? d : 1);
-    size_t cells = (size_t)w * rows;
+    const int pitch = edt_pitch(dim, w, h, d, ws_bytes);
     uint16_t* vx = static_cast<uint16_t*>(ws);
-    long long blocks = (rows * 32 + 255) / 256;
-    long long cap = (long long)g_num_sms * 16;
     {
         ProfScope ps("edt_x", st);
-        k_edt_x<<<(int)(blocks < cap ? blocks : cap), 256, 0, st>>>(mask, vx, w, rows);
+        run_edt_x(mask, vx, w, pitch, rows, g_num_sms, st);
     }
     if (dim == 2) {
         ProfScope ps("edt_y_final", st);
-        line_pass<uint16_t, true>(vx, out, w, h, 1, 0, form, err, st);
+        line_pass<uint16_t, true>(vx, out, w, pitch, h, 1, 0, form, err, st);
     } else {
-        size_t off = (cells * sizeof(uint16_t) + 255) & ~(size_t)255;
+        const size_t off = edt_bytes(2, pitch, h * d, 1);
         uint32_t* ey = reinterpret_cast<uint32_t*>(static_cast<char*>(ws) + off);
-        const bool blk = blocked_layout_ok(vx, ey, w, h, d);
+        const bool blk = blocked_layout_ok(vx, ey, pitch, h, d);
         {
             ProfScope ps("edt_y", st);
-            line_pass<uint16_t, false>(vx, ey, w, h, d, 0, form, err, st, 0, -1, blk ? 1 : 0);   // y lines
+            line_pass<uint16_t, false>(vx, ey, w, pitch, h, d, 0, form, err, st, 0, -1, blk ? 1 : 0);   // y lines
         }
         ProfScope ps("edt_z_final", st);
-        line_pass<uint32_t, true>(ey, out, w, h, d, 1, form, err, st, 0, -1, blk ? 2 : 0);   // z lines
+        line_pass<uint32_t, true>(ey, out, w, pitch, h, d, 1, form, err, st, 0, -1, blk ? 2 : 0);   // z lines
     }
 }
 
@@ -991,32 +1050,30 @@ void launch_edt_mask(int dim, const uint32_t* mask, float* out, int w, int h, in
 // last (z) pass over `chunks` ranges of y, each followed by `done(ctx, y0, y1)`
 // (the caller queues work on rows y0..y1-1 of every slice, e.g. their copy
 // back to the host).  Both hooks run on the host after / before the launches.
-void launch_edt_mask_3d_chunked(const uint32_t* mask, float* out, int w, int h, int d, int form, void* ws, int* err,
-                                cudaStream_t st, int slabs, void (*ready)(void*, int, int), int chunks,
-                                void (*done)(void*, int, int), void* ctx)
+void launch_edt_mask_3d_chunked(const uint32_t* mask, float* out, int w, int h, int d, int form, void* ws,
+                                size_t ws_bytes, int* err, cudaStream_t st, int slabs, void (*ready)(void*, int, int),
+                                int chunks, void (*done)(void*, int, int), void* ctx)
 {
-    const size_t cells = (size_t)w * h * d;
+    const int pitch = edt_pitch(3, w, h, d, ws_bytes);
     const int words = words_per_row(w);
     uint16_t* vx = static_cast<uint16_t*>(ws);
-    const size_t off = (cells * sizeof(uint16_t) + 255) & ~(size_t)255;
+    const size_t off = edt_bytes(2, pitch, h * d, 1);
     uint32_t* ey = reinterpret_cast<uint32_t*>(static_cast<char*>(ws) + off);
-    const bool blk = blocked_layout_ok(vx, ey, w, h, d);
+    const bool blk = blocked_layout_ok(vx, ey, pitch, h, d);
     slabs = slabs < 1 ? 1 : (slabs > d ? d : slabs);
     for (int s = 0; s < slabs; s++) {
         const int z0 = (int)((long long)d * s / slabs), z1 = (int)((long long)d * (s + 1) / slabs);
         if (z1 <= z0) continue;
         if (ready) ready(ctx, z0, z1);
-        const long long rows = (long long)(z1 - z0) * h;
-        const long long blocks = (rows * 32 + 255) / 256, cap = (long long)g_num_sms * 16;
-        k_edt_x<<<(int)(blocks < cap ? blocks : cap), 256, 0, st>>>(mask + (size_t)z0 * h * words,
-                                                                    vx + (size_t)z0 * h * w, w, rows);
-        line_pass<uint16_t, false>(vx, ey, w, h, d, 0, form, err, st, z0, z1 - z0, blk ? 1 : 0);
+        run_edt_x(mask + (size_t)z0 * h * words, vx + (size_t)z0 * h * pitch, w, pitch, (long long)(z1 - z0) * h,
+                  g_num_sms, st);
+        line_pass<uint16_t, false>(vx, ey, w, pitch, h, d, 0, form, err, st, z0, z1 - z0, blk ? 1 : 0);
     }
     chunks = chunks < 1 ? 1 : (chunks > h ? h : chunks);
     for (int c = 0; c < chunks; c++) {
         const int y0 = (int)((long long)h * c / chunks), y1 = (int)((long long)h * (c + 1) / chunks);
         if (y1 <= y0) continue;
-        line_pass<uint32_t, true>(ey, out, w, h, d, 1, form, err, st, y0, y1 - y0, blk ? 2 : 0);
+        line_pass<uint32_t, true>(ey, out, w, pitch, h, d, 1, form, err, st, y0, y1 - y0, blk ? 2 : 0);
         if (done) done(ctx, y0, y1);
     }
 }
@@ -1027,93 +1084,14 @@ void launch_edt_mask_3d_chunked(const uint32_t* mask, float* out, int w, int h, 
 void launch_edt_mask_2d_plain(const uint32_t* mask, float* out, int w, int h, int form, uint16_t* scratch, int sms,
                               cudaStream_t st)
 {
-    long long blocks = ((long long)h * 32 + 255) / 256;
-    long long cap = (long long)sms * 16;
-    k_edt_x<<<(int)(blocks < cap ? blocks : cap), 256, 0, st>>>(mask, scratch, w, h);
-    line_pass_plain<uint16_t, true>(scratch, out, w, h, w, 1, 0, form, st, 0, false);
+    run_edt_x(mask, scratch, w, w, h, sms, st);   // rows unpadded: the scratch holds w * h cells
+    line_pass_plain<uint16_t, true>(scratch, out, w, h, 1, LineStrides{w, 0, w, 0}, form, st, 0, false);
 }
 
 cudaError_t prepare_edt_mask_2d_plain()
 {
     return cudaFuncSetAttribute(k_edt_line<uint16_t, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)kStageLimit);
-}
-
-// ------------------------------------------------ faithful float Felzenszwalb ----
-// DOL::Felzenszwalb(w, h, float[]) on arbitrary input: the same 1D lower
-// envelope in the same float operations (DistanceOcclusionLib.cpp:1026-1062),
-// one thread per line.  Column pass into a scratch field, then row pass back.
-// Envelope stacks live in the workspace, interleaved by line for coalescing.
-
-__device__ void felz_line_dev(int n, const float* f, long long fstride, float* out, long long ostride, int* v, float* z,
-                              long long sstride)
-{
-    int k = 0;
-    v[0] = 0;
-    z[0] = -FLT_MAX;
-    z[sstride] = FLT_MAX;
-    for (int q = 1; q < n; q++) {
-        float hq = f[q * fstride] + (float)(q * q);
-        float s;
-        for (;;) {
-            int p = v[k * sstride];
-            float hp = f[p * fstride] + (float)(p * p);
-            s = __fdiv_rn(hq - hp, (float)(2 * (q - p)));
-            if (s > z[k * sstride]) break;
-            k--;
-        }
-        k++;
-        v[k * sstride] = q;
-        z[k * sstride] = s;
-        z[(k + 1) * sstride] = FLT_MAX;
-    }
-    k = 0;
-    for (int q = 0; q < n; q++) {
-        while (z[(k + 1) * sstride] < (float)q) k++;
-        int p = v[k * sstride];
-        out[q * ostride] = __fadd_rn((float)((q - p) * (q - p)), f[p * fstride]);
-    }
-}
-
-__global__ void k_felz_cols(const float* __restrict__ in, float* __restrict__ td, int w, int h, int* v, float* z)
-{
-    int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= w) return;
-    // column x (stride w) -> td[x*h + q] (the reference's transposed scratch)
-    felz_line_dev(h, in + x, w, td + (long long)x * h, 1, v + x, z + x, w);
-}
-
-__global__ void k_felz_rows(const float* __restrict__ td, float* __restrict__ out, int w, int h, int* v, float* z)
-{
-    int y = blockIdx.x * blockDim.x + threadIdx.x;
-    if (y >= h) return;
-    felz_line_dev(w, td + y, h, out + (long long)y * w, 1, v + y, z + y, h);
-}
-
-size_t felz_float_workspace_bytes(int w, int h)
-{
-    size_t n = (size_t)(w > h ? w : h);
-    size_t lines = (size_t)(w > h ? w : h);
-    size_t td = ((size_t)w * h * sizeof(float) + 255) & ~(size_t)255;
-    size_t vb = (n * lines * sizeof(int) + 255) & ~(size_t)255;
-    size_t zb = (n + 1) * lines * sizeof(float);
-    return td + vb + zb;
-}
-
-void launch_felz_float_2d(float* dist, int w, int h, void* ws, cudaStream_t st)
-{
-    size_t n = (size_t)(w > h ? w : h);
-    size_t lines = n;
-    char* p = static_cast<char*>(ws);
-    float* td = reinterpret_cast<float*>(p);
-    p += ((size_t)w * h * sizeof(float) + 255) & ~(size_t)255;
-    int* v = reinterpret_cast<int*>(p);
-    p += (n * lines * sizeof(int) + 255) & ~(size_t)255;
-    float* z = reinterpret_cast<float*>(p);
-    (void)lines;
-    // stacks are indexed [position * lines_in_pass + line]; each pass uses its own line count as the stride
-    k_felz_cols<<<(w + 127) / 128, 128, 0, st>>>(dist, td, w, h, v, z);
-    k_felz_rows<<<(h + 127) / 128, 128, 0, st>>>(td, dist, w, h, v, z);
 }
 
 }  // namespace dolk

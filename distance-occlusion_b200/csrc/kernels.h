@@ -74,17 +74,20 @@ void launch_init_deltas(int dim, const uint32_t* mask, void* deltas, int w, long
 void launch_init_border(int dim, const uint32_t* mask, void* deltas, int w, int h, int d, cudaStream_t st);
 
 // k_edt.cu -- mask-driven exact EDT
+// rows padded to 8 cells; the _min form (rows packed, slower for widths that
+// are no multiple of 8) is enough to run
 size_t edt_workspace_bytes(int dim, int w, int h, int d);
-void launch_edt_mask(int dim, const uint32_t* mask, float* out, int w, int h, int d, int form, void* ws, int* err,
-                     cudaStream_t st);
-void launch_edt_mask_3d_chunked(const uint32_t* mask, float* out, int w, int h, int d, int form, void* ws, int* err,
-                                cudaStream_t st, int slabs, void (*ready)(void*, int, int), int chunks,
-                                void (*done)(void*, int, int), void* ctx);
+size_t edt_workspace_bytes_min(int dim, int w, int h, int d);
+void launch_edt_mask(int dim, const uint32_t* mask, float* out, int w, int h, int d, int form, void* ws,
+                     size_t ws_bytes, int* err, cudaStream_t st);
+void launch_edt_mask_3d_chunked(const uint32_t* mask, float* out, int w, int h, int d, int form, void* ws,
+                                size_t ws_bytes, int* err, cudaStream_t st, int slabs, void (*ready)(void*, int, int),
+                                int chunks, void (*done)(void*, int, int), void* ctx);
 void launch_edt_mask_2d_plain(const uint32_t* mask, float* out, int w, int h, int form, uint16_t* scratch, int sms,
                               cudaStream_t st);
 // the kernel attributes launch_edt_mask_2d_plain relies on (set once per device)
 cudaError_t prepare_edt_mask_2d_plain();
-// faithful float Felzenszwalb (2D, arbitrary input)
+// k_felz.cu -- faithful float Felzenszwalb (2D, arbitrary input)
 size_t felz_float_workspace_bytes(int w, int h);
 void launch_felz_float_2d(float* dist, int w, int h, void* ws, cudaStream_t st);
 
@@ -120,7 +123,7 @@ void launch_batch_sdf(const void* items, const int* order, int n, const uint32_t
                       int* counter, cudaStream_t st);
 void launch_fastsweep_3d(void* deltas, int w, int h, int d, int cw, void* ws, int* err, cudaStream_t st);
 
-// k_chamfer.cu -- Chamfer 3-4 on int16 / int32 fields (one CTA walks the rows)
+// k_chamfer.cu -- Chamfer 3-4 on int16 / int32 fields
 template <typename T>
 void launch_chamfer_2d(T* dist, int w, int h, cudaStream_t st);
 template <typename T>

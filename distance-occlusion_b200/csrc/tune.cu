@@ -273,6 +273,7 @@ DOL_API dol_status dol_autotune(int kind, int w, int h, int d, void* stream)
                 break;
             case kTuneEdt:
                 launch_edt_mask(3, static_cast<uint32_t*>(dm), static_cast<float*>(dl), tw, th, td, DOL_EDT_SIGNED, ws,
+                                ws_bytes,
                                 err, st);
                 break;
             case kTuneDanRows:
