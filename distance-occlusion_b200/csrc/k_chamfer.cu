@@ -15,14 +15,17 @@
 // (suffix min, right neighbour).
 //
 // A CTA walks a run of rows (each row needs the one before); a thread owns 4
-// consecutive cells, so rows of up to 4096 cells.  The previous row sits in
-// shared memory with "no value" sentinels at x = -1 and x = w; two barriers
-// per row (warp totals, the next row's neighbours).  Fields of 64 rows or more
-// run in blocks of 32 rows, all blocks at once (see below); smaller ones, or
+// consecutive cells, so rows of up to 4096 cells.  The previous row stays in
+// registers, its neighbours across threads come by shuffle, across warps from
+// the row's own scan, so a row costs one barrier.  Fields of 16 rows or more
+// run in blocks of 8 rows, all blocks at once (see below); smaller ones, or
 // when the small boundary scratch cannot be had, in one CTA.
+#include <limits.h>
+
 #include <type_traits>
 
 #include "common.cuh"
+#include "grid_barrier.cuh"
 #include "kernels.h"
 
 namespace dolk {
@@ -51,91 +54,126 @@ __device__ __forceinline__ K shfl_down_k(K v, int o)
     return __shfl_down_sync(0xFFFFFFFFu, v, o);
 }
 
-// Block-wide scan of the per-thread totals: for kFwd the min over all earlier
-// threads (exclusive prefix), else the min over all later threads (exclusive
-// suffix).  wtot: one slot per warp; one barrier.
-template <typename K, bool kFwd>
-__device__ __forceinline__ K block_excl_min(K tot, K* wtot, K inf)
+// The min over the lanes whose `on` holds
+__device__ __forceinline__ int warp_min_k(int v, bool on) { return __reduce_min_sync(0xFFFFFFFFu, on ? v : INT_MAX); }
+__device__ __forceinline__ long long warp_min_k(long long v, bool on)
 {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    long long m = on ? v : LLONG_MAX;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = min(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
+    return m;
+}
+
+// Inclusive scan of m over the thread's cells and the warp's lanes before it in
+// scan direction (kFwd: lower lanes); returns the exclusive part.
+template <typename K, bool kFwd>
+__device__ __forceinline__ K warp_excl_min(K tot, K inf, K* incl_out)
+{
+    const int lane = threadIdx.x & 31;
     K incl = tot;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const K v = kFwd ? shfl_up_k(incl, o) : shfl_down_k(incl, o);
         if (kFwd ? lane >= o : lane + o < 32) incl = min(incl, v);
     }
-    K excl = kFwd ? shfl_up_k(incl, 1) : shfl_down_k(incl, 1);
-    if (kFwd ? lane == 0 : lane == 31) excl = inf;
-    if (kFwd ? lane == 31 : lane == 0) wtot[wid] = incl;
-    __syncthreads();
-    // every warp scans the (at most 32) warp totals for itself
-    K wv = lane < nw ? wtot[lane] : inf;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const K v = kFwd ? shfl_up_k(wv, o) : shfl_down_k(wv, o);
-        if (kFwd ? lane >= o : lane + o < 32) wv = min(wv, v);
-    }
-    K wex = kFwd ? shfl_up_k(wv, 1) : shfl_down_k(wv, 1);
-    if (kFwd ? lane == 0 : lane == 31) wex = inf;
-    const K mine = __shfl_sync(0xFFFFFFFFu, wex, wid);
-    return min(excl, mine);
+    *incl_out = incl;
+    const K excl = kFwd ? shfl_up_k(incl, 1) : shfl_down_k(incl, 1);
+    return (kFwd ? lane == 0 : lane == 31) ? inf : excl;
 }
 
-// Rows ya, ya + dir, ..., yb of one pass (dir = +1 down, -1 up), the first of
-// them with no row before it; one CTA, a thread per 4 consecutive cells.
-template <typename T, bool kFwd>
-__device__ __forceinline__ void chamfer_rows(T* __restrict__ dist, int w, int ya, int yb, unsigned char* smem_raw)
+// Shared words of a row's scan: per warp its total and the key of the cell that
+// the warp on the other side of it needs, double-buffered by row parity
+template <typename K>
+struct ChamferShared {
+    K tot[2][32];
+    K edge[2][32];
+};
+
+// Rows ya, ya + dir, ..., yb of one pass (dir = +1 down, -1 up); one CTA, a
+// thread per 4 consecutive cells.  `before`: the row before ya (null: none).
+// kWrite: rows go back to dist.  `last`: receives the last row (null: not wanted).
+template <typename T, bool kFwd, bool kWrite>
+__device__ __forceinline__ void chamfer_rows(T* __restrict__ dist, int w, int ya, int yb,
+                                             const typename ChamferKey<T>::K* before, typename ChamferKey<T>::K* last,
+                                             ChamferShared<typename ChamferKey<T>::K>& sh)
 {
     using K = typename ChamferKey<T>::K;
     constexpr K kInf = ChamferKey<T>::kInf;
     constexpr int C = kChamferCells;
-    K* prev = reinterpret_cast<K*>(smem_raw);   // [2][w + 2], cell x at index x + 1
-    K* wtot = prev + 2 * (w + 2);               // [32]
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int x0 = threadIdx.x * C;
-    if (threadIdx.x == 0) {
-        prev[0] = prev[w + 1] = kInf;
-        prev[w + 2] = prev[2 * (w + 2) - 1] = kInf;
+    K r[C], re = kInf, le = kInf;   // the previous row's cells x0 .. x0+3, x0+4 and x0-1
+#pragma unroll
+    for (int c = 0; c < C; c++) r[c] = kInf;
+    bool have = before != nullptr;
+    if (have) {
+#pragma unroll
+        for (int c = 0; c < C; c++)
+            if (x0 + c < w) r[c] = before[x0 + c];
+        if (x0 > 0 && x0 <= w) le = before[x0 - 1];
+        if (x0 + C < w) re = before[x0 + C];
     }
-    __syncthreads();
-    int b = 0;
     const int dir = kFwd ? 1 : -1;
-    for (int y = ya;; y += dir) {
-        const K* pv = y == ya ? nullptr : prev + b * (w + 2);
-        K* pn = prev + (b ^ 1) * (w + 2);
-        K u[C];
+    K nv[C];
+    auto fetch = [&](int y) {
+#pragma unroll
+        for (int c = 0; c < C; c++) nv[c] = x0 + c < w ? (K)dist[(long long)y * w + x0 + c] : kInf;
+    };
+    fetch(ya);
+    int b = 0;
+    __syncthreads();   // an earlier walk of this CTA may still read the shared words
+    for (int y = ya;; y += dir, b ^= 1) {
+        K m[C];
 #pragma unroll
         for (int c = 0; c < C; c++) {
-            const int x = x0 + c;
-            u[c] = x < w ? (K)dist[(long long)y * w + x] : kInf;
-            if (pv && x < w) u[c] = min(u[c], min(min(pv[x], pv[x + 2]) + 4, pv[x + 1] + 3));
+            K u = nv[c];
+            if (have) u = min(u, min(min(c ? r[c - 1] : le, c < C - 1 ? r[c + 1] : re) + 4, r[c] + 3));
+            m[c] = x0 + c < w ? (kFwd ? u - 3 * (K)(x0 + c) : u + 3 * (K)(x0 + c)) : kInf;
         }
-        K m[C];
+        if (y != yb) fetch(y + dir);   // the next row's cells, while this one is scanned
+        const K own_edge = kFwd ? m[0] : m[C - 1];
         if (kFwd) {
 #pragma unroll
-            for (int c = 0; c < C; c++) {
-                const K key = x0 + c < w ? u[c] - 3 * (K)(x0 + c) : kInf;
-                m[c] = c ? min(m[c - 1], key) : key;
-            }
+            for (int c = 1; c < C; c++) m[c] = min(m[c - 1], m[c]);
         } else {
 #pragma unroll
-            for (int c = C - 1; c >= 0; c--) {
-                const K key = x0 + c < w ? u[c] + 3 * (K)(x0 + c) : kInf;
-                m[c] = c < C - 1 ? min(m[c + 1], key) : key;
-            }
+            for (int c = C - 2; c >= 0; c--) m[c] = min(m[c + 1], m[c]);
         }
-        const K ex = block_excl_min<K, kFwd>(kFwd ? m[C - 1] : m[0], wtot, kInf);
+        K incl;
+        const K excl = warp_excl_min<K, kFwd>(kFwd ? m[C - 1] : m[0], kInf, &incl);
+        if (lane == (kFwd ? 31 : 0)) sh.tot[b][wid] = incl;
+        if (lane == (kFwd ? 0 : 31)) sh.edge[b][wid] = own_edge;
+        __syncthreads();
+        // the min over the warps before mine (kInf: none)
+        const K wex = min(kInf, warp_min_k(lane < nw ? sh.tot[b][lane] : kInf, kFwd ? lane < wid : lane > wid));
+        const K ex = min(excl, wex);
 #pragma unroll
         for (int c = 0; c < C; c++) {
             const int x = x0 + c;
-            const K r = kFwd ? min(ex, m[c]) + 3 * (K)x : min(ex, m[c]) - 3 * (K)x;
-            if (x < w) {
-                dist[(long long)y * w + x] = (T)r;
-                pn[x + 1] = r;
-            }
+            r[c] = x < w ? (kFwd ? min(ex, m[c]) + 3 * (K)x : min(ex, m[c]) - 3 * (K)x) : kInf;
         }
-        __syncthreads();   // the next row reads pn; the next scan rewrites wtot
-        b ^= 1;
+        if (kWrite) {
+#pragma unroll
+            for (int c = 0; c < C; c++)
+                if (x0 + c < w) dist[(long long)y * w + x0 + c] = (T)r[c];
+        }
         if (y == yb) break;
+        // neighbours in this row for the next: by shuffle inside the warp; the
+        // cell before the warp in scan order is the scan of all warps before,
+        // the cell after it the scan through this warp and that cell's own key
+        le = shfl_up_k(r[C - 1], 1);
+        re = shfl_down_k(r[0], 1);
+        const K thru = min(wex, sh.tot[b][wid]);
+        if (lane == 0)
+            le = wid == 0 ? kInf : (kFwd ? wex : min(thru, sh.edge[b][wid - 1])) + (kFwd ? 3 : -3) * (K)(x0 - 1);
+        if (lane == 31)
+            re = x0 + C >= w ? kInf : (kFwd ? min(thru, sh.edge[b][wid + 1]) : wex) + (kFwd ? 3 : -3) * (K)(x0 + C);
+        have = true;
+    }
+    if (last) {
+#pragma unroll
+        for (int c = 0; c < C; c++)
+            if (x0 + c < w) last[x0 + c] = r[c];
     }
 }
 
@@ -143,133 +181,130 @@ __device__ __forceinline__ void chamfer_rows(T* __restrict__ dist, int w, int ya
 template <typename T>
 __global__ void __launch_bounds__(1024) k_chamfer2(T* __restrict__ dist, int w, int h)
 {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    chamfer_rows<T, true>(dist, w, 0, h - 1, smem_raw);
-    chamfer_rows<T, false>(dist, w, h - 1, 0, smem_raw);
+    using K = typename ChamferKey<T>::K;
+    __shared__ ChamferShared<K> sh;
+    chamfer_rows<T, true, true>(dist, w, 0, h - 1, nullptr, nullptr, sh);
+    chamfer_rows<T, false, true>(dist, w, h - 1, 0, nullptr, nullptr, sh);
 }
 
 // ---- the same passes over blocks of R rows ----
 // A pass only takes mins of sums of exact integers, so it is min-plus linear:
-// a block's result is the min of (a) the block run with nothing before its
-// first row and (b) the boundary row before it carried through the block with
-// every cell of the block "no value".  (b) has a closed form: a cell r rows
-// past the boundary row gets min over j of T[j] + c(x - j, r), c the cheapest
-// path of the pass's steps (3 straight, 4 diagonal, along the row only in the
-// scan direction): c = 3 max(|dx|, r) + min(|dx|, r) where the path can reach,
-// i.e. |dx| <= r, or any dx on the side the row scan moves towards.  So:
-//   1. every block runs with nothing before it (parallel over blocks);
-//   2. one CTA walks the blocks: a block's true last row is the min of its
-//      row from step 1 and the previous true last row carried R rows;
-//   3. every row of every block takes the min with the previous block's true
-//      last row carried to it (parallel over rows).
-constexpr int kChamferBlockRows = 32;
+// a block's last row is the min of (a) its last row when nothing comes before
+// the block and (b) the true last row of the block before carried through R
+// rows of "no value".  The carry has a closed form: a cell gets min over j of
+// in[j] + c(x - j), c the cheapest path of the pass's steps (3 straight, 4
+// diagonal, along the row only in the scan direction): 3 R + |dx| for
+// |dx| <= R, 3 |dx| + R beyond that on the side the row scan comes from.  A
+// row that went through the row scan never rises by more than 3 from one cell
+// to the next, so the far side never beats the window's edge cell, and the
+// carry is  carry_r(in)[x] = 3 r + min over |dx| <= r of in[x - dx] + |dx|.
+// Carries compose (carry_a after carry_b is carry_(a + b)), so the blocks'
+// true last rows are a scan over the blocks: with s = 1, 4, 16, ...
+//     row_k <- min(row_k, carry_(sR) of row_(k-s), carry_(2sR) of row_(k-2s),
+//                  carry_(3sR) of row_(k-3s))
+// makes row_k right for 4s blocks.  One cooperative launch, a CTA per block:
+//   1. run the block with nothing before it, keep its last row;
+//   2. the scan, one grid barrier per level;
+//   3. run the block again from the previous block's true last row, writing it;
+// and the same upwards.
+//
+// What bounds it: the barrier and shuffle latency of the 4 R rows a CTA walks
+// and the scan's grid barriers.  1024 x 1024 int16: 0.47 ms when one CTA
+// carried the rows from block to block and each cell searched its window;
+// 0.11 ms now.
+constexpr int kChamferBlockRows = 8;
 
-template <typename T, bool kFwd>
-__global__ void __launch_bounds__(1024) k_chamfer_blocks(T* __restrict__ dist, int w, int h, int R)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int y0 = blockIdx.x * R, y1 = min(h, y0 + R);
-    if (kFwd)
-        chamfer_rows<T, true>(dist, w, y0, y1 - 1, smem_raw);
-    else
-        chamfer_rows<T, false>(dist, w, y1 - 1, y0, smem_raw);
-}
+template <typename K>
+struct ChamferCoop {
+    K* rows;          // [2][nb][w]: the scan's rows, by level parity
+    unsigned* ctl;    // [0] count, [1] generation of the grid barrier
+    int* err;
+    int w, h, R, nb;
+};
 
-// The boundary row bt carried r rows into the next block, at cell x: the window
-// |x - j| <= r (cost 3r + |x - j|) and the far side the scan moves from (pre:
-// prefix min of bt[j] - 3j going down, suffix min of bt[j] + 3j going up).
-template <typename K, bool kFwd>
-__device__ __forceinline__ K carried(const K* bt, const K* pre, int w, int x, int r, K inf)
+// in <- carry of `in` by r rows, less its 3 r: window minima by doubling,
+// D_2a[x] = min(D_a[x], D_a[x - a] + a, D_a[x + a] + a).  Returns the buffer
+// that holds the result.
+template <typename K>
+__device__ __forceinline__ K* chamfer_window(K* in, K* out, int w, int r)
 {
-    K best = inf;
-    const int ja = max(0, x - r), jb = min(w - 1, x + r);
-    for (int j = ja; j <= jb; j++) best = min(best, bt[j] + 3 * (K)r + (K)abs(x - j));
-    if (kFwd) {
-        if (x - r - 1 >= 0) best = min(best, pre[x - r - 1] + 3 * (K)x + (K)r);
-    } else {
-        if (x + r + 1 < w) best = min(best, pre[x + r + 1] - 3 * (K)x + (K)r);
-    }
-    return best;
-}
-
-// Step 2: one CTA walks the blocks in scan order and keeps each true boundary
-// row (bt[blk]) with its prefix / suffix minima (pre[blk]) for step 3.
-template <typename T, bool kFwd>
-__global__ void __launch_bounds__(1024) k_chamfer_chain(T* __restrict__ dist, int w, int h, int R,
-                                                        typename ChamferKey<T>::K* __restrict__ bt,
-                                                        typename ChamferKey<T>::K* __restrict__ pre)
-{
-    using K = typename ChamferKey<T>::K;
-    constexpr K kInf = ChamferKey<T>::kInf;
-    constexpr int C = kChamferCells;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    K* cur = reinterpret_cast<K*>(smem_raw);   // [w] boundary row
-    K* cpre = cur + w;                          // [w] its prefix / suffix minima
-    K* wtot = cpre + w;                         // [32]
-    const int nb = (h + R - 1) / R;
-    const int x0 = threadIdx.x * C;
-    for (int s = 0; s < nb - 1; s++) {
-        const int blk = kFwd ? s : nb - 1 - s;          // the block whose boundary row this is
-        const int yb = kFwd ? min(h, (blk + 1) * R) - 1 : blk * R;   // its last row in scan order
-        K v[C];
-#pragma unroll
-        for (int c = 0; c < C; c++) {
-            const int x = x0 + c;
-            v[c] = x < w ? (K)dist[(long long)yb * w + x] : kInf;
-            if (s > 0 && x < w) {
-                const int rows = kFwd ? yb - (blk * R - 1) : (blk + 1) * R - yb;
-                v[c] = min(v[c], carried<K, kFwd>(cur, cpre, w, x, rows, kInf));
-            }
-        }
-        __syncthreads();   // every thread has read the previous boundary row
-        K m[C];
-        if (kFwd) {
-#pragma unroll
-            for (int c = 0; c < C; c++) {
-                const K key = x0 + c < w ? v[c] - 3 * (K)(x0 + c) : kInf;
-                m[c] = c ? min(m[c - 1], key) : key;
-            }
-        } else {
-#pragma unroll
-            for (int c = C - 1; c >= 0; c--) {
-                const K key = x0 + c < w ? v[c] + 3 * (K)(x0 + c) : kInf;
-                m[c] = c < C - 1 ? min(m[c + 1], key) : key;
-            }
-        }
-        const K ex = block_excl_min<K, kFwd>(kFwd ? m[C - 1] : m[0], wtot, kInf);
-#pragma unroll
-        for (int c = 0; c < C; c++) {
-            const int x = x0 + c;
-            if (x < w) {
-                const K pm = min(ex, m[c]);
-                cur[x] = v[c];
-                cpre[x] = pm;
-                bt[(long long)blk * w + x] = v[c];
-                pre[(long long)blk * w + x] = pm;
-            }
+    constexpr K kInf = sizeof(K) == 8 ? (K)(1LL << 62) : (K)(1 << 29);
+    for (int have = 0; have < r && have < w;) {
+        const int o = have ? have : 1;   // window 0 -> 1 -> 2 -> 4 ... -> r
+        for (int x = threadIdx.x; x < w; x += blockDim.x) {
+            const K l = x >= o ? in[x - o] : kInf, g = x + o < w ? in[x + o] : kInf;
+            out[x] = min(in[x], min(l, g) + (K)o);
         }
         __syncthreads();
+        K* t = in;
+        in = out;
+        out = t;
+        have += o;
     }
+    return in;
 }
 
-// Step 3: every row of a block after the first in scan order takes the min with
-// the previous block's true boundary row carried to it.
+// One way (down or up) of the field.  Returns false when a grid barrier gave up.
 template <typename T, bool kFwd>
-__global__ void __launch_bounds__(256) k_chamfer_apply(T* __restrict__ dist, int w, int h, int R,
-                                                       const typename ChamferKey<T>::K* __restrict__ bt,
-                                                       const typename ChamferKey<T>::K* __restrict__ pre)
+__device__ __forceinline__ bool chamfer_way(T* __restrict__ dist, const ChamferCoop<typename ChamferKey<T>::K>& p,
+                                            ChamferShared<typename ChamferKey<T>::K>& sh,
+                                            typename ChamferKey<T>::K* buf, int& parity)
 {
     using K = typename ChamferKey<T>::K;
-    constexpr K kInf = ChamferKey<T>::kInf;
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y;
-    const int blk = y / R, nb = (h + R - 1) / R;
-    if (x >= w || (kFwd ? blk == 0 : blk == nb - 1)) return;
-    const int src = kFwd ? blk - 1 : blk + 1;
-    const int rows = kFwd ? y - (blk * R - 1) : (blk + 1) * R - y;
-    const K c = carried<K, kFwd>(bt + (long long)src * w, pre + (long long)src * w, w, x, rows, kInf);
-    T* p = dist + (long long)y * w + x;
-    if (c < (K)*p) *p = (T)c;
+    const int w = p.w;
+    const int pos = kFwd ? blockIdx.x : p.nb - 1 - blockIdx.x;   // the block's place in scan order
+    const int y0 = blockIdx.x * p.R, y1 = min(p.h, y0 + p.R);
+    auto row = [&](int which, int q) { return p.rows + ((size_t)which * p.nb + q) * w; };
+    K* mine = buf;             // this block's row
+    K* wa = buf + w;           // two window buffers
+    K* wb = buf + 2 * w;
+    // a last block of fewer than R rows is last downwards (no block needs its
+    // row) and first upwards (its row is its whole result)
+    chamfer_rows<T, kFwd, false>(dist, w, kFwd ? y0 : y1 - 1, kFwd ? y1 - 1 : y0, nullptr, mine, sh);
+    __syncthreads();
+    for (int s = 1; s < p.nb; s *= 4) {
+        parity ^= 1;
+        for (int x = threadIdx.x; x < w; x += blockDim.x) row(parity, pos)[x] = mine[x];
+        if (!grid_barrier(p.ctl, p.ctl + 1, p.err, kGridWaitNs)) return false;
+        const int terms = min(3, pos / s);
+        if (terms > 0) {
+            const int r = s * p.R;
+            K* in = wa;
+            for (int t = terms; t > 0; t--) {   // the farthest first, each carried s more blocks with the next
+                K* other = in == wa ? wb : wa;
+                for (int x = threadIdx.x; x < w; x += blockDim.x) {
+                    const K v = __ldcg(row(parity, pos - t * s) + x);
+                    in[x] = t == terms ? v : min(v, in[x] + 3 * (K)r);
+                }
+                __syncthreads();
+                in = chamfer_window(in, other, w, r);
+            }
+            for (int x = threadIdx.x; x < w; x += blockDim.x) mine[x] = min(mine[x], in[x] + 3 * (K)r);
+            __syncthreads();
+        }
+    }
+    parity ^= 1;
+    for (int x = threadIdx.x; x < w; x += blockDim.x) row(parity, pos)[x] = mine[x];
+    if (!grid_barrier(p.ctl, p.ctl + 1, p.err, kGridWaitNs)) return false;
+    if (pos > 0) {
+        for (int x = threadIdx.x; x < w; x += blockDim.x) mine[x] = __ldcg(row(parity, pos - 1) + x);
+        __syncthreads();
+    }
+    chamfer_rows<T, kFwd, true>(dist, w, kFwd ? y0 : y1 - 1, kFwd ? y1 - 1 : y0, pos ? mine : nullptr, nullptr, sh);
+    return true;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(1024) k_chamfer_coop(T* __restrict__ dist, ChamferCoop<typename ChamferKey<T>::K> p)
+{
+    using K = typename ChamferKey<T>::K;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ ChamferShared<K> sh;
+    K* buf = reinterpret_cast<K*>(smem_raw);   // three rows
+    int parity = 0;
+    if (!chamfer_way<T, true>(dist, p, sh, buf, parity)) return;
+    __syncthreads();
+    chamfer_way<T, false>(dist, p, sh, buf, parity);   // a block's rows are its own: no barrier in between
 }
 
 template <typename T>
@@ -292,39 +327,45 @@ int chamfer_threads(int w)
 }
 
 template <typename T>
-void launch_chamfer_2d(T* dist, int w, int h, cudaStream_t st)
+void launch_chamfer_2d(T* dist, int w, int h, int* err, cudaStream_t st)
 {
     using K = typename ChamferKey<T>::K;
-    const size_t smem = (2 * (size_t)(w + 2) + 32) * sizeof(K);
     const int threads = chamfer_threads(w);
     ProfScope ps("chamfer_2d", st);
-    const int R = kChamferBlockRows, nb = (h + R - 1) / R;
-    void* scratch = nullptr;
-    const size_t sb = 2 * (size_t)nb * w * sizeof(K);
-    if (nb >= 2 && h <= 65535 && cudaMallocAsync(&scratch, sb, st) == cudaSuccess) {
-        K* bt = static_cast<K*>(scratch);
-        K* pre = bt + (size_t)nb * w;
-        const size_t csmem = (2 * (size_t)w + 32) * sizeof(K);
-        auto set = [](const void* f, size_t b) {
-            if (b > 48 * 1024) cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b);
-        };
-        set((const void*)k_chamfer_blocks<T, true>, smem);
-        set((const void*)k_chamfer_blocks<T, false>, smem);
-        set((const void*)k_chamfer_chain<T, true>, csmem);
-        set((const void*)k_chamfer_chain<T, false>, csmem);
-        const dim3 ag((w + 255) / 256, h);
-        k_chamfer_blocks<T, true><<<nb, threads, smem, st>>>(dist, w, h, R);
-        k_chamfer_chain<T, true><<<1, threads, csmem, st>>>(dist, w, h, R, bt, pre);
-        k_chamfer_apply<T, true><<<ag, 256, 0, st>>>(dist, w, h, R, bt, pre);
-        k_chamfer_blocks<T, false><<<nb, threads, smem, st>>>(dist, w, h, R);
-        k_chamfer_chain<T, false><<<1, threads, csmem, st>>>(dist, w, h, R, bt, pre);
-        k_chamfer_apply<T, false><<<ag, 256, 0, st>>>(dist, w, h, R, bt, pre);
-        cudaFreeAsync(scratch, st);
-        return;
+    if (h >= 2 * kChamferBlockRows) {
+        const size_t smem = 3 * (size_t)w * sizeof(K);
+        if (smem > 48 * 1024)
+            cudaFuncSetAttribute(k_chamfer_coop<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        int per_sm = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_chamfer_coop<T>, threads, smem);
+        // every block's CTA has to be resident: longer blocks for taller fields
+        const long long resident = (long long)per_sm * g_num_sms;
+        int R = kChamferBlockRows;
+        while (resident > 0 && (h + R - 1) / R > resident) R *= 2;
+        const int nb = (h + R - 1) / R;
+        void* scratch = nullptr;
+        const size_t rows = 2 * (size_t)nb * w * sizeof(K);
+        if (resident > 0 && nb >= 2 && cudaMallocAsync(&scratch, rows + 256, st) == cudaSuccess) {
+            ChamferCoop<K> p{static_cast<K*>(scratch), reinterpret_cast<unsigned*>(static_cast<char*>(scratch) + rows),
+                             err, w, h, R, nb};
+            cudaMemsetAsync(p.ctl, 0, 2 * sizeof(unsigned), st);
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(nb);
+            cfg.blockDim = dim3(threads);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = st;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeCooperative;
+            attr[0].val.cooperative = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            const bool ok = cudaLaunchKernelEx(&cfg, k_chamfer_coop<T>, dist, p) == cudaSuccess;
+            cudaFreeAsync(scratch, st);
+            if (ok) return;
+        }
+        cudaGetLastError();   // no scratch or no cooperative launch: walk the whole field in one CTA
     }
-    cudaGetLastError();   // a failed scratch allocation: walk the whole field in one CTA
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_chamfer2<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_chamfer2<T><<<1, threads, smem, st>>>(dist, w, h);
+    k_chamfer2<T><<<1, threads, 0, st>>>(dist, w, h);
 }
 
 template <typename T>
@@ -336,8 +377,8 @@ void launch_init_distances_int(const uint32_t* mask, T* dist, int w, long long r
     k_init_distances_int<T><<<(int)(blocks < cap ? blocks : cap), 256, 0, st>>>(mask, dist, w, rows, max_d);
 }
 
-template void launch_chamfer_2d<int16_t>(int16_t*, int, int, cudaStream_t);
-template void launch_chamfer_2d<int32_t>(int32_t*, int, int, cudaStream_t);
+template void launch_chamfer_2d<int16_t>(int16_t*, int, int, int*, cudaStream_t);
+template void launch_chamfer_2d<int32_t>(int32_t*, int, int, int*, cudaStream_t);
 template void launch_init_distances_int<int16_t>(const uint32_t*, int16_t*, int, long long, int16_t, cudaStream_t);
 template void launch_init_distances_int<int32_t>(const uint32_t*, int32_t*, int, long long, int32_t, cudaStream_t);
 

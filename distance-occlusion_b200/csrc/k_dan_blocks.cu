@@ -29,6 +29,7 @@
 // blocks are taken from a work list, a block that changed queues its
 // dependents for the next round, and two grid barriers (bounded waits) close
 // each round.
+#include "grid_barrier.cuh"
 #include "kernels.h"
 #include "scan.cuh"
 
@@ -85,43 +86,6 @@ struct DanBlk {
     int nblocks;  // nk * nc
     int max_rounds;
 };
-
-__device__ __forceinline__ unsigned long long global_ns()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// Grid barrier for a cooperative launch (all CTAs resident).  The wait gives
-// up after `limit_ns`, sets *err and returns false in every thread of the CTA.
-__device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned* gen, int* err, unsigned long long limit_ns)
-{
-    __syncthreads();
-    int ok = 1;
-    if (threadIdx.x == 0) {
-        volatile unsigned* vg = gen;
-        const unsigned g = *vg;
-        __threadfence();
-        if (atomicAdd(count, 1u) == gridDim.x - 1) {
-            atomicExch(count, 0u);
-            __threadfence();
-            atomicAdd(gen, 1u);
-        } else {
-            const unsigned long long t0 = global_ns();
-            while (*vg == g) {
-                __nanosleep(100);
-                if (global_ns() - t0 > limit_ns) {
-                    atomicExch(err, 2);
-                    ok = 0;
-                    break;
-                }
-            }
-        }
-        __threadfence();
-    }
-    return __syncthreads_and(ok);
-}
 
 // bits of DanBlk::chg
 constexpr int kChgLast = 1;    // a row of the block's last slice changed  -> block (k+1, c)
@@ -317,7 +281,6 @@ __global__ void __launch_bounds__(T, 512 / T) k_dan_blocks(DanBlk p)
     __shared__ ScanShared<Cell, T> sh;
     __shared__ int s_item, s_chg;
     const int t = threadIdx.x;
-    const unsigned long long kLimit = 20ull * 1000 * 1000 * 1000;   // 20 s per barrier wait
     int round = 0;
     for (;; round++) {
         const int cur = round & 1;
@@ -355,7 +318,7 @@ __global__ void __launch_bounds__(T, 512 / T) k_dan_blocks(DanBlk p)
             }
             __syncthreads();   // s_item / s_chg are rewritten by the next take
         }
-        if (!grid_barrier(p.ctl + 3, p.ctl + 4, p.err, kLimit)) return;
+        if (!grid_barrier(p.ctl + 3, p.ctl + 4, p.err, kGridWaitNs)) return;
         // commit: blocks whose output changed now hold it in the other version
         for (unsigned i = blockIdx.x * blockDim.x + t; i < nwork; i += gridDim.x * blockDim.x) {
             const int b = __ldcg(wl + i);
@@ -365,7 +328,7 @@ __global__ void __launch_bounds__(T, 512 / T) k_dan_blocks(DanBlk p)
             p.ctl[2] = 0;
             p.ctl[cur] = 0;
         }
-        if (!grid_barrier(p.ctl + 3, p.ctl + 4, p.err, kLimit)) return;
+        if (!grid_barrier(p.ctl + 3, p.ctl + 4, p.err, kGridWaitNs)) return;
         if (__ldcg(p.ctl + (cur ^ 1)) == 0) break;
     }
     if (blockIdx.x == 0 && t == 0) p.ctl[5] = (unsigned)(round + 1);
