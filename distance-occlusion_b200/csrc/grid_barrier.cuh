@@ -12,29 +12,29 @@ __device__ __forceinline__ unsigned long long global_ns()
     return t;
 }
 
-// Grid barrier for a cooperative launch (all CTAs resident).  The wait gives
-// up after `limit_ns`, sets *err and returns false in every thread of the CTA.
-__device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned* gen, int* err, unsigned long long limit_ns)
+// Grid barrier for a cooperative launch (all CTAs resident): `count` counts
+// arrivals over the whole launch (zero at its start), `passed` the barriers
+// that this CTA has been through (kept by the caller, the same in all
+// threads).  The wait gives up after kGridWaitNs, sets *err and returns false in
+// every thread of the CTA.
+__device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned& passed, int* err)
 {
+    passed++;
     __syncthreads();
     int ok = 1;
     if (threadIdx.x == 0) {
-        volatile unsigned* vg = gen;
-        const unsigned g = *vg;
+        const unsigned target = passed * gridDim.x;
         __threadfence();
-        if (atomicAdd(count, 1u) == gridDim.x - 1) {
-            atomicExch(count, 0u);
-            __threadfence();
-            atomicAdd(gen, 1u);
-        } else {
-            const unsigned long long t0 = global_ns();
-            while (*vg == g) {
-                __nanosleep(32);
-                if (global_ns() - t0 > limit_ns) {
-                    atomicExch(err, 2);
-                    ok = 0;
-                    break;
-                }
+        atomicAdd(count, 1u);
+        const unsigned long long t0 = global_ns();
+        for (unsigned polls = 1;; polls++) {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+            if ((int)(v - target) >= 0) break;
+            if (polls % 64 == 0 && global_ns() - t0 > kGridWaitNs) {
+                atomicExch(err, 2);
+                ok = 0;
+                break;
             }
         }
         __threadfence();

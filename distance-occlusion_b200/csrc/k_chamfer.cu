@@ -217,7 +217,7 @@ constexpr int kChamferBlockRows = 8;
 template <typename K>
 struct ChamferCoop {
     K* rows;          // [2][nb][w]: the scan's rows, by level parity
-    unsigned* ctl;    // [0] count, [1] generation of the grid barrier
+    unsigned* ctl;    // arrivals at the grid barrier
     int* err;
     int w, h, R, nb;
 };
@@ -248,7 +248,7 @@ __device__ __forceinline__ K* chamfer_window(K* in, K* out, int w, int r)
 template <typename T, bool kFwd>
 __device__ __forceinline__ bool chamfer_way(T* __restrict__ dist, const ChamferCoop<typename ChamferKey<T>::K>& p,
                                             ChamferShared<typename ChamferKey<T>::K>& sh,
-                                            typename ChamferKey<T>::K* buf, int& parity)
+                                            typename ChamferKey<T>::K* buf, int& parity, unsigned& passed)
 {
     using K = typename ChamferKey<T>::K;
     const int w = p.w;
@@ -265,7 +265,7 @@ __device__ __forceinline__ bool chamfer_way(T* __restrict__ dist, const ChamferC
     for (int s = 1; s < p.nb; s *= 4) {
         parity ^= 1;
         for (int x = threadIdx.x; x < w; x += blockDim.x) row(parity, pos)[x] = mine[x];
-        if (!grid_barrier(p.ctl, p.ctl + 1, p.err, kGridWaitNs)) return false;
+        if (!grid_barrier(p.ctl, passed, p.err)) return false;
         const int terms = min(3, pos / s);
         if (terms > 0) {
             const int r = s * p.R;
@@ -285,7 +285,7 @@ __device__ __forceinline__ bool chamfer_way(T* __restrict__ dist, const ChamferC
     }
     parity ^= 1;
     for (int x = threadIdx.x; x < w; x += blockDim.x) row(parity, pos)[x] = mine[x];
-    if (!grid_barrier(p.ctl, p.ctl + 1, p.err, kGridWaitNs)) return false;
+    if (!grid_barrier(p.ctl, passed, p.err)) return false;
     if (pos > 0) {
         for (int x = threadIdx.x; x < w; x += blockDim.x) mine[x] = __ldcg(row(parity, pos - 1) + x);
         __syncthreads();
@@ -302,9 +302,10 @@ __global__ void __launch_bounds__(1024) k_chamfer_coop(T* __restrict__ dist, Cha
     __shared__ ChamferShared<K> sh;
     K* buf = reinterpret_cast<K*>(smem_raw);   // three rows
     int parity = 0;
-    if (!chamfer_way<T, true>(dist, p, sh, buf, parity)) return;
+    unsigned passed = 0;
+    if (!chamfer_way<T, true>(dist, p, sh, buf, parity, passed)) return;
     __syncthreads();
-    chamfer_way<T, false>(dist, p, sh, buf, parity);   // a block's rows are its own: no barrier in between
+    chamfer_way<T, false>(dist, p, sh, buf, parity, passed);   // a block's rows are its own: no barrier in between
 }
 
 template <typename T>
@@ -348,7 +349,7 @@ void launch_chamfer_2d(T* dist, int w, int h, int* err, cudaStream_t st)
         if (resident > 0 && nb >= 2 && cudaMallocAsync(&scratch, rows + 256, st) == cudaSuccess) {
             ChamferCoop<K> p{static_cast<K*>(scratch), reinterpret_cast<unsigned*>(static_cast<char*>(scratch) + rows),
                              err, w, h, R, nb};
-            cudaMemsetAsync(p.ctl, 0, 2 * sizeof(unsigned), st);
+            cudaMemsetAsync(p.ctl, 0, sizeof(unsigned), st);
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(nb);
             cfg.blockDim = dim3(threads);

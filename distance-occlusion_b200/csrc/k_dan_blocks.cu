@@ -3,370 +3,478 @@
 //
 // The reference's Danielsson (DistanceOcclusionLib.cpp:702-778 2D,
 // :2264-2394 3D) is one long chain: every row needs the previous row, every
-// slice the previous slice after its full 2D sweep.  Cut each sweep phase (the
-// 2D image; each z direction of a volume) into blocks of R rows of one slice.
-// A block runs the reference's steps over its rows -- z pull from the
-// previous slice, then rows y0..y1-1 going down, then y1-1..y0 going up --
-// from three inputs that other blocks produce:
+// slice the previous slice after its full 2D sweep, every cell of an x pass
+// the cell before it.  Cut each sweep phase (the 2D image; each z direction of
+// a volume) into blocks of 32 S columns, R rows and Z slices, a warp each.  A
+// block runs the reference's steps over its own cells -- slice by slice the z
+// pull, rows y0..y1-1 going down, then y1-1..y0 going up, each with its x
+// passes -- from the inputs that other blocks produce:
 //
-//   Z  the previous slice's rows y0..y1-1 after its sweep  (block (z-dir, c))
-//   D  row y0-1 after the down sweep                         (block (z, c-1))
-//   U  row y1 after the up sweep                             (block (z, c+1))
+//   Z  the previous slice's cells after its sweep               (block k-1)
+//   D  row y0-1 after the down sweep                            (block c-1)
+//   U  row y1 after the up sweep                                (block c+1)
+//   L  per row and sweep, the cell left of the block after the
+//      pass to the right                                        (block xb-1)
+//   R  the cell right of it after the pass to the left          (block xb+1)
 //
-// Every block starts from guesses (the phase input's own rows), all blocks
-// run in parallel, and each round recomputes exactly the blocks whose inputs
-// changed in the round before.  At the stop every block's inputs equal its
-// producers' outputs, so by induction along the serial order (split into down
-// and up halves it is acyclic: down(c) needs down(c-1); up(c) needs up(c+1)
-// and down(c)) every output is the serial one.  Round r finalises at least
-// one more half-block of the chain, so the iteration ends; in practice after
-// about as many rounds as the longest distance in cells (a seed's influence
-// crosses one slice per round), whatever R is.
+// Every block starts from guesses (the phase input's own rows, no cell at the
+// sides), all blocks run in parallel, and each round recomputes exactly the
+// blocks whose inputs changed in the round before.  At the stop every block's
+// inputs equal its producers' outputs, so by induction along the serial order
+// (split into the half sweeps and their passes it is acyclic) every output is
+// the serial one.  Round r finalises at least one more piece of the chain, so
+// the iteration ends; in practice after about as many rounds as the longest
+// distance in blocks that a seed's influence travels.
+//
+// What bounds it: rounds x the latency of a block, one dependent row step after
+// another, and with all blocks busy the integer pipe (some 400 instructions per
+// step of 128 cells).  Short segments make short steps, and cutting rows into
+// x blocks costs no rounds (a model of the iteration on the 256^3 volume of
+// boxes and spheres: 19 + 14 rounds at 256 and at 128 columns, 20 + 15 at 64,
+// with 9 / 8 / 7 times the serial work), while it takes the exchange between
+// the warps of a row out of every pass.
+// 256^3 boxes and spheres 17.4 -> 8.8 ms, 1024^2 with 100 points 1.41 -> 0.51 ms
+// against one CTA per block of whole rows.
 //
 // Outputs alternate between two version buffers per block, so a round reads
-// only the previous round's outputs; a block's version flips when its new
-// output differs from the old one.  One cooperative launch runs all rounds:
-// blocks are taken from a work list, a block that changed queues its
-// dependents for the next round, and two grid barriers (bounded waits) close
-// each round.
+// only the previous round's outputs; a block's version flips whenever it runs,
+// and the cells that other blocks read are compared with their old values to
+// find the blocks that have to run again.  One cooperative launch runs all
+// rounds, each closed by one grid barrier (bounded waits).  With a warp for
+// every block a block that changed marks its dependents for the next round;
+// larger fields take blocks from a work list.
+#include "dan_serial.cuh"
 #include "grid_barrier.cuh"
 #include "kernels.h"
-#include "scan.cuh"
 
 namespace dolk {
 
-constexpr int kBlkThreads = 256;   // the widest CTA (rows up to 8 x 256 cells)
-
-template <class Cell>
-struct CellIO;
-template <>
-struct CellIO<C2> {
-    using P = uint32_t;
-    static constexpr int kWords = 1;
-    static __device__ __forceinline__ C2 ld(const P* p, long long i) { return unpack2(__ldcg(p + i)); }
-    static __device__ __forceinline__ void st(P* p, long long i, C2 c) { p[i] = pack2(c); }
-};
-template <>
-struct CellIO<C3> {
-    using P = int16_t;
-    static constexpr int kWords = 3;
-    static __device__ __forceinline__ C3 ld(const P* p, long long i)
-    {
-        const P* c = p + 3 * i;
-        return C3{__ldcg(c), __ldcg(c + 1), __ldcg(c + 2)};
-    }
-    static __device__ __forceinline__ void st(P* p, long long i, C3 c)
-    {
-        P* o = p + 3 * i;
-        o[0] = (P)c.x;
-        o[1] = (P)c.y;
-        o[2] = (P)c.z;
-    }
-};
-
-DOL_HD C2 yshift(C2 c, int dy) { return add(c, 0, dy); }
-DOL_HD C3 yshift(C3 c, int dy) { return add(c, 0, dy, 0); }
+constexpr int kBlkMaxWidth = 2048;
+constexpr int kBlkMaxRows = 16;    // rows of a block: a lane per row and sweep
 
 struct DanBlk {
     const void* A;         // phase input, unchanged during the phase
     void* V[2];            // output versions (cells, same layout as A)
-    void* DB[2];           // per block and version: its last row after the down sweep
-    uint8_t* lat;          // per block: version holding its output (2: none yet, the input's rows stand)
-    uint8_t* chg;          // per block: change bits of its last computation
-    int* stamp;            // per block: last round it was queued for
-    int* wl[2];            // work lists by round parity
-    unsigned* ctl;         // [0],[1] work-list sizes, [2] work counter, [3],[4] grid barrier, [5] rounds used
+    void* DB[2];           // per slice, chunk of rows and version: its last row after the down sweep
+    uint2* XR[2];          // per row, sweep, x block and version: its last cell after the pass to the right (xy, z)
+    uint2* XL[2];          // its first cell after the pass to the left
+    unsigned* state;       // per block: round it last ran in + 1, version after and before that (block_state)
+    uint8_t* dirty[2];     // few blocks: per block, to run in the round of that parity
+    int* stamp;            // many blocks: per block, last round it was queued for
+    int* wl[2];            // and the work lists by round parity
+    unsigned* ctl;         // by round modulo 3: [0..2] a block changed / work-list size, [3..5] work counter;
+                           // [6] grid barrier, [7] rounds used
     int* err;
-    int w, h, d, R, nc, cw;
+    int w, h, d, R, nc, nx, cw;
     int dir;      // +1: slices zfirst, zfirst+1, ...; -1: downwards
     int zfirst;   // first slice of the phase's chain (the slice before it keeps its input)
     int nchain;   // slices in the chain (2D: 1)
     int Z;        // slices per block
     int nk;       // blocks along the chain: ceil(nchain / Z)
-    int nblocks;  // nk * nc
+    int nblocks;  // nk * nc * nx, block (k, c, xb) at (k * nc + c) * nx + xb
     int max_rounds;
 };
 
-// bits of DanBlk::chg
+// A block's state word: the round it last ran in plus 1, the version that holds
+// its output since and the one before (2: none yet, the input's rows stand).
+// One word, so that a reader of the same round sees either it or the word
+// before it, and takes the output of before this round from both.
+__device__ __forceinline__ unsigned block_state(int round, int now, int before)
+{
+    return ((unsigned)(round + 1) << 4) | ((unsigned)now << 2) | (unsigned)before;
+}
+__device__ __forceinline__ int block_version(unsigned state, int round)
+{
+    return (int)((state >> 4) == (unsigned)(round + 1) ? state & 3u : (state >> 2) & 3u);
+}
+
+// what a run changed for other blocks
 constexpr int kChgLast = 1;    // a row of the block's last slice changed  -> block (k+1, c)
 constexpr int kChgFirst = 2;   // row y0 of some slice changed             -> block (k, c-1)
 constexpr int kChgDown = 4;    // the down-sweep row y1-1 of some slice    -> block (k, c+1)
-constexpr int kChgAny = 8;     // any output changed: the block's version flips
+constexpr int kChgRight = 8;   // a last cell after a pass to the right    -> block xb+1
+constexpr int kChgLeft = 16;   // a first cell after a pass to the left    -> block xb-1
 
-// One block: rows y0..y1-1 of Z consecutive slices (in the phase's order),
-// T threads of S cells each.
-template <class Cell, int kDim, int S, int T>
-__device__ __forceinline__ void dan_block(const DanBlk& p, int b, ScanShared<Cell, T>& sh, int* s_chg)
+template <int DIM, int S>
+using BlockIO = RowIO<DIM, S, 2>;
+
+// Shared memory of a warp: its RowIO strips, then its part of the block's R
+// rows, cell s of lane l at [row][s][l]: after the down sweep a row's down
+// result, after the up sweep its result, which the next slice pulls from.
+template <int DIM, int S>
+__host__ __device__ constexpr size_t dan_warp_bytes(int R)
 {
-    using IO = CellIO<Cell>;
-    using P = typename IO::P;
-    const int t = threadIdx.x;
+    return BlockIO<DIM, S>::kBytes + (size_t)R * S * 32 * (DIM == 3 ? 6 : 4);
+}
+
+template <int DIM, int S>
+struct BlockRows;
+template <int S>
+struct BlockRows<2, S> {
+    uint32_t* c;
+
+    DOL_DI void put(int r, const Cells<2, S>& v) const
+    {
+#pragma unroll
+        for (int s = 0; s < S; s++) c[(r * S + s) * 32 + (threadIdx.x & 31)] = v.xy[s];
+    }
+    DOL_DI void get(int r, uint32_t (&xy)[S], int (&z)[S]) const
+    {
+#pragma unroll
+        for (int s = 0; s < S; s++) {
+            xy[s] = c[(r * S + s) * 32 + (threadIdx.x & 31)];
+            z[s] = 0;
+        }
+    }
+};
+template <int S>
+struct BlockRows<3, S> {
+    uint32_t* c;
+    int16_t* zz;
+
+    DOL_DI void put(int r, const Cells<3, S>& v) const
+    {
+#pragma unroll
+        for (int s = 0; s < S; s++) {
+            c[(r * S + s) * 32 + (threadIdx.x & 31)] = v.xy[s];
+            zz[(r * S + s) * 32 + (threadIdx.x & 31)] = (int16_t)v.z[s];
+        }
+    }
+    DOL_DI void get(int r, uint32_t (&xy)[S], int (&z)[S]) const
+    {
+#pragma unroll
+        for (int s = 0; s < S; s++) {
+            xy[s] = c[(r * S + s) * 32 + (threadIdx.x & 31)];
+            z[s] = zz[(r * S + s) * 32 + (threadIdx.x & 31)];
+        }
+    }
+};
+
+// One block by one warp; returns what changed (bits above, per lane).
+template <int DIM, int S>
+__device__ __forceinline__ int dan_block(const DanBlk& p, int b, int round, const BlockIO<DIM, S>& io,
+                                         const BlockRows<DIM, S>& T)
+{
+    using IO = BlockIO<DIM, S>;
+    using Row = Cells<DIM, S>;
+    const int lane = threadIdx.x & 31;
     const int w = p.w, h = p.h, cw = p.cw;
-    const int nseg = (w + S - 1) / S;
-    const bool active = t < nseg;
-    const int n = active ? min(S, w - t * S) : 0;
-    const long long x0 = (long long)t * S;
-    const int k = b / p.nc;
-    const int c = b - k * p.nc;
+    const int xb = b % p.nx, kc = b / p.nx;
+    const int k = kc / p.nc;
+    const int c = kc - k * p.nc;
+    const int xw = xb * 32 * S;
     const int y0 = c * p.R, y1 = min(y0 + p.R, h), L = y1 - y0;
     const long long plane = (long long)w * h;
-    const P* A = static_cast<const P*>(p.A);
-    auto ver = [&](int v) -> const P* { return v == 2 ? A : static_cast<const P*>(p.V[v]); };
-    const int vo = __ldcg(p.lat + b), vn = vo == 0 ? 1 : 0;
-    const P* oldv = ver(vo);
-    P* out = static_cast<P*>(p.V[vn]);
-    // neighbour blocks' versions (fixed for the whole round)
-    const int vd = c > 0 ? __ldcg(p.lat + b - 1) : 2;
-    const int vu = y1 < h ? __ldcg(p.lat + b + 1) : 2;
-    const int vz = (kDim == 3 && k > 0) ? __ldcg(p.lat + b - p.nc) : 2;
-    const int dz = kDim == 3 ? -p.dir * cw : 0;
+    const long long abytes = plane * p.d * IO::kCell, dbytes = (long long)p.nc * p.d * w * IO::kCell;
+    // neighbour blocks' versions (fixed for the whole round): lane i looks one up
+    int nb = b;
+    if (lane == 1) nb = c > 0 ? b - p.nx : -1;
+    if (lane == 2) nb = y1 < h ? b + p.nx : -1;
+    if (lane == 3) nb = DIM == 3 && k > 0 ? b - p.nc * p.nx : -1;
+    if (lane == 4) nb = xb > 0 ? b - 1 : -1;
+    if (lane == 5) nb = xb + 1 < p.nx ? b + 1 : -1;
+    const int ver = lane < 6 && nb >= 0 ? block_version(__ldcg(p.state + nb), round) : 2;
+    const int vo = __shfl_sync(0xFFFFFFFFu, ver, 0), vn = vo == 0 ? 1 : 0;
+    const int vd = __shfl_sync(0xFFFFFFFFu, ver, 1), vu = __shfl_sync(0xFFFFFFFFu, ver, 2);
+    const int vz = __shfl_sync(0xFFFFFFFFu, ver, 3);
+    const int vl = __shfl_sync(0xFFFFFFFFu, ver, 4), vr = __shfl_sync(0xFFFFFFFFu, ver, 5);
+    const int dz = -p.dir * cw;
     const int pos0 = k * p.Z, nsl = min(p.Z, p.nchain - pos0);
+    auto arr = [&](int v) { return static_cast<unsigned char*>(v == 2 ? const_cast<void*>(p.A) : p.V[v]); };
+    auto cell_at = [&](int z, int y) { return ((long long)z * plane + (long long)y * w + xw) * IO::kCell; };
+    auto fetch_a = [&](int r, int v, int z, int y) {
+        unsigned char* q = arr(v);
+        io.fetch(r, q + cell_at(z, y), q, q + abytes);
+    };
+    // the down-boundary row of chunk cc of slice z in version v (2: the input's row yy)
+    auto fetch_d = [&](int r, int v, int z, int cc, int yy) -> const unsigned char* {
+        if (v == 2) {
+            fetch_a(r, 2, z, yy);
+            return arr(2) + cell_at(z, yy);
+        }
+        unsigned char* q = static_cast<unsigned char*>(p.DB[v]);
+        const unsigned char* a = q + (((long long)z * p.nc + cc) * w + xw) * IO::kCell;
+        io.fetch(r, a, q, q + dbytes);
+        return a;
+    };
+    auto cells_xyz = [&](int r, const unsigned char* a, uint32_t (&xy)[S], int (&z)[S]) {
+        uint32_t wd[IO::kWords];
+        io.words(wd, r, a);
+        IO::split(wd, xy, z);
+    };
+    // does the fetched row differ from c in one of this lane's cells?
+    auto differs = [&](int r, const unsigned char* a, const Row& c) -> bool {
+        uint32_t xy[S];
+        int z[S];
+        cells_xyz(r, a, xy, z);
+        const int n = io.live();
+        bool d = false;
+#pragma unroll
+        for (int s = 0; s < S; s++) d |= s < n && (xy[s] != c.xy[s] || (DIM == 3 && z[s] != c.z[s]));
+        return d;
+    };
 
-    auto ldrow = [&](Cell (&dst)[S], const P* base, long long first) {
+    // a row as candidate only: cells that win against none when shifted by +-cw in y
+    auto absent = [&](Row& r) {
 #pragma unroll
-        for (int s = 0; s < S; s++)
-            if (s < n) dst[s] = IO::ld(base, first + s);
+        for (int s = 0; s < S; s++) {
+            r.xy[s] = 0;
+            r.z[s] = 0;
+            r.W[s] = 0;
+            r.L[s] = INT_MAX - cw * cw;
+        }
     };
-    auto strow = [&](P* base, long long first, const Cell (&src)[S]) {
-#pragma unroll
-        for (int s = 0; s < S; s++)
-            if (s < n) IO::st(base, first + s, src[s]);
-    };
-    auto zpull = [&](Cell cc, Cell q) -> Cell {
-        if constexpr (kDim == 3)
-            return closer(cc, add(q, 0, 0, dz));
-        else
-            return cc;
-    };
-
-    Cell Pr[S], V[S], Rr[S], D[S], Cn[S], Qn[S];
-#pragma unroll
-    for (int s = 0; s < S; s++) Pr[s] = V[s] = Rr[s] = D[s] = Cn[s] = Qn[s] = Cell{};
+    Row P, C;
+    // strips: the next step's row; the row beside it (slice before, block
+    // below); the row above the block, in the strip that stores use: it is
+    // loaded after a slice's last store and read before the next one's first
+    constexpr int rc = 0, rq = 1, rd = IO::kStrips - 1;
     int bits = 0;
-    int g = 0;
+    const bool has_d = c > 0, has_u = y1 < h;
+    const unsigned char* ad = nullptr;
+    auto first_rows = [&](int j) {   // what the first step of slice j needs
+        const int z = p.zfirst + p.dir * (pos0 + j);
+        if (has_d) ad = fetch_d(rd, vd, z, c - 1, y0 - 1);
+        fetch_a(rc, 2, z, y0);
+        if (DIM == 3 && j == 0) fetch_a(rq, vz, z - p.dir, y0);
+    };
+    // the sides: lane t holds the cells of step t of a slice
+    const bool sides = p.nx > 1;
+    const int yt = lane < L ? y0 + lane : y0 + 2 * L - 1 - lane;
+    auto side_at = [&](int z) { return (((long long)z * h + yt) * 2 + (lane < L ? 0 : 1)) * p.nx + xb; };
+    const uint2 kNoCell = make_uint2(0x80000000u, 0x80000000u);   // (z is never that: 16 bits)
+    uint2 inL = kNoCell, inR = kNoCell, nextL = kNoCell, nextR = kNoCell;
+    auto load_sides = [&](int j) {
+        const int z = p.zfirst + p.dir * (pos0 + j);
+        if (lane < 2 * L) {
+            if (vl != 2) nextL = __ldcg(p.XR[vl] + side_at(z) - 1);
+            if (vr != 2) nextR = __ldcg(p.XL[vr] + side_at(z) + 1);
+        }
+    };
+    auto side_input = [&](const uint2& in, int t) -> Chain {
+        const uint32_t xy = __shfl_sync(0xFFFFFFFFu, in.x, t);
+        const int z = (int)__shfl_sync(0xFFFFFFFFu, in.y, t);
+        if (z == (int)0x80000000u) return chain_none(cw);
+        return Chain{xy, w_of<DIM>(xy, z), z};
+    };
+    __syncwarp();
+    first_rows(0);
+    if (sides) load_sides(0);
 
     for (int j = 0; j < nsl; j++) {
         const int z = p.zfirst + p.dir * (pos0 + j);
-        const long long sb = (long long)z * plane;
         const bool last = j == nsl - 1;
-        // the previous slice after its sweep: this block's own output, or the
-        // block before in z (or the fixed slice, which keeps the input)
-        const P* zin = nullptr;
-        if (kDim == 3) zin = (j > 0 ? static_cast<const P*>(out) : ver(vz)) + IO::kWords * (sb - p.dir * plane);
-        const long long dbi = ((long long)z * p.nc + c) * w;   // this slice's down-boundary row slot
-        const P* gd = nullptr;   // row y0-1 after the down sweep
-        if (c > 0)
-            gd = vd == 2 ? A + IO::kWords * (sb + (long long)(y0 - 1) * w)
-                         : static_cast<const P*>(p.DB[vd]) + IO::kWords * (dbi - w);
-        const P* gu = nullptr;   // row y1 after the up sweep
-        if (y1 < h) gu = ver(vu) + IO::kWords * (sb + (long long)y1 * w);
-        const P* dbo = vo == 2 ? A + IO::kWords * (sb + (long long)(y1 - 1) * w)
-                               : static_cast<const P*>(p.DB[vo]) + IO::kWords * dbi;
-        P* dbn = static_cast<P*>(p.DB[vn]) + IO::kWords * dbi;
-
-        // row y0 before its x passes
-        ldrow(Cn, A, sb + (long long)y0 * w + x0);
-        if (kDim == 3) ldrow(Qn, zin, (long long)y0 * w + x0);
-#pragma unroll
-        for (int s = 0; s < S; s++) V[s] = kDim == 3 ? zpull(Cn[s], Qn[s]) : Cn[s];
-        if (gd) {
-            ldrow(Qn, gd, x0);
-#pragma unroll
-            for (int s = 0; s < S; s++) V[s] = closer(V[s], yshift(Qn[s], -cw));
-        }
-        __syncthreads();   // the previous slice's last pass may still read the guess slots
-        if (active) sh.guess[g][t] = seg_edge<Cell, S, +1>(V, n);
-        __syncthreads();
-
+        uint2 outR = kNoCell, outL = kNoCell;   // lane t: this block's own side cells of step t
+        inL = nextL;
+        inR = nextR;
+        // the row above the block after its down sweep is the first step's candidate
+        if (has_d) io.cells_of(P, rd, ad, cw);
+        else absent(P);
+        // steps 0 .. L-1 go down the rows, L .. 2L-1 back up
+#pragma unroll 1
         for (int i = 0; i < 2 * L; i++) {
             const bool down = i < L;
-            const int y = down ? y0 + i : y1 - 1 - (i - L);
-            const bool pass = down ? y > 0 : y < h - 1;
-            const int nx = i + 1;                     // next step
-            const bool more = nx < 2 * L;
-            const bool nx_down = nx < L;
-            const bool nx_turn = nx == L;             // first up step: base = this result, candidate = U
-            const bool has_u = gu != nullptr;
-            const long long rf = sb + (long long)y * w + x0;
-            // the old output this step's result is compared with, loaded
-            // before the passes so its latency hides behind them
-            Cell O[S];
-#pragma unroll
-            for (int s = 0; s < S; s++) O[s] = Cell{};
-            if (!down)
-                ldrow(O, oldv, rf);
-            else if (i == L - 1)
-                ldrow(O, dbo, x0);
-            // prefetch what the next step needs
-            if (more) {
-                if (nx_down) {
-                    ldrow(Cn, A, sb + (long long)(y + 1) * w + x0);
-                    if (kDim == 3) ldrow(Qn, zin, (long long)(y + 1) * w + x0);
-                } else if (nx_turn) {
-                    if (has_u) ldrow(Cn, gu, x0);
-                } else {
-                    ldrow(Cn, out, sb + (long long)(y - 1) * w + x0);   // its down-sweep result
+            const int q = down ? i : 2 * L - 1 - i, y = y0 + q;
+            uint32_t xy[S];
+            int zz[S];
+            if (down) {   // its own cells, then the slice before
+                io.cells_of(C, rc, arr(2) + cell_at(z, y), cw);
+                if constexpr (DIM == 3) {
+                    if (j == 0) cells_xyz(rq, arr(vz) + cell_at(z - p.dir, y), xy, zz);
+                    else T.get(q, xy, zz);
+                    pull_z<S>(C, xy, zz, dz);
                 }
-            }
-            // the next step's row before its x passes, from this step's result X
-            auto next_edge = [&](const Cell (&X)[S]) -> Cell {
-                const Cell e = seg_edge<Cell, S, +1>(X, n);
-                if (nx_down) {
-                    const Cell cb = kDim == 3 ? zpull(seg_edge<Cell, S, +1>(Cn, n), seg_edge<Cell, S, +1>(Qn, n))
-                                              : seg_edge<Cell, S, +1>(Cn, n);
-                    return closer(cb, yshift(e, -cw));
-                }
-                if (nx_turn) return has_u ? closer(e, yshift(seg_edge<Cell, S, +1>(Cn, n), cw)) : e;
-                return closer(seg_edge<Cell, S, +1>(Cn, n), yshift(e, cw));
-            };
-            if (pass) {
-                const Cell in0 = (active && t > 0) ? sh.guess[g][t - 1] : V[0];
-                row_pass<Cell, S, false, +1>(Rr, V, t, nseg, n, cw, sh, D, in0, [&](const Cell (&X)[S]) {
-                    if (active) sh.guess[g ^ 1][t] = X[0];
-                });
-                g ^= 1;
-                const Cell in1 = (active && t + 1 < nseg) ? sh.guess[g][t + 1] : Rr[0];
-                row_pass<Cell, S, false, -1>(Pr, Rr, t, nseg, n, cw, sh, D, in1, [&](const Cell (&X)[S]) {
-                    if (more && active) sh.guess[g ^ 1][t] = next_edge(X);
-                });
-                g ^= 1;
-            } else {
+            } else if (i > L) {   // its down result
+                T.get(q, xy, zz);
 #pragma unroll
-                for (int s = 0; s < S; s++) Pr[s] = V[s];
-                if (more && active) sh.guess[g][t] = next_edge(Pr);
-                __syncthreads();
-            }
-            if (down) {
-                strow(out, rf, Pr);
-                if (i == L - 1) {
+                for (int s = 0; s < S; s++) {
+                    C.xy[s] = xy[s];
+                    C.z[s] = zz[s];
+                    C.W[s] = w_of<DIM>(xy[s], zz[s]);
+                    C.L[s] = len_of(xy[s], C.W[s]);
+                }
+                const int n = io.live();
+                if (n < S) {
 #pragma unroll
                     for (int s = 0; s < S; s++)
-                        if (s < n && !same(O[s], Pr[s])) bits |= kChgDown | kChgAny;
-                    strow(dbn, x0, Pr);
+                        if (s >= n) set_none(C, s, cw);
                 }
-            } else {
-                bool diff = false;
-#pragma unroll
-                for (int s = 0; s < S; s++)
-                    if (s < n && !same(O[s], Pr[s])) diff = true;
-                if (diff) bits |= kChgAny | (last ? kChgLast : 0) | (y == y0 ? kChgFirst : 0);
-                strow(out, rf, Pr);
+            } else {   // the turn: its down result is at hand, the candidate is the row below the block
+                C = P;
+                if (has_u) io.cells_of(P, rq, arr(vu) + cell_at(z, y1), cw);
+                else absent(P);
             }
-            if (more) {
-                if (nx_down) {
-#pragma unroll
-                    for (int s = 0; s < S; s++) {
-                        const Cell cb = kDim == 3 ? zpull(Cn[s], Qn[s]) : Cn[s];
-                        V[s] = closer(cb, yshift(Pr[s], -cw));
-                    }
-                } else if (nx_turn) {
-#pragma unroll
-                    for (int s = 0; s < S; s++) V[s] = has_u ? closer(Pr[s], yshift(Cn[s], cw)) : Pr[s];
-                } else {
-#pragma unroll
-                    for (int s = 0; s < S; s++) V[s] = closer(Cn[s], yshift(Pr[s], cw));
+            // old results are compared where another block reads them: the
+            // block below reads the last down row, the block above the first
+            // row, the next block in z the last slice
+            const bool cmp_d = has_u && i == L - 1;
+            const bool cmp_u = !down && ((last && k + 1 < p.nk) || (q == 0 && has_d));
+            const unsigned char* ao = nullptr;
+            // loaded behind this step's passes: the old result, what the next step needs
+            if (i + 1 < L) {
+                fetch_a(rc, 2, z, y + 1);
+                if (DIM == 3 && j == 0) fetch_a(rq, vz, z - p.dir, y + 1);
+            } else if (i == L - 1) {
+                if (has_u) {
+                    ao = fetch_d(rc, vo, z, c, y);
+                    fetch_a(rq, vu, z, y1);
+                }
+            } else if (cmp_u) {
+                fetch_a(rc, vo, z, y);
+                ao = arr(vo) + cell_at(z, y);
+            }
+            merge_y<DIM, S>(P, C, down ? -cw : cw);
+            if (down ? y > 0 : y < h - 1) {
+                RowShared<1> none;
+                int par = 0;
+                Chain wl = chain_none(cw), wr = wl;
+                if (sides) {
+                    wl = side_input(inL, i);
+                    wr = side_input(inR, i);
+                }
+                row_pass_w<DIM, S, 1, +1, NoDiag>(P, NoDiag{}, cw, none, par, wl);
+                if (sides) {
+                    const uint32_t oxy = __shfl_sync(0xFFFFFFFFu, P.xy[S - 1], 31);
+                    const int oz = DIM == 3 ? __shfl_sync(0xFFFFFFFFu, P.z[S - 1], 31) : 0;
+                    if (lane == i) outR = make_uint2(oxy, (uint32_t)oz);
+                }
+                row_pass_w<DIM, S, 1, -1, NoDiag>(P, NoDiag{}, cw, none, par, wr);
+                if (sides) {
+                    const uint32_t oxy = __shfl_sync(0xFFFFFFFFu, P.xy[0], 0);
+                    const int oz = DIM == 3 ? __shfl_sync(0xFFFFFFFFu, P.z[0], 0) : 0;
+                    if (lane == i) outL = make_uint2(oxy, (uint32_t)oz);
                 }
             }
+            if (DIM == 3 || down) T.put(q, P);
+            if (cmp_d) {
+                if (differs(rc, ao, P)) bits |= kChgDown;
+                unsigned char* db = static_cast<unsigned char*>(p.DB[vn]);
+                io.put_cells(db + (((long long)z * p.nc + c) * w + xw) * IO::kCell, P);
+            }
+            if (!down) {
+                if (cmp_u && differs(rc, ao, P)) bits |= (last ? kChgLast : 0) | (q == 0 ? kChgFirst : 0);
+                io.put_cells(static_cast<unsigned char*>(p.V[vn]) + cell_at(z, y), P);
+            }
+            if (sides && i == L && !last) load_sides(j + 1);
+            if (i == 2 * L - 1 && !last) first_rows(j + 1);
+        }
+        if (sides && lane < 2 * L) {
+            const long long at = side_at(z);
+            auto post = [&](uint2* const (&x)[2], const uint2& v) -> bool {
+                const uint2 o = vo == 2 ? kNoCell : __ldcg(x[vo == 1 ? 1 : 0] + at);
+                x[vn][at] = v;
+                return o.x != v.x || o.y != v.y;
+            };
+            if (xb + 1 < p.nx && post(p.XR, outR)) bits |= kChgRight;
+            if (xb > 0 && post(p.XL, outL)) bits |= kChgLeft;
         }
     }
-    if (bits) atomicOr(s_chg, bits);
-    __syncthreads();
+    __syncwarp();   // every lane's stores, before the state word that shows them
+    if (lane == 0) __stcg(p.state + b, block_state(round, vn, vo));
+    return bits;
 }
 
-// T threads per CTA (a multiple of 32 covering the row's segments); the
-// register budget allows 512 / T * ... CTAs: 128 registers a thread
-template <class Cell, int kDim, int S, int T>
-__global__ void __launch_bounds__(T, 512 / T) k_dan_blocks(DanBlk p)
+constexpr int kBlkWarps = 4;   // per CTA, each taking blocks by itself
+
+template <int DIM, int S>
+__global__ void __launch_bounds__(32 * kBlkWarps, 4) k_dan_blocks(DanBlk p)
 {
-    __shared__ ScanShared<Cell, T> sh;
-    __shared__ int s_item, s_chg;
-    const int t = threadIdx.x;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31;
+    unsigned char* mine = smem_raw + (threadIdx.x >> 5) * dan_warp_bytes<DIM, S>(p.R);
+    BlockRows<DIM, S> T;
+    T.c = reinterpret_cast<uint32_t*>(mine + BlockIO<DIM, S>::kBytes);
+    if constexpr (DIM == 3) T.zz = reinterpret_cast<int16_t*>(T.c + p.R * S * 32);
+    const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    const int warps = (int)((gridDim.x * blockDim.x) >> 5);
+    const bool own = p.nblocks <= warps;   // a warp per block: no lists
+    unsigned passed = 0;
     int round = 0;
     for (;; round++) {
-        const int cur = round & 1;
+        const int cur = round & 1, r3 = round % 3, n3 = (round + 1) % 3;
         if (round >= p.max_rounds) {
-            if (blockIdx.x == 0 && t == 0) atomicExch(p.err, 3);
+            if (blockIdx.x == 0 && threadIdx.x == 0) atomicExch(p.err, 3);
             return;
         }
-        const unsigned nwork = __ldcg(p.ctl + cur);
-        const int* wl = p.wl[cur];
-        int* wln = p.wl[cur ^ 1];
-        for (;;) {
-            if (t == 0) {
-                s_item = (int)atomicAdd(p.ctl + 2, 1u);
-                s_chg = 0;
+        const unsigned nwork = own || round == 0 ? (unsigned)p.nblocks : __ldcg(p.ctl + (round + 2) % 3);
+        for (bool first = true;; first = false) {
+            int b;
+            if (own) {
+                if (!first || warp >= p.nblocks || (round > 0 && __ldcg(p.dirty[cur] + warp) == 0)) break;
+                b = warp;
+                if (lane == 0) p.dirty[cur][b] = 0;
+            } else {
+                unsigned it = 0;
+                if (lane == 0) it = atomicAdd(p.ctl + 3 + r3, 1u);
+                it = __shfl_sync(0xFFFFFFFFu, it, 0);
+                if (it >= nwork) break;
+                b = round == 0 ? (int)it : __ldcg(p.wl[cur] + it);
             }
-            __syncthreads();
-            const unsigned it = (unsigned)s_item;
-            if (it >= nwork) break;
-            const int b = __ldcg(wl + it);
-            dan_block<Cell, kDim, S, T>(p, b, sh, &s_chg);   // ends with a barrier
-            if (t == 0) {
-                const int bits = s_chg;
-                p.chg[b] = (uint8_t)bits;
-                if (bits) {
-                    const int k = b / p.nc;
-                    const int c = b - k * p.nc;
-                    auto queue = [&](int dep) {
-                        if (atomicMax(p.stamp + dep, round + 1) < round + 1)
-                            wln[atomicAdd(p.ctl + (cur ^ 1), 1u)] = dep;
-                    };
-                    if ((bits & kChgLast) && k + 1 < p.nk) queue(b + p.nc);
-                    if ((bits & kChgFirst) && c > 0) queue(b - 1);
-                    if ((bits & kChgDown) && c + 1 < p.nc) queue(b + 1);
+            const int xb = b % p.nx;
+            const BlockIO<DIM, S> io{mine, min(32 * S, p.w - xb * 32 * S)};
+            const unsigned bits = __reduce_or_sync(0xFFFFFFFFu, (unsigned)dan_block<DIM, S>(p, b, round, io, T));
+            if (lane < 5 && ((bits >> lane) & 1u)) {   // lane i queues the dependent of bit i
+                const int k = b / p.nx / p.nc, c = b / p.nx - k * p.nc;
+                int dep = -1;
+                if (lane == 0 && k + 1 < p.nk) dep = b + p.nc * p.nx;
+                if (lane == 1 && c > 0) dep = b - p.nx;
+                if (lane == 2 && c + 1 < p.nc) dep = b + p.nx;
+                if (lane == 3 && xb + 1 < p.nx) dep = b + 1;
+                if (lane == 4 && xb > 0) dep = b - 1;
+                if (dep >= 0) {
+                    if (own) {
+                        p.dirty[cur ^ 1][dep] = 1;
+                        __stcg(p.ctl + r3, 1u);
+                    } else if (atomicMax(p.stamp + dep, round + 1) < round + 1) {
+                        p.wl[cur ^ 1][atomicAdd(p.ctl + r3, 1u)] = dep;
+                    }
                 }
             }
-            __syncthreads();   // s_item / s_chg are rewritten by the next take
+            __syncwarp();
         }
-        if (!grid_barrier(p.ctl + 3, p.ctl + 4, p.err, kGridWaitNs)) return;
-        // commit: blocks whose output changed now hold it in the other version
-        for (unsigned i = blockIdx.x * blockDim.x + t; i < nwork; i += gridDim.x * blockDim.x) {
-            const int b = __ldcg(wl + i);
-            if (__ldcg(p.chg + b) & kChgAny) p.lat[b] = __ldcg(p.lat + b) == 0 ? 1 : 0;
+        if (blockIdx.x == 0 && threadIdx.x == 0) {   // the next round's words: last read two barriers ago
+            __stcg(p.ctl + n3, 0u);
+            __stcg(p.ctl + 3 + n3, 0u);
         }
-        if (blockIdx.x == 0 && t == 0) {
-            p.ctl[2] = 0;
-            p.ctl[cur] = 0;
-        }
-        if (!grid_barrier(p.ctl + 3, p.ctl + 4, p.err, kGridWaitNs)) return;
-        if (__ldcg(p.ctl + (cur ^ 1)) == 0) break;
+        if (!grid_barrier(p.ctl + 6, passed, p.err)) return;
+        if (__ldcg(p.ctl + r3) == 0) break;
     }
-    if (blockIdx.x == 0 && t == 0) p.ctl[5] = (unsigned)(round + 1);
+    if (blockIdx.x == 0 && threadIdx.x == 0) p.ctl[7] = (unsigned)(round + 1);
 }
 
-// every block takes its rows from the input, and all are queued
+// every block takes its rows from the input; the first round runs all
 __global__ void k_dan_blocks_init(DanBlk p)
 {
     for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < p.nblocks; b += gridDim.x * blockDim.x) {
-        p.lat[b] = 2;
-        p.chg[b] = 0;
+        p.state[b] = (2u << 2) | 2u;
+        p.dirty[0][b] = 0;
+        p.dirty[1][b] = 0;
         p.stamp[b] = 0;
-        p.wl[0][b] = b;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        p.ctl[0] = (unsigned)p.nblocks;
-        for (int i = 1; i < 8; i++) p.ctl[i] = 0;
-    }
+    if (blockIdx.x == 0 && threadIdx.x < 8) p.ctl[threadIdx.x] = 0;
 }
 
-// the converged outputs back into the caller's array
-template <class Cell>
-__global__ void k_dan_blocks_store(DanBlk p, typename CellIO<Cell>::P* __restrict__ dl)
+// the converged outputs back into the caller's array, by 16-bit halves: kCell
+// of them per cell, x blocks of bx cells
+template <int kCell>
+__global__ void k_dan_blocks_store(DanBlk p, uint16_t* __restrict__ dl, int bx)
 {
-    using IO = CellIO<Cell>;
-    using P = typename IO::P;
-    const long long plane = (long long)p.w * p.h, cells = plane * p.d;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < cells;
-         i += (long long)gridDim.x * blockDim.x) {
-        const int z = (int)(i / plane);
-        const int y = (int)((i - z * plane) / p.w);
+    const long long row_halves = (long long)p.w * kCell;
+    const long long rows = (long long)p.h * p.d;
+    for (long long r = blockIdx.x; r < rows; r += gridDim.x) {
+        const int z = (int)(r / p.h), y = (int)(r - (long long)z * p.h);
         const int pos = (z - p.zfirst) * p.dir;
         if (pos < 0 || pos >= p.nchain) continue;   // the fixed slice
-        const int v = p.lat[(pos / p.Z) * p.nc + y / p.R];
-        if (v != 2) {
-            const P* src = static_cast<const P*>(p.V[v]);
-#pragma unroll
-            for (int k = 0; k < IO::kWords; k++) dl[IO::kWords * i + k] = src[IO::kWords * i + k];
+        const unsigned* state = p.state + ((pos / p.Z) * p.nc + y / p.R) * p.nx;
+        const uint16_t* s0 = static_cast<const uint16_t*>(p.V[0]) + r * row_halves;
+        const uint16_t* s1 = static_cast<const uint16_t*>(p.V[1]) + r * row_halves;
+        uint16_t* dst = dl + r * row_halves;
+        const int span = bx * kCell;   // a multiple of 64 halves
+        if ((((uintptr_t)s0 | (uintptr_t)s1 | (uintptr_t)dst) & 15) == 0 && row_halves % 8 == 0) {
+            for (int i = threadIdx.x; i < row_halves / 8; i += blockDim.x)
+                reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(state[8 * i / span] >> 2 & 1u ? s1 : s0)[i];
+        } else {
+            for (int i = threadIdx.x; i < row_halves; i += blockDim.x) dst[i] = (state[i / span] >> 2 & 1u ? s1 : s0)[i];
         }
     }
 }
@@ -376,122 +484,156 @@ static size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 int dan_blocks_rows(int dim, int w, int h, int d)
 {
     const int tv = tune_get(kTuneDanRows, w);
-    if (tv > 0) return tv;
-    // small images: the serial engine's launch is cheaper than the rounds
+    if (tv > 0) return tv >= kDanSerial ? kDanSerial : min(tv, kBlkMaxRows);
+    // tiny fields: the serial engine's launch is cheaper than the rounds
     const long long cells = (long long)w * h * (dim == 3 ? d : 1);
-    if (cells < 65536 || w > 8 * kBlkThreads) return kDanSerial;
-    return 8;
+    if (cells < 1024 || w > kBlkMaxWidth) return kDanSerial;
+    // 8 rows; tall images of several x blocks 16 (1024^2, 100 points: 0.51
+    // against 0.62 ms; 501 x 700 noise: 0.53 against 0.43); volumes whose
+    // blocks of 4 rows do not outnumber the resident warps by much 4 (101 x 77
+    // x 90: 1.6 against 2.0 ms; 256^3: 9.3 against 8.8)
+    if (dim == 2) return w > 256 && h >= 1024 ? 16 : 8;
+    return cells <= (1 << 21) ? 4 : 8;
+}
+
+// Cells per lane.  Images of at most 256 columns take one x block (250 x 180
+// noise: 0.22 ms, 0.27 as two), wider ones blocks of 128 (1024^2, 100 points:
+// 0.51 ms, 0.64 with 256); volumes blocks of 64 (256^3 boxes and spheres: 8.8
+// ms, 9.4 with 128 and 11.8 with 256), from 512 columns on 128.
+static int dan_blocks_s(int dim, int w)
+{
+    int s = tune_get(dim == 2 ? kTuneDan2 : kTuneDan3, w);
+    if (s != 2 && s != 4 && s != 8) {
+        if (dim == 2) s = w <= 64 ? 2 : (w <= 128 ? 4 : (w <= 256 ? 8 : 4));
+        else s = w < 512 ? 2 : 4;
+    }
+    return s;
+}
+
+// bytes of the pieces of the workspace
+struct DanSizes {
+    size_t field, down, side, flag, list, total;
+};
+static DanSizes dan_sizes(int dim, int w, int h, int d, int R)
+{
+    const size_t cb = dim == 3 ? 6 : 4;
+    const size_t nd = dim == 3 ? d : 1;
+    const int bx = 32 * dan_blocks_s(dim, w);
+    const size_t nc = (h + R - 1) / R, nx = (w + bx - 1) / bx;
+    DanSizes z;
+    z.field = al256((size_t)w * h * nd * cb);
+    z.down = al256(nc * nd * w * cb);
+    z.side = nx > 1 ? al256(nd * h * 2 * nx * sizeof(uint2)) : 0;
+    z.flag = al256(nc * nd * nx);
+    z.list = al256(nc * nd * nx * sizeof(int));
+    z.total = 2 * z.field + 2 * z.down + 4 * z.side + 2 * z.flag + 4 * z.list + 256;
+    return z;
 }
 
 size_t dan_blocks_workspace_bytes(int dim, int w, int h, int d, int R)
 {
-    const size_t cb = dim == 3 ? 6 : 4;
-    const size_t cells = (size_t)w * h * (dim == 3 ? d : 1);
-    const int nc = (h + R - 1) / R;
-    const size_t nb = (size_t)nc * (dim == 3 ? d : 1);
-    return 2 * al256(cells * cb) + 2 * al256(nb * w * cb) + 2 * al256(nb) + 3 * al256(nb * sizeof(int)) + 256;
+    return dan_sizes(dim, w, h, d, min(R, kBlkMaxRows)).total;
 }
 
-template <class Cell, int kDim, int S, int T>
+template <int kDim, int S>
 static bool run_phase(DanBlk& p, void* dl, cudaStream_t st)
 {
+    auto kern = k_dan_blocks<kDim, S>;
+    const size_t warp_bytes = dan_warp_bytes<kDim, S>(p.R);
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kBlkWarps * warp_bytes));
+    cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dan_blocks<Cell, kDim, S, T>, T, 0) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kBlkWarps, kBlkWarps * warp_bytes) !=
             cudaSuccess ||
         per_sm < 1)
         return false;
-    const int resident = per_sm * g_num_sms;
-    // slices per block: long enough that few rounds are needed, short enough
-    // that about four block columns per resident CTA keep every SM busy, and
-    // at most 16 (on 1024^3 noise, 16 slices ran 686 -> 553 ms against the
-    // 110 the column rule gives; 32 and 64 were slower than 16)
+    const int resident = per_sm * g_num_sms * kBlkWarps;   // warps
+    // slices per block: 2 while that gives at most two blocks per resident warp
+    // (101 x 77 x 90: 1.6 ms, 1.8 with 4), else 4, more where there would be
+    // over 8 blocks per resident warp, at most 16
     int Z = tune_get(kTuneDanSlices, p.w);
     if (Z < 1) {
-        const long long cols = 4LL * resident;
-        Z = (int)((long long)p.nchain * p.nc / cols);
-        if (Z < 1) Z = 1;
-        if (Z > 16) Z = 16;
+        Z = (int)((long long)p.nchain * p.nc * p.nx / (8LL * resident));
+        const bool few = (long long)p.nchain * p.nc * p.nx <= 4LL * resident;
+        Z = max(few ? 2 : 4, min(Z, 16));
     }
     if (Z > p.nchain) Z = p.nchain;
     p.Z = Z;
     p.nk = (p.nchain + Z - 1) / Z;
-    p.nblocks = p.nk * p.nc;
-    p.max_rounds = 2 * p.nblocks + 8;
-    k_dan_blocks_init<<<(p.nblocks + 255) / 256, 256, 0, st>>>(p);
-    int grid = resident < p.nblocks ? resident : p.nblocks;
+    p.nblocks = p.nk * p.nc * p.nx;
+    p.max_rounds = 4 * p.nblocks + 8;
+    k_dan_blocks_init<<<min((p.nblocks + 255) / 256, g_num_sms * 8), 256, 0, st>>>(p);
+    // a warp per CTA while that spreads the blocks over more SMs
+    const int warps = p.nblocks <= 2 * g_num_sms ? 1 : kBlkWarps;
+    const int ctas = (p.nblocks + warps - 1) / warps;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(T);
+    cfg.gridDim = dim3(min(per_sm * g_num_sms, ctas));
+    cfg.blockDim = dim3(32 * warps);
+    cfg.dynamicSmemBytes = warps * warp_bytes;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, k_dan_blocks<Cell, kDim, S, T>, p) != cudaSuccess) return false;
-    const long long cells = (long long)p.w * p.h * p.d;
-    long long gb = (cells + 255) / 256;
+    if (cudaLaunchKernelEx(&cfg, kern, p) != cudaSuccess) return false;
+    long long gb = (long long)p.h * p.d;
     if (gb > (long long)g_num_sms * 32) gb = (long long)g_num_sms * 32;
-    k_dan_blocks_store<Cell><<<(int)gb, 256, 0, st>>>(p, static_cast<typename CellIO<Cell>::P*>(dl));
+    k_dan_blocks_store<kDim == 3 ? 3 : 2>
+        <<<(int)gb, p.w >= 128 ? 256 : 64, 0, st>>>(p, static_cast<uint16_t*>(dl), 32 * S);
     return true;
 }
 
-template <class Cell, int kDim, int S, int T>
+template <int kDim, int S>
 static bool run_all(int w, int h, int d, int cw, int R, void* deltas, void* ws, int* err, cudaStream_t st)
 {
-    const size_t cb = kDim == 3 ? 6 : 4;
-    const size_t cells = (size_t)w * h * d;
-    const int nc = (h + R - 1) / R;
-    const int nb = nc * d;   // (slice, chunk) pairs: down-boundary row slots, and a bound on the blocks
+    const DanSizes z = dan_sizes(kDim, w, h, d, R);
     char* q = static_cast<char*>(ws);
+    auto take = [&](size_t bytes) {
+        char* r = q;
+        q += bytes;
+        return r;
+    };
     DanBlk p{};
     p.A = deltas;
-    p.V[0] = q;
-    q += al256(cells * cb);
-    p.V[1] = q;
-    q += al256(cells * cb);
-    p.DB[0] = q;
-    q += al256((size_t)nb * w * cb);
-    p.DB[1] = q;
-    q += al256((size_t)nb * w * cb);
-    p.lat = reinterpret_cast<uint8_t*>(q);
-    q += al256(nb);
-    p.chg = reinterpret_cast<uint8_t*>(q);
-    q += al256(nb);
-    p.stamp = reinterpret_cast<int*>(q);
-    q += al256((size_t)nb * sizeof(int));
-    p.wl[0] = reinterpret_cast<int*>(q);
-    q += al256((size_t)nb * sizeof(int));
-    p.wl[1] = reinterpret_cast<int*>(q);
-    q += al256((size_t)nb * sizeof(int));
+    for (int v = 0; v < 2; v++) p.V[v] = take(z.field);
+    for (int v = 0; v < 2; v++) p.DB[v] = take(z.down);
+    for (int v = 0; v < 2; v++) p.XR[v] = reinterpret_cast<uint2*>(take(z.side));
+    for (int v = 0; v < 2; v++) p.XL[v] = reinterpret_cast<uint2*>(take(z.side));
+    p.state = reinterpret_cast<unsigned*>(take(z.list));
+    for (int v = 0; v < 2; v++) p.dirty[v] = reinterpret_cast<uint8_t*>(take(z.flag));
+    p.stamp = reinterpret_cast<int*>(take(z.list));
+    p.wl[0] = reinterpret_cast<int*>(take(z.list));
+    p.wl[1] = reinterpret_cast<int*>(take(z.list));
     p.ctl = reinterpret_cast<unsigned*>(q);
     p.err = err;
     p.w = w;
     p.h = h;
     p.d = d;
     p.R = R;
-    p.nc = nc;
+    p.nc = (h + R - 1) / R;
+    p.nx = (w + 32 * S - 1) / (32 * S);
     p.cw = cw;
     if (kDim == 2) {
         p.dir = 1;
         p.zfirst = 0;
         p.nchain = 1;
-        return run_phase<Cell, kDim, S, T>(p, deltas, st);
+        return run_phase<kDim, S>(p, deltas, st);
     }
     // slices 1..d-1 pull from the slice before, then d-2..0 from the slice after
     p.dir = 1;
     p.zfirst = 1;
     p.nchain = d - 1;
-    if (!run_phase<Cell, kDim, S, T>(p, deltas, st)) return false;
+    if (!run_phase<kDim, S>(p, deltas, st)) return false;
     p.dir = -1;
     p.zfirst = d - 2;
-    return run_phase<Cell, kDim, S, T>(p, deltas, st);
+    return run_phase<kDim, S>(p, deltas, st);
 }
 
 size_t danielsson_workspace_bytes(int dim, int w, int h, int d)
 {
     const int R = dan_blocks_rows(dim, w, h, d);
-    if (R >= kDanSerial || w > 8 * kBlkThreads) return 0;
+    if (R >= kDanSerial || w > kBlkMaxWidth) return 0;
     return dan_blocks_workspace_bytes(dim, w, h, d, R);
 }
 
@@ -510,41 +652,20 @@ bool launch_danielsson_blocks(int dim, void* deltas, int w, int h, int d, int cw
                               cudaStream_t st)
 {
     if (dim == 3 && d < 2) return true;   // the reference's slice loops do not run
+    if (w > kBlkMaxWidth) return false;
+    R = min(R, kBlkMaxRows);
     ProfScope ps("danielsson_blocks", st);
-    // cells per thread: tuned, else the fewest that keep the row within 128
-    // threads in 3D (short segments, CTAs of 2-4 warps, many blocks per SM;
-    // cells stop at 4 per thread, where the register file still holds every
-    // array) and within 256 in 2D, where an image has fewer blocks than the
-    // GPU has SMs and the widest CTA finishes a block soonest (1024^2, 100
-    // points: 1.96 ms at 128 threads, 1.37 ms at 256)
-    int s = tune_get(dim == 2 ? kTuneDan2 : kTuneDan3, w);
-    if (s != 1 && s != 2 && s != 4 && s != 8) {
-        const int tmax = dim == 2 ? kBlkThreads : 128;
-        s = 1;
-        while ((w + s - 1) / s > tmax && s < (dim == 3 ? 4 : 8)) s *= 2;
+    switch (dan_blocks_s(dim, w)) {
+        case 2:
+            return dim == 2 ? run_all<2, 2>(w, h, 1, cw, R, deltas, ws, err, st)
+                            : run_all<3, 2>(w, h, d, cw, R, deltas, ws, err, st);
+        case 4:
+            return dim == 2 ? run_all<2, 4>(w, h, 1, cw, R, deltas, ws, err, st)
+                            : run_all<3, 4>(w, h, d, cw, R, deltas, ws, err, st);
+        default:
+            return dim == 2 ? run_all<2, 8>(w, h, 1, cw, R, deltas, ws, err, st)
+                            : run_all<3, 8>(w, h, d, cw, R, deltas, ws, err, st);
     }
-    while ((w + s - 1) / s > kBlkThreads && s < 8) s *= 2;
-    const int nseg = (w + s - 1) / s;
-    if (nseg > kBlkThreads) return false;
-    const int t = nseg <= 64 ? 64 : (nseg <= 128 ? 128 : 256);
-#define DOL_BLK_RUN(SV, TV)                                                                             \
-    return dim == 2 ? run_all<C2, 2, SV, TV>(w, h, 1, cw, R, deltas, ws, err, st)                     \
-                    : run_all<C3, 3, SV, TV>(w, h, d, cw, R, deltas, ws, err, st);
-#define DOL_BLK_CASE(SV)                                                                                \
-    case SV:                                                                                            \
-        if (t == 64) { DOL_BLK_RUN(SV, 64) }                                                            \
-        if (t == 128) { DOL_BLK_RUN(SV, 128) }                                                          \
-        DOL_BLK_RUN(SV, 256)
-    switch (s) {
-        DOL_BLK_CASE(1)
-        DOL_BLK_CASE(2)
-        DOL_BLK_CASE(4)
-        DOL_BLK_CASE(8)
-        default: break;
-    }
-#undef DOL_BLK_CASE
-#undef DOL_BLK_RUN
-    return false;
 }
 
 }  // namespace dolk

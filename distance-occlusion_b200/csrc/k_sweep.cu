@@ -2,11 +2,12 @@
 //
 // Danielsson (DistanceOcclusionLib.cpp:702-778 2D, :2264-2394 3D) and FastSweep
 // 2D (:633-697) are serial in the sweep axis: every row needs the whole
-// previous row.  One CTA walks the rows of an image (or the slices and rows of
-// a volume); each thread keeps S consecutive cells of the current and previous
-// row in registers, so the vertical (and z) pulls are thread-local and only the
-// x passes talk across threads (row_pass in scan.cuh, exact).  The next row is
-// loaded while the current one is scanned.
+// previous row.  One group of warps walks the rows of an image (or the slices
+// and rows of a volume); a lane keeps S consecutive cells of the row in
+// registers, so the vertical (and z) pulls are lane-local and only the x
+// passes talk across lanes (row.cuh, exact).  The next row is loaded while the
+// current one is scanned.  A row of up to 256 cells is one warp's (nothing
+// crosses a barrier), wider rows take one warp per 256 cells.
 //
 // FastSweep 3D (:2186-2260) has more parallelism: row (y, z) of an octant
 // sweep needs only row (y-1, z) and row (y, z-1) of the same sweep, so rows on
@@ -17,6 +18,8 @@
 // the earliest unfinished row can always proceed.
 #include <limits.h>
 
+#include "dan_serial.cuh"
+#include "dan_slices.cuh"
 #include "kernels.h"
 #include "scan.cuh"
 
@@ -45,241 +48,98 @@ __device__ __forceinline__ C3 cell_load_cg(const int16_t* p, long long i)
     return C3{__ldcg(c), __ldcg(c + 1), __ldcg(c + 2)};
 }
 
-// ------------------------------------------------------------ Danielsson 2D ----
-// Rows 1..h-1 going down, then h-2..0 going up (:709-777): one "step" per row,
-// the row taking the previous step's row with a y offset of -cw (down) or
-// +cw (up), then an x pass to the right and one to the left.  The next step's
-// row is loaded during the current one, and each pass posts what the next
-// pass needs (row_pass), so a step costs two barriers when the passes settle
-// in one round.
+// ------------------------------------------------------------ Danielsson ----
 
-// One CTA runs the whole 2D Danielsson of one image (used by the single-image
-// kernel and by the batched kernel).
-template <int S>
-__device__ __forceinline__ void danielsson2_cta(uint32_t* __restrict__ dl, int w, int h, int cw, ScanShared<C2>& sh)
+template <int DIM, int S, int NW>
+__global__ void __launch_bounds__(32 * NW) k_dan_serial(void* __restrict__ dl, int w, int h, int d, int cw)
 {
-    const int t = threadIdx.x;
-    const int nseg = (w + S - 1) / S;
-    const bool active = t < nseg;
-    const int n = active ? min(S, w - t * S) : 0;
-    const long long x0 = (long long)t * S;
-    if (h < 2) return;
-    const int steps = 2 * (h - 1);
-    auto row_of = [&](int i) { return i < h - 1 ? i + 1 : 2 * h - 3 - i; };
-    auto dy_of = [&](int i) { return i < h - 1 ? -cw : cw; };
-    C2 P[S], C[S], V[S], R[S], D[S];
-#pragma unroll
-    for (int s = 0; s < S; s++) P[s] = C[s] = V[s] = R[s] = D[s] = C2{0, 0};
-
-    load_row<C2, S>(P, dl, x0, n);
-    load_row<C2, S>(C, dl, (long long)row_of(0) * w + x0, n);
-#pragma unroll
-    for (int s = 0; s < S; s++) V[s] = closer(C[s], add(P[s], 0, dy_of(0)));
-    int g = 0;
-    if (active) sh.guess[g][t] = seg_edge<C2, S, +1>(V, n);
-    __syncthreads();
-    for (int i = 0; i < steps; i++) {
-        const int y = row_of(i);
-        const bool more = i + 1 < steps;
-        const int dyn = more ? dy_of(i + 1) : 0;
-        if (more) load_row<C2, S>(C, dl, (long long)row_of(i + 1) * w + x0, n);
-        const C2 in0 = (active && t > 0) ? sh.guess[g][t - 1] : V[0];
-        row_pass<C2, S, false, +1>(R, V, t, nseg, n, cw, sh, D, in0, [&](const C2 (&X)[S]) {
-            if (active) sh.guess[g ^ 1][t] = X[0];
-        });
-        g ^= 1;
-        const C2 in1 = (active && t + 1 < nseg) ? sh.guess[g][t + 1] : R[0];
-        row_pass<C2, S, false, -1>(P, R, t, nseg, n, cw, sh, D, in1, [&](const C2 (&X)[S]) {
-            if (more && active)
-                sh.guess[g ^ 1][t] = closer(seg_edge<C2, S, +1>(C, n), add(seg_edge<C2, S, +1>(X, n), 0, dyn));
-        });
-        g ^= 1;
-        store_row<C2, S>(dl, (long long)y * w + x0, P, n);
-        if (more) {
-#pragma unroll
-            for (int s = 0; s < S; s++) V[s] = closer(C[s], add(P[s], 0, dyn));
-        }
+    extern __shared__ __align__(16) unsigned char strips[];
+    __shared__ RowShared<NW> sh;
+    if constexpr (NW > 1) {
+        if (threadIdx.x == 0) sh.bar = 0;
+        __syncthreads();
     }
-}
-
-template <int S>
-__global__ void __launch_bounds__(512) k_danielsson2(uint32_t* __restrict__ dl, int w, int h, int cw)
-{
-    __shared__ ScanShared<C2> sh;
-    danielsson2_cta<S>(dl, w, h, cw, sh);
-}
-
-// ------------------------------------------------------------ Danielsson 3D ----
-// Slices 1..d-1 then d-2..0 (:2355-2393); each slice takes the neighbouring
-// slice's cell with the z offset, then runs the 2D steps over its rows
-// (:2264-2345).  The z pull is folded into the first load of each row (rows of
-// the down sweep); the up sweep reads the down sweep's results.
-
-template <int S>
-__device__ __forceinline__ void danielsson3_cta(int16_t* __restrict__ dl, int w, int h, int d, int cw,
-                                                ScanShared<C3>& sh)
-{
-    const int t = threadIdx.x;
-    const int nseg = (w + S - 1) / S;
-    const bool active = t < nseg;
-    const int n = active ? min(S, w - t * S) : 0;
-    const long long x0 = (long long)t * S;
-    const long long plane = (long long)w * h;
-    const int steps = 2 * (h - 1);
-    auto row_of = [&](int i) { return i < h - 1 ? i + 1 : 2 * h - 3 - i; };
-    auto dy_of = [&](int i) { return i < h - 1 ? -cw : cw; };
-    C3 P[S], C[S], Q[S], V[S], R[S], D[S];
-#pragma unroll
-    for (int s = 0; s < S; s++) P[s] = C[s] = Q[s] = V[s] = R[s] = D[s] = C3{0, 0, 0};
-
-    for (int pass = 0; pass < 2; pass++) {
-        const int dz = pass == 0 ? -cw : +cw;
-        for (int k = 1; k < d; k++) {
-            const int z = pass == 0 ? k : d - 1 - k;
-            const int zp = pass == 0 ? z - 1 : z + 1;
-            const long long sb = z * plane, pb = (long long)zp * plane;
-            // row 0: z pull only
-            load_row<C3, S>(C, dl, sb + x0, n);
-            load_row<C3, S>(Q, dl, pb + x0, n);
-#pragma unroll
-            for (int s = 0; s < S; s++) P[s] = closer(C[s], add(Q[s], 0, 0, dz));
-            store_row<C3, S>(dl, sb + x0, P, n);
-            if (h < 2) continue;
-            // first step: row 1 of the down sweep (z pull, then y pull)
-            load_row<C3, S>(C, dl, sb + (long long)w + x0, n);
-            load_row<C3, S>(Q, dl, pb + (long long)w + x0, n);
-#pragma unroll
-            for (int s = 0; s < S; s++) V[s] = closer(closer(C[s], add(Q[s], 0, 0, dz)), add(P[s], 0, -cw, 0));
-            int g = 0;
-            __syncthreads();   // the previous slice's last pass may still read the guess slots
-            if (active) sh.guess[g][t] = seg_edge<C3, S, +1>(V, n);
-            __syncthreads();
-            for (int i = 0; i < steps; i++) {
-                const int y = row_of(i);
-                const bool more = i + 1 < steps;
-                const bool next_down = more && i + 1 < h - 1;
-                const int dyn = more ? dy_of(i + 1) : 0;
-                if (more) {
-                    const long long off = (long long)row_of(i + 1) * w + x0;
-                    load_row<C3, S>(C, dl, sb + off, n);
-                    if (next_down) load_row<C3, S>(Q, dl, pb + off, n);
-                }
-                const C3 in0 = (active && t > 0) ? sh.guess[g][t - 1] : V[0];
-                row_pass<C3, S, false, +1>(R, V, t, nseg, n, cw, sh, D, in0, [&](const C3 (&X)[S]) {
-                    if (active) sh.guess[g ^ 1][t] = X[0];
-                });
-                g ^= 1;
-                const C3 in1 = (active && t + 1 < nseg) ? sh.guess[g][t + 1] : R[0];
-                row_pass<C3, S, false, -1>(P, R, t, nseg, n, cw, sh, D, in1, [&](const C3 (&X)[S]) {
-                    if (more && active) {
-                        C3 c = seg_edge<C3, S, +1>(C, n);
-                        if (next_down) c = closer(c, add(seg_edge<C3, S, +1>(Q, n), 0, 0, dz));
-                        sh.guess[g ^ 1][t] = closer(c, add(seg_edge<C3, S, +1>(X, n), 0, dyn, 0));
-                    }
-                });
-                g ^= 1;
-                store_row<C3, S>(dl, sb + (long long)y * w + x0, P, n);
-                if (more) {
-#pragma unroll
-                    for (int s = 0; s < S; s++) {
-                        C3 c = next_down ? closer(C[s], add(Q[s], 0, 0, dz)) : C[s];
-                        V[s] = closer(c, add(P[s], 0, dyn, 0));
-                    }
-                }
-            }
-        }
-    }
-}
-
-template <int S>
-__global__ void __launch_bounds__(512) k_danielsson3(int16_t* __restrict__ dl, int w, int h, int d, int cw)
-{
-    __shared__ ScanShared<C3> sh;
-    danielsson3_cta<S>(dl, w, h, d, cw, sh);
+    dan_serial<DIM, S, NW>(dl, w, h, d, cw, strips + (NW > 1 ? threadIdx.x >> 5 : 0) * SerialIO<DIM, S>::kBytes, sh);
 }
 
 // ------------------------------------------------------------- FastSweep 2D ----
 // Four quadrant sweeps; the first row of each sweep is left as is; each later
 // row takes the previous row's cell, then along x the previous cell of the row
 // and the diagonal cell of the previous row, in that order (:655-693).  The
-// diagonal candidate of a segment's first cell is its predecessor's boundary
-// cell of the previous row, posted during the previous row's pass.
+// diagonal candidate of a lane's first cell is its predecessor's edge cell of
+// the previous row: a shuffle inside the warp, shared memory across warps.
 
-template <int S>
-__global__ void __launch_bounds__(512) k_fastsweep2(uint32_t* __restrict__ dl, int w, int h, int cw)
+template <int S, int NW, int DX>
+__device__ __forceinline__ void fastsweep2_sweep(const Field<2, S>& f, const SerialIO<2, S>& io, int dy, int cw,
+                                                 RowShared<NW>& sh, int& par, uint32_t (*edge)[NW])
 {
-    __shared__ ScanShared<C2> sh;
-    const int t = threadIdx.x;
-    const int nseg = (w + S - 1) / S;
-    const bool active = t < nseg;
-    const int n = active ? min(S, w - t * S) : 0;
-    const long long x0 = (long long)t * S;
-    C2 P[S], C[S], V[S], R[S], D[S];
+    using Row = Cells<2, S>;
+    const int lane = threadIdx.x & 31, wi = NW > 1 ? threadIdx.x >> 5 : 0;
+    const int ox = -cw * DX, oy = -cw * dy;
+    const int y0 = dy > 0 ? 0 : f.h - 1;
+    const int x0 = f.xw + lane * S;
+    Row P, V;
+    Diag<S> D;
+    constexpr int rc = 0;   // strip of the next row
+    __syncwarp();   // the previous sweep's last rows are stored
+    io.fetch(rc, f.row(0, y0), f.lo, f.hi);
+    io.cells_of(P, rc, f.row(0, y0), cw);
+    io.fetch(rc, f.row(0, y0 + dy), f.lo, f.hi);
+    for (int j = 1; j < f.h; j++) {
+        const int y = y0 + j * dy;
+        io.cells_of(V, rc, f.row(0, y), cw);
+        if (j + 1 < f.h) io.fetch(rc, f.row(0, y + dy), f.lo, f.hi);
+        // the previous row's cell before this lane's first in scan order
+        const uint32_t mine = P.xy[DX > 0 ? S - 1 : 0];
+        uint32_t before = __shfl_sync(0xFFFFFFFFu, mine, DX > 0 ? (lane + 31) & 31 : (lane + 1) & 31);
+        if constexpr (NW > 1) {
+            if (lane == (DX > 0 ? 31 : 0)) edge[j & 1][wi] = mine;
+            __syncthreads();
+            const int pw = wi - DX;
+            if (lane == (DX > 0 ? 0 : 31) && pw >= 0 && pw < NW) before = edge[j & 1][pw];
+        }
 #pragma unroll
-    for (int s = 0; s < S; s++) P[s] = C[s] = V[s] = R[s] = D[s] = C2{0, 0};
-    if (h < 2) return;
+        for (int s = 0; s < S; s++) {
+            const uint32_t from = DX > 0 ? (s > 0 ? P.xy[s > 0 ? s - 1 : 0] : before)
+                                         : (s + 1 < S ? P.xy[s + 1 < S ? s + 1 : s] : before);
+            D.xy[s] = y_shift(from + ((uint32_t)ox << 16), oy);
+            D.W[s] = w_of<2>(D.xy[s], 0);
+            const bool has = DX > 0 ? x0 + s > 0 : x0 + s < f.w - 1;
+            D.L[s] = has ? len_of(D.xy[s], D.W[s]) : INT_MAX;
+        }
+        merge_y<2, S>(P, V, oy);
+        row_pass_w<2, S, NW, DX, Diag<S>>(P, D, cw, sh, par, chain_none(cw));
+        io.put_cells(f.row(0, y), P);
+    }
+}
 
-    for (int sweep = 0; sweep < 4; sweep++) {
-        const int dx = (sweep & 1) ? -1 : 1, dy = (sweep & 2) ? -1 : 1;
-        const int ox = -cw * dx, oy = -cw * dy;
-        const int y0 = dy > 0 ? 0 : h - 1;
-        const int pred = t - dx;   // predecessor in this sweep's scan order
-        const bool has_pred = active && pred >= 0 && pred < nseg;
-        load_row<C2, S>(P, dl, (long long)y0 * w + x0, n);
-        load_row<C2, S>(C, dl, (long long)(y0 + dy) * w + x0, n);
-#pragma unroll
-        for (int s = 0; s < S; s++) V[s] = closer(C[s], add(P[s], 0, oy));
-        int g = 0;
-        __syncthreads();   // the previous sweep's last pass may still read the slots
-        if (active) {
-            sh.guess[g][t] = dx > 0 ? seg_edge<C2, S, +1>(V, n) : seg_edge<C2, S, -1>(V, n);
-            sh.edge[g][t] = dx > 0 ? seg_edge<C2, S, +1>(P, n) : seg_edge<C2, S, -1>(P, n);
-        }
+template <int S, int NW>
+__global__ void __launch_bounds__(32 * NW) k_fastsweep2(void* __restrict__ dl, int w, int h, int cw)
+{
+    extern __shared__ __align__(16) unsigned char strips[];
+    __shared__ RowShared<NW> sh;
+    __shared__ uint32_t edge[2][NW];
+    if (h < 2) return;
+    if constexpr (NW > 1) {
+        if (threadIdx.x == 0) sh.bar = 0;
         __syncthreads();
-        for (int j = 1; j < h; j++) {
-            const int y = y0 + j * dy;
-            const bool more = j + 1 < h;
-            if (more) load_row<C2, S>(C, dl, (long long)(y + dy) * w + x0, n);
-            // diagonal candidates from the previous row (P): own cells, then the predecessor's edge
-            if (dx > 0) {
-#pragma unroll
-                for (int s = 1; s < S; s++) D[s] = add(P[s - 1], ox, oy);
-            } else {
-#pragma unroll
-                for (int s = 0; s + 1 < S; s++) D[s] = add(P[s + 1], ox, oy);
-            }
-            if (has_pred) {
-                const C2 e = add(sh.edge[g][pred], ox, oy);
-                if (dx > 0) D[0] = e;
-                else {
-#pragma unroll
-                    for (int s = 0; s < S; s++)
-                        if (s == n - 1) D[s] = e;
-                }
-            }
-            const C2 in0 = has_pred ? sh.guess[g][pred] : V[0];
-            auto post = [&](const C2 (&X)[S]) {
-                if (!active) return;
-                if (dx > 0) {
-                    sh.edge[g ^ 1][t] = seg_edge<C2, S, +1>(X, n);
-                    if (more) sh.guess[g ^ 1][t] = closer(seg_edge<C2, S, +1>(C, n), add(seg_edge<C2, S, +1>(X, n), 0, oy));
-                } else {
-                    sh.edge[g ^ 1][t] = seg_edge<C2, S, -1>(X, n);
-                    if (more) sh.guess[g ^ 1][t] = closer(seg_edge<C2, S, -1>(C, n), add(seg_edge<C2, S, -1>(X, n), 0, oy));
-                }
-            };
-            if (dx > 0)
-                row_pass<C2, S, true, +1>(R, V, t, nseg, n, cw, sh, D, in0, post);
-            else
-                row_pass<C2, S, true, -1>(R, V, t, nseg, n, cw, sh, D, in0, post);
-            g ^= 1;
-            store_row<C2, S>(dl, (long long)y * w + x0, R, n);
-#pragma unroll
-            for (int s = 0; s < S; s++) {
-                P[s] = R[s];
-                if (more) V[s] = closer(C[s], add(P[s], 0, oy));
-            }
-        }
+    }
+    const int wi = NW > 1 ? threadIdx.x >> 5 : 0;
+    Field<2, S> f;
+    f.lo = static_cast<unsigned char*>(dl);
+    f.hi = f.lo + (long long)w * h * 4;
+    f.w = w;
+    f.h = h;
+    f.xw = wi * 32 * S;
+    const SerialIO<2, S> io{strips + wi * SerialIO<2, S>::kBytes, min(32 * S, w - f.xw)};
+    int par = 0;
+    for (int sweep = 0; sweep < 4; sweep++) {
+        const int dy = (sweep & 2) ? -1 : 1;
+        if (sweep & 1)
+            fastsweep2_sweep<S, NW, -1>(f, io, dy, cw, sh, par, edge);
+        else
+            fastsweep2_sweep<S, NW, +1>(f, io, dy, cw, sh, par, edge);
+        __syncthreads();   // the edge slots are reused
     }
 }
 
@@ -482,174 +342,6 @@ __global__ void __launch_bounds__(256) k_fastsweep3_slices(int16_t* __restrict__
     }
 }
 
-// ------------------------------------------------------- single-warp engines ----
-// Rows of at most 32*S cells: one warp per image (or volume), every exchange a
-// shuffle, no shared memory and no CTA barrier (row_pass_warp).  Same steps
-// and candidate order as the CTA engines above.
-
-template <int S>
-__device__ __forceinline__ void danielsson2_warp(uint32_t* __restrict__ dl, int w, int h, int cw)
-{
-    const int lane = threadIdx.x & 31;
-    const int nseg = (w + S - 1) / S;
-    const bool active = lane < nseg;
-    const int n = active ? min(S, w - lane * S) : 0;
-    const long long x0 = (long long)lane * S;
-    if (h < 2) return;
-    const int steps = 2 * (h - 1);
-    auto row_of = [&](int i) { return i < h - 1 ? i + 1 : 2 * h - 3 - i; };
-    auto dy_of = [&](int i) { return i < h - 1 ? -cw : cw; };
-    C2 P[S], C[S], V[S], R[S], D[S];
-#pragma unroll
-    for (int s = 0; s < S; s++) P[s] = C[s] = V[s] = R[s] = D[s] = C2{0, 0};
-    load_row<C2, S>(P, dl, x0, n);
-    load_row<C2, S>(C, dl, (long long)row_of(0) * w + x0, n);
-#pragma unroll
-    for (int s = 0; s < S; s++) V[s] = closer(C[s], add(P[s], 0, dy_of(0)));
-    for (int i = 0; i < steps; i++) {
-        const int y = row_of(i);
-        const bool more = i + 1 < steps;
-        if (more) load_row<C2, S>(C, dl, (long long)row_of(i + 1) * w + x0, n);
-        row_pass_warp<C2, S, false, +1>(R, V, lane, nseg, n, cw, D, warp_round0_input<C2, S, +1>(V, n, lane));
-        row_pass_warp<C2, S, false, -1>(P, R, lane, nseg, n, cw, D, warp_round0_input<C2, S, -1>(R, n, lane));
-        store_row<C2, S>(dl, (long long)y * w + x0, P, n);
-        if (more) {
-            const int dyn = dy_of(i + 1);
-#pragma unroll
-            for (int s = 0; s < S; s++) V[s] = closer(C[s], add(P[s], 0, dyn));
-        }
-    }
-}
-
-template <int S>
-__device__ __forceinline__ void danielsson3_warp(int16_t* __restrict__ dl, int w, int h, int d, int cw)
-{
-    const int lane = threadIdx.x & 31;
-    const int nseg = (w + S - 1) / S;
-    const bool active = lane < nseg;
-    const int n = active ? min(S, w - lane * S) : 0;
-    const long long x0 = (long long)lane * S;
-    const long long plane = (long long)w * h;
-    const int steps = 2 * (h - 1);
-    auto row_of = [&](int i) { return i < h - 1 ? i + 1 : 2 * h - 3 - i; };
-    auto dy_of = [&](int i) { return i < h - 1 ? -cw : cw; };
-    C3 P[S], C[S], Q[S], V[S], R[S], D[S];
-#pragma unroll
-    for (int s = 0; s < S; s++) P[s] = C[s] = Q[s] = V[s] = R[s] = D[s] = C3{0, 0, 0};
-    for (int pass = 0; pass < 2; pass++) {
-        const int dz = pass == 0 ? -cw : +cw;
-        for (int k = 1; k < d; k++) {
-            const int z = pass == 0 ? k : d - 1 - k;
-            const int zp = pass == 0 ? z - 1 : z + 1;
-            const long long sb = z * plane, pb = (long long)zp * plane;
-            load_row<C3, S>(C, dl, sb + x0, n);
-            load_row<C3, S>(Q, dl, pb + x0, n);
-#pragma unroll
-            for (int s = 0; s < S; s++) P[s] = closer(C[s], add(Q[s], 0, 0, dz));
-            store_row<C3, S>(dl, sb + x0, P, n);
-            if (h < 2) continue;
-            load_row<C3, S>(C, dl, sb + (long long)w + x0, n);
-            load_row<C3, S>(Q, dl, pb + (long long)w + x0, n);
-#pragma unroll
-            for (int s = 0; s < S; s++) V[s] = closer(closer(C[s], add(Q[s], 0, 0, dz)), add(P[s], 0, -cw, 0));
-            for (int i = 0; i < steps; i++) {
-                const int y = row_of(i);
-                const bool more = i + 1 < steps;
-                const bool next_down = more && i + 1 < h - 1;
-                if (more) {
-                    const long long off = (long long)row_of(i + 1) * w + x0;
-                    load_row<C3, S>(C, dl, sb + off, n);
-                    if (next_down) load_row<C3, S>(Q, dl, pb + off, n);
-                }
-                row_pass_warp<C3, S, false, +1>(R, V, lane, nseg, n, cw, D, warp_round0_input<C3, S, +1>(V, n, lane));
-                row_pass_warp<C3, S, false, -1>(P, R, lane, nseg, n, cw, D, warp_round0_input<C3, S, -1>(R, n, lane));
-                store_row<C3, S>(dl, sb + (long long)y * w + x0, P, n);
-                if (more) {
-                    const int dyn = dy_of(i + 1);
-#pragma unroll
-                    for (int s = 0; s < S; s++) {
-                        C3 c = next_down ? closer(C[s], add(Q[s], 0, 0, dz)) : C[s];
-                        V[s] = closer(c, add(P[s], 0, dyn, 0));
-                    }
-                }
-            }
-        }
-    }
-}
-
-template <int S>
-__global__ void __launch_bounds__(32) k_danielsson2_w(uint32_t* __restrict__ dl, int w, int h, int cw)
-{
-    danielsson2_warp<S>(dl, w, h, cw);
-}
-
-template <int S>
-__global__ void __launch_bounds__(32) k_danielsson3_w(int16_t* __restrict__ dl, int w, int h, int d, int cw)
-{
-    danielsson3_warp<S>(dl, w, h, d, cw);
-}
-
-template <int S>
-__global__ void __launch_bounds__(32) k_fastsweep2_w(uint32_t* __restrict__ dl, int w, int h, int cw)
-{
-    const int lane = threadIdx.x & 31;
-    const int nseg = (w + S - 1) / S;
-    const bool active = lane < nseg;
-    const int n = active ? min(S, w - lane * S) : 0;
-    const long long x0 = (long long)lane * S;
-    C2 P[S], C[S], V[S], R[S], D[S];
-#pragma unroll
-    for (int s = 0; s < S; s++) P[s] = C[s] = V[s] = R[s] = D[s] = C2{0, 0};
-    if (h < 2) return;
-    for (int sweep = 0; sweep < 4; sweep++) {
-        const int dx = (sweep & 1) ? -1 : 1, dy = (sweep & 2) ? -1 : 1;
-        const int ox = -cw * dx, oy = -cw * dy;
-        const int y0 = dy > 0 ? 0 : h - 1;
-        const int pred = lane - dx;
-        const bool has_pred = active && pred >= 0 && pred < nseg;
-        const int src = pred < 0 ? 0 : (pred > 31 ? 31 : pred);
-        load_row<C2, S>(P, dl, (long long)y0 * w + x0, n);
-        load_row<C2, S>(C, dl, (long long)(y0 + dy) * w + x0, n);
-#pragma unroll
-        for (int s = 0; s < S; s++) V[s] = closer(C[s], add(P[s], 0, oy));
-        for (int j = 1; j < h; j++) {
-            const int y = y0 + j * dy;
-            const bool more = j + 1 < h;
-            if (more) load_row<C2, S>(C, dl, (long long)(y + dy) * w + x0, n);
-            // diagonal candidates from the previous row: own cells, then the predecessor's edge
-            C2 e;
-            if (dx > 0) {
-#pragma unroll
-                for (int s = 1; s < S; s++) D[s] = add(P[s - 1], ox, oy);
-                e = shfl_cell(0xFFFFFFFFu, seg_edge<C2, S, +1>(P, n), src);
-            } else {
-#pragma unroll
-                for (int s = 0; s + 1 < S; s++) D[s] = add(P[s + 1], ox, oy);
-                e = shfl_cell(0xFFFFFFFFu, seg_edge<C2, S, -1>(P, n), src);
-            }
-            if (has_pred) {
-                e = add(e, ox, oy);
-                if (dx > 0) D[0] = e;
-                else {
-#pragma unroll
-                    for (int s = 0; s < S; s++)
-                        if (s == n - 1) D[s] = e;
-                }
-            }
-            if (dx > 0)
-                row_pass_warp<C2, S, true, +1>(R, V, lane, nseg, n, cw, D, warp_round0_input<C2, S, +1>(V, n, lane));
-            else
-                row_pass_warp<C2, S, true, -1>(R, V, lane, nseg, n, cw, D, warp_round0_input<C2, S, -1>(V, n, lane));
-            store_row<C2, S>(dl, (long long)y * w + x0, R, n);
-#pragma unroll
-            for (int s = 0; s < S; s++) {
-                P[s] = R[s];
-                if (more) V[s] = closer(C[s], add(P[s], 0, oy));
-            }
-        }
-    }
-}
-
 // --------------------------------------------------------------- launchers ----
 
 // cells per thread: aim for at most 256 threads (fewer warps at every barrier),
@@ -664,108 +356,58 @@ static int pick_s(int w, int max_threads)
     return 0;
 }
 
-// the tuned cells-per-thread for this family and width, if it fits
-static int tuned_s(int kind, int w, int max_threads)
-{
-    const int v = tune_get(kind, w);
-    if ((v == 1 || v == 2 || v == 4 || v == 8) && (w + v - 1) / v <= max_threads) return v;
-    return pick_s(w, max_threads);
-}
-
 static int threads_for(int w, int s)
 {
     int n = (w + s - 1) / s;
     return ((n + 31) / 32) * 32;
 }
 
-// The single-warp engines take rows up to 32 * 16 cells (2D) / 32 * 8 (3D).
-// Tuning value kWarpEngine selects them; 1/2/4/8 select the CTA engine with
-// that many cells per thread; 0 (untuned) picks the warp engine when it fits.
-constexpr int kWarpEngine = 32;
-
-static int warp_s(int w, int max_s)
+// Cells per lane and warps of a row: 256 cells per warp, fewer per lane for
+// rows that one warp holds with fewer.  Tuning values 4 and 8 set the cells
+// per lane (any other: this rule).
+static void row_shape(int kind, int w, int* s, int* nw)
 {
-    for (int s = 1; s <= max_s; s *= 2)
-        if (32 * s >= w) return s;
-    return 0;
+    const int tv = tune_get(kind, w);
+    *s = tv == 4 || tv == 8 ? tv : (w <= 64 ? 2 : (w <= 128 ? 4 : 8));
+    if (*s < 8 && w > 32 * *s * 16) *s = 8;
+    const int need = (w + 32 * *s - 1) / (32 * *s);
+    *nw = 1;
+    while (*nw < need) *nw *= 2;
 }
+
+// every shape row_shape gives, up to 4096 cells: f(S, NW)
+#define DOL_ROW_SHAPES(f) \
+    f(2, 1) f(4, 1) f(4, 2) f(4, 4) f(4, 8) f(4, 16) f(8, 1) f(8, 2) f(8, 4) f(8, 8) f(8, 16)
 
 void launch_danielsson(int dim, void* deltas, int w, int h, int d, int cw, cudaStream_t st)
 {
-    const int kind = dim == 2 ? kTuneDan2 : kTuneDan3;
-    const int tv = tune_get(kind, w);
-    const int ws = warp_s(w, dim == 2 ? 16 : 8);
+    int s, nw;
+    row_shape(dim == 2 ? kTuneDan2 : kTuneDan3, w, &s, &nw);
     ProfScope ps("danielsson", st);
-    if (ws && (tv == kWarpEngine || tv == 0)) {
-#define DOL_DANW_CASE(SV)                                                                             \
-    case SV:                                                                                          \
-        if (dim == 2)                                                                                 \
-            k_danielsson2_w<SV><<<1, 32, 0, st>>>(static_cast<uint32_t*>(deltas), w, h, cw);         \
-        else                                                                                          \
-            k_danielsson3_w<(SV > 8 ? 8 : SV)><<<1, 32, 0, st>>>(static_cast<int16_t*>(deltas), w, h, d, cw); \
-        return;
-        switch (ws) {
-            DOL_DANW_CASE(1)
-            DOL_DANW_CASE(2)
-            DOL_DANW_CASE(4)
-            DOL_DANW_CASE(8)
-            DOL_DANW_CASE(16)
-            default: break;
-        }
-#undef DOL_DANW_CASE
+    auto run = [&](auto kern, int warps, size_t strips) {
+        if (strips > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)strips);
+        kern<<<1, 32 * warps, strips, st>>>(deltas, w, h, dim == 2 ? 1 : d, cw);
+    };
+#define DOL_DAN_CASE(SV, NWV)                                                          \
+    if (s == SV && nw == NWV) {                                                        \
+        if (dim == 2)                                                                  \
+            run(k_dan_serial<2, SV, NWV>, NWV, NWV * SerialIO<2, SV>::kBytes);         \
+        else                                                                           \
+            run(k_dan_serial<3, SV, NWV>, NWV, NWV * SerialIO<3, SV>::kBytes);         \
     }
-    const int s = tuned_s(kind, w, 512);
-    const int T = threads_for(w, s);
-#define DOL_DAN_CASE(SV)                                                                              \
-    case SV:                                                                                          \
-        if (dim == 2)                                                                                 \
-            k_danielsson2<SV><<<1, T, 0, st>>>(static_cast<uint32_t*>(deltas), w, h, cw);            \
-        else                                                                                          \
-            k_danielsson3<SV><<<1, T, 0, st>>>(static_cast<int16_t*>(deltas), w, h, d, cw);          \
-        break;
-    switch (s) {
-        DOL_DAN_CASE(1)
-        DOL_DAN_CASE(2)
-        DOL_DAN_CASE(4)
-        DOL_DAN_CASE(8)
-        default: break;
-    }
+    DOL_ROW_SHAPES(DOL_DAN_CASE)
 #undef DOL_DAN_CASE
 }
 
 void launch_fastsweep_2d(void* deltas, int w, int h, int cw, cudaStream_t st)
 {
-    const int tv = tune_get(kTuneFs2, w);
-    const int ws = warp_s(w, 16);
+    int s, nw;
+    row_shape(kTuneFs2, w, &s, &nw);
     ProfScope ps("fastsweep_2d", st);
-    if (ws && (tv == kWarpEngine || tv == 0)) {
-#define DOL_FSW_CASE(SV)                                                                              \
-    case SV:                                                                                          \
-        k_fastsweep2_w<SV><<<1, 32, 0, st>>>(static_cast<uint32_t*>(deltas), w, h, cw);              \
-        return;
-        switch (ws) {
-            DOL_FSW_CASE(1)
-            DOL_FSW_CASE(2)
-            DOL_FSW_CASE(4)
-            DOL_FSW_CASE(8)
-            DOL_FSW_CASE(16)
-            default: break;
-        }
-#undef DOL_FSW_CASE
-    }
-    const int s = tuned_s(kTuneFs2, w, 512);
-    const int T = threads_for(w, s);
-#define DOL_FS_CASE(SV)                                                                                      \
-    case SV:                                                                                                 \
-        k_fastsweep2<SV><<<1, T, 0, st>>>(static_cast<uint32_t*>(deltas), w, h, cw);                         \
-        break;
-    switch (s) {
-        DOL_FS_CASE(1)
-        DOL_FS_CASE(2)
-        DOL_FS_CASE(4)
-        DOL_FS_CASE(8)
-        default: break;
-    }
+#define DOL_FS_CASE(SV, NWV) \
+    if (s == SV && nw == NWV)  \
+        k_fastsweep2<SV, NWV><<<1, 32 * NWV, NWV * SerialIO<2, SV>::kBytes, st>>>(deltas, w, h, cw);
+    DOL_ROW_SHAPES(DOL_FS_CASE)
 #undef DOL_FS_CASE
 }
 
@@ -878,165 +520,159 @@ struct BatchItemDev {
     long long dist_off;    // floats, < 0: none
 };
 
-__device__ __forceinline__ void border2_cta(const uint32_t* mask, uint32_t* dl, int w, int h)
+// Border initialisation and signed distances of an item by `nu` warps, this
+// being warp u of them.  A warp takes 32 mask words at a time: lane q forms the
+// bit planes of word q, then all lanes write one word's 32 cells after the
+// other, so that stores run along the row.
+template <int DIM>
+__device__ __forceinline__ void border_warps(const uint32_t* mask, void* dl, int w, int h, int d, int u, int nu)
 {
+    const int lane = threadIdx.x & 31;
     const int ws = words_per_row(w);
-    for (long long wid = threadIdx.x; wid < (long long)ws * h; wid += blockDim.x) {
-        const int y = (int)(wid / ws), k = (int)(wid - (long long)y * ws);
-        Planes2 p = border2_word(w, h, mask, y, k);
-        const int n = min(32, w - 32 * k);
-        uint32_t* row = dl + (long long)y * w + 32 * k;
-        for (int b = 0; b < n; b++) row[b] = pack2(decode2(p, b));
-    }
-}
-
-__device__ __forceinline__ void border3_cta(const uint32_t* mask, int16_t* dl, int w, int h, int d)
-{
-    const int ws = words_per_row(w);
-    const long long words = (long long)ws * h * d;
-    for (long long wid = threadIdx.x; wid < words; wid += blockDim.x) {
-        const long long row = wid / ws;
-        const int k = (int)(wid - row * ws);
-        const int z = (int)(row / h), y = (int)(row - (long long)z * h);
-        Planes3 p = border3_word(w, h, d, mask, z, y, k);
-        const int n = min(32, w - 32 * k);
-        for (int b = 0; b < n; b++) cell_store(dl, row * w + 32 * k + b, decode3(p, b));
+    const int words = ws * h * d;
+    for (int base = 32 * u; base < words; base += 32 * nu) {
+        const int wid = min(base + lane, words - 1);
+        const int row = wid / ws, k = wid - row * ws;
+        uint32_t pl[7];
+        if (DIM == 2) {
+            const Planes2 p = border2_word(w, h, mask, row, k);
+            pl[0] = p.mx; pl[1] = p.xn; pl[2] = p.xs; pl[3] = p.yn; pl[4] = p.ys; pl[5] = pl[6] = 0;
+        } else {
+            const int z = row / h;
+            const Planes3 p = border3_word(w, h, d, mask, z, row - z * h, k);
+            pl[0] = p.mx; pl[1] = p.xn; pl[2] = p.xs; pl[3] = p.yn; pl[4] = p.ys; pl[5] = p.zn; pl[6] = p.zs;
+        }
+        const int first = row * w + 32 * k, live = min(32, w - 32 * k);
+        const int n = min(32, words - base);
+        for (int q = 0; q < n; q++) {
+            uint32_t b[7];
+#pragma unroll
+            for (int i = 0; i < (DIM == 2 ? 5 : 7); i++) b[i] = __shfl_sync(0xFFFFFFFFu, pl[i], q);
+            const int at = __shfl_sync(0xFFFFFFFFu, first, q) + lane;
+            const int nq = __shfl_sync(0xFFFFFFFFu, live, q);
+            if (lane < nq) {
+                if (DIM == 2)
+                    static_cast<uint32_t*>(dl)[at] = pack2(decode2(Planes2{b[0], b[1], b[2], b[3], b[4]}, lane));
+                else
+                    cell_store(static_cast<int16_t*>(dl), at,
+                               decode3(Planes3{b[0], b[1], b[2], b[3], b[4], b[5], b[6]}, lane));
+            }
+        }
     }
 }
 
 template <class Cell, class P>
-__device__ __forceinline__ void signed_dist_cta(const uint32_t* mask, const P* dl, float* out, int w, long long rows)
-{
-    const int ws = words_per_row(w);
-    for (long long i = threadIdx.x; i < rows * w; i += blockDim.x) {
-        const long long row = i / w;
-        const int x = (int)(i - row * w);
-        float r = __fdiv_rn(sqrtf((float)len(cell_load(dl, i))), 2.0f);
-        if ((mask[row * ws + (x >> 5)] >> (x & 31)) & 1u) r = -r;
-        out[i] = r;
-    }
-}
-
-// warp-cooperative pieces for items whose rows fit one warp
-__device__ __forceinline__ void border2_warp(const uint32_t* mask, uint32_t* dl, int w, int h)
+__device__ __forceinline__ void signed_dist_warps(const uint32_t* mask, const P* dl, float* out, int w, int rows, int u,
+                                                  int nu)
 {
     const int lane = threadIdx.x & 31;
     const int ws = words_per_row(w);
-    for (long long wid = lane; wid < (long long)ws * h; wid += 32) {
-        const int y = (int)(wid / ws), k = (int)(wid - (long long)y * ws);
-        Planes2 p = border2_word(w, h, mask, y, k);
-        const int n = min(32, w - 32 * k);
-        uint32_t* row = dl + (long long)y * w + 32 * k;
-        for (int b = 0; b < n; b++) row[b] = pack2(decode2(p, b));
+    for (int row = u; row < rows; row += nu) {
+        const long long first = (long long)row * w;
+        for (int x = lane; x < w; x += 32) {
+            float r = __fdiv_rn(sqrtf((float)len(cell_load(dl, first + x))), 2.0f);
+            if ((mask[(long long)row * ws + (x >> 5)] >> lane) & 1u) r = -r;
+            out[first + x] = r;
+        }
     }
 }
 
-__device__ __forceinline__ void border3_warp(const uint32_t* mask, int16_t* dl, int w, int h, int d)
+// Danielsson of one field by one warp: rows of at most 256 cells
+template <int DIM>
+__device__ __noinline__ void batch_dan_warp(void* dl, int w, int h, int d, unsigned char* strip)
 {
-    const int lane = threadIdx.x & 31;
-    const int ws = words_per_row(w);
-    const long long words = (long long)ws * h * d;
-    for (long long wid = lane; wid < words; wid += 32) {
-        const long long row = wid / ws;
-        const int k = (int)(wid - row * ws);
-        const int z = (int)(row / h), y = (int)(row - (long long)z * h);
-        Planes3 p = border3_word(w, h, d, mask, z, y, k);
-        const int n = min(32, w - 32 * k);
-        for (int b = 0; b < n; b++) cell_store(dl, row * w + 32 * k + b, decode3(p, b));
-    }
+    RowShared<1> none;
+    if (w <= 64) dan_serial<DIM, 2, 1>(dl, w, h, d, 2, strip, none);
+    else if (w <= 128) dan_serial<DIM, 4, 1>(dl, w, h, d, 2, strip, none);
+    else dan_serial<DIM, 8, 1>(dl, w, h, d, 2, strip, none);
 }
-
-template <class Cell, class P>
-__device__ __forceinline__ void signed_dist_warp(const uint32_t* mask, const P* dl, float* out, int w, long long rows)
+// by a group of 4 warps: rows of at most 1024 cells
+template <int DIM, int S>
+__device__ __noinline__ void batch_dan_group(void* dl, int w, int h, int d, unsigned char* strip, RowShared<4>& sh)
 {
-    const int lane = threadIdx.x & 31;
-    const int ws = words_per_row(w);
-    for (long long i = lane; i < rows * w; i += 32) {
-        const long long row = i / w;
-        const int x = (int)(i - row * w);
-        float r = __fdiv_rn(sqrtf((float)len(cell_load(dl, i))), 2.0f);
-        if ((mask[row * ws + (x >> 5)] >> (x & 31)) & 1u) r = -r;
-        out[i] = r;
-    }
+    dan_serial<DIM, S, 4>(dl, w, h, d, 2, strip, sh);
+}
+// a volume by the whole CTA: rows of at most 128 cells, as many as fit in shared memory
+template <int S, int NW>
+__device__ __noinline__ void batch_dan_slices(void* dl, int w, int h, int d, unsigned char* smem)
+{
+    dan_slices<S, NW>(dl, w, h, d, 2, smem);
 }
 
-// an item processed by one warp: rows of at most 256 cells
+// an image processed by one warp
 __device__ __noinline__ void batch_item_warp(const BatchItemDev& b, const uint32_t* masks, unsigned char* deltas,
-                                             float* dist)
+                                             float* dist, unsigned char* strip)
 {
     const uint32_t* m = masks + b.mask_off;
-    if (b.d <= 1) {
-        uint32_t* dl = reinterpret_cast<uint32_t*>(deltas + b.delta_off);
-        border2_warp(m, dl, b.w, b.h);
-        __syncwarp();
-        if (b.w <= 64) danielsson2_warp<2>(dl, b.w, b.h, 2);
-        else if (b.w <= 128) danielsson2_warp<4>(dl, b.w, b.h, 2);
-        else danielsson2_warp<8>(dl, b.w, b.h, 2);
-        __syncwarp();
-        if (dist && b.dist_off >= 0) signed_dist_warp<C2>(m, dl, dist + b.dist_off, b.w, b.h);
-    } else {
-        int16_t* dl = reinterpret_cast<int16_t*>(deltas + b.delta_off);
-        border3_warp(m, dl, b.w, b.h, b.d);
-        __syncwarp();
-        if (b.w <= 64) danielsson3_warp<2>(dl, b.w, b.h, b.d, 2);
-        else if (b.w <= 128) danielsson3_warp<4>(dl, b.w, b.h, b.d, 2);
-        else danielsson3_warp<8>(dl, b.w, b.h, b.d, 2);
-        __syncwarp();
-        if (dist && b.dist_off >= 0) signed_dist_warp<C3>(m, dl, dist + b.dist_off, b.w, (long long)b.h * b.d);
-    }
+    uint32_t* dl = reinterpret_cast<uint32_t*>(deltas + b.delta_off);
+    border_warps<2>(m, dl, b.w, b.h, 1, 0, 1);
+    __syncwarp();
+    batch_dan_warp<2>(dl, b.w, b.h, 1, strip);
+    __syncwarp();
+    if (dist && b.dist_off >= 0) signed_dist_warps<C2>(m, dl, dist + b.dist_off, b.w, b.h, 0, 1);
 }
 
 // Two queues.  Queue A (order[0 .. nv)) holds the volumes whose rows fit one
 // warp (up to 256 cells), longest chain first; queue B (order[nv .. n)) the
-// items with rows over 256 cells, then the narrow images.  A CTA takes queue A
-// items while there are any: the whole CTA runs the volume's border init and
-// its distances, while warp 0 alone runs the serial sweep with the
-// single-warp engine (no CTA barriers in the chain; 1.5-2x faster than the
-// CTA engine on rows this narrow).  Then it turns to queue B: items with wide
-// rows take the whole CTA; the first narrow image it draws switches it to
-// per-warp draining.  counter: [0] queue B, [1] queue A, [2] nv (written by
-// dol_batch_prepare).
-template <int S>
-__global__ void __launch_bounds__(256) k_batch_sdf(const BatchItemDev* __restrict__ items, const int* __restrict__ order,
-                                                   int n, const uint32_t* __restrict__ masks,
-                                                   unsigned char* __restrict__ deltas, float* __restrict__ dist,
-                                                   int* __restrict__ counter)
+// items with rows over 256 cells, then the narrow images.  A CTA (one per SM)
+// takes queue A items while there are any, the slices' rows in parallel chunks
+// (dan_slices.cuh), or, where a slice does not fit in shared memory, warp 0
+// walking it serially.  Then each group of 4 warps turns to queue B by itself
+// (its own barrier): items with wide rows take the group; the first narrow
+// image it draws switches it to per-warp draining.
+// 4096 images and 64 volumes: 98 ms with every volume walked serially by one
+// warp, 55 ms.
+// counter: [0] queue B, [1] queue A, [2] nv (written by dol_batch_prepare).
+constexpr size_t kBatchSmem = 216 * 1024;
+constexpr int kBatchStrip = (int)SerialIO<3, 8>::kBytes;   // a warp's strips in queue B, the widest
+
+template <int NW>
+__global__ void __launch_bounds__(32 * NW) k_batch_sdf(const BatchItemDev* __restrict__ items,
+                                                       const int* __restrict__ order, int n,
+                                                       const uint32_t* __restrict__ masks,
+                                                       unsigned char* __restrict__ deltas, float* __restrict__ dist,
+                                                       int* __restrict__ counter)
 {
-    __shared__ ScanShared<C3> sh3;   // the larger of the two; the 2D engine reuses its storage
-    __shared__ int s_item;
-    ScanShared<C2>& sh2 = *reinterpret_cast<ScanShared<C2>*>(&sh3);
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ RowShared<4> sh[NW / 4];
+    __shared__ int s_item[NW / 4 + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nv = counter[2];
     for (;;) {
-        if (threadIdx.x == 0) s_item = atomicAdd(counter + 1, 1);
+        if (threadIdx.x == 0) s_item[0] = atomicAdd(counter + 1, 1);
         __syncthreads();
-        const int it = s_item;
+        const int it = s_item[0];
         __syncthreads();
         if (it >= nv) break;
         const BatchItemDev b = items[order[it]];
         const uint32_t* m = masks + b.mask_off;
         int16_t* dl = reinterpret_cast<int16_t*>(deltas + b.delta_off);
-        border3_cta(m, dl, b.w, b.h, b.d);
+        border_warps<3>(m, dl, b.w, b.h, b.d, warp, NW);
         __syncthreads();
-        if (warp == 0) {
-            if (b.w <= 64) danielsson3_warp<2>(dl, b.w, b.h, b.d, 2);
-            else if (b.w <= 128) danielsson3_warp<4>(dl, b.w, b.h, b.d, 2);
-            else danielsson3_warp<8>(dl, b.w, b.h, b.d, 2);
-        }
+        if (b.w <= 64 && SliceIO<2>::bytes(b.h, NW) <= kBatchSmem) batch_dan_slices<2, NW>(dl, b.w, b.h, b.d, smem);
+        else if (b.w <= 128 && SliceIO<4>::bytes(b.h, NW) <= kBatchSmem)
+            batch_dan_slices<4, NW>(dl, b.w, b.h, b.d, smem);
+        else if (warp == 0) batch_dan_warp<3>(dl, b.w, b.h, b.d, smem);
         __syncthreads();
-        if (dist && b.dist_off >= 0) signed_dist_cta<C3>(m, dl, dist + b.dist_off, b.w, (long long)b.h * b.d);
+        if (dist && b.dist_off >= 0)
+            signed_dist_warps<C3>(m, dl, dist + b.dist_off, b.w, b.h * b.d, warp, NW);
         __syncthreads();
     }
+    const int group = warp >> 2, gw = warp & 3;
+    RowShared<4>& gsh = sh[group];
+    unsigned char* strip = smem + warp * kBatchStrip;
+    if ((threadIdx.x & 127) == 0) gsh.bar = 1 + group;
+    auto sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); };
     for (;;) {
-        if (threadIdx.x == 0) s_item = nv + atomicAdd(counter, 1);
-        __syncthreads();
-        const int it = s_item;
-        __syncthreads();
+        if ((threadIdx.x & 127) == 0) s_item[1 + group] = nv + atomicAdd(counter, 1);
+        sync();
+        const int it = s_item[1 + group];
+        sync();
         if (it >= n) return;
         const BatchItemDev b = items[order[it]];
         if (b.w <= 256) {
-            // narrow images from here on: warp 0 takes this item, every warp then drains the queue
-            int mine = warp == 0 ? it : -1;
+            // narrow images from here on: the group's first warp takes this item, every warp then drains the queue
+            int mine = gw == 0 ? it : -1;
             for (;;) {
                 if (mine < 0) {
                     int v = 0;
@@ -1044,27 +680,31 @@ __global__ void __launch_bounds__(256) k_batch_sdf(const BatchItemDev* __restric
                     mine = __shfl_sync(0xFFFFFFFFu, v, 0);
                     if (mine >= n) return;
                 }
-                batch_item_warp(items[order[mine]], masks, deltas, dist);
+                batch_item_warp(items[order[mine]], masks, deltas, dist, strip);
                 mine = -1;
             }
         }
         const uint32_t* m = masks + b.mask_off;
+        void* dl = deltas + b.delta_off;
+        const int rows = b.h * b.d;
         if (b.d <= 1) {
-            uint32_t* dl = reinterpret_cast<uint32_t*>(deltas + b.delta_off);
-            border2_cta(m, dl, b.w, b.h);
-            __syncthreads();
-            danielsson2_cta<S>(dl, b.w, b.h, 2, sh2);
-            __syncthreads();
-            if (dist && b.dist_off >= 0) signed_dist_cta<C2>(m, dl, dist + b.dist_off, b.w, b.h);
+            border_warps<2>(m, dl, b.w, b.h, 1, gw, 4);
+            sync();
+            if (b.w <= 512) batch_dan_group<2, 4>(dl, b.w, b.h, 1, strip, gsh);
+            else batch_dan_group<2, 8>(dl, b.w, b.h, 1, strip, gsh);
+            sync();
+            if (dist && b.dist_off >= 0)
+                signed_dist_warps<C2>(m, static_cast<uint32_t*>(dl), dist + b.dist_off, b.w, rows, gw, 4);
         } else {
-            int16_t* dl = reinterpret_cast<int16_t*>(deltas + b.delta_off);
-            border3_cta(m, dl, b.w, b.h, b.d);
-            __syncthreads();
-            danielsson3_cta<S>(dl, b.w, b.h, b.d, 2, sh3);
-            __syncthreads();
-            if (dist && b.dist_off >= 0) signed_dist_cta<C3>(m, dl, dist + b.dist_off, b.w, (long long)b.h * b.d);
+            border_warps<3>(m, dl, b.w, b.h, b.d, gw, 4);
+            sync();
+            if (b.w <= 512) batch_dan_group<3, 4>(dl, b.w, b.h, b.d, strip, gsh);
+            else batch_dan_group<3, 8>(dl, b.w, b.h, b.d, strip, gsh);
+            sync();
+            if (dist && b.dist_off >= 0)
+                signed_dist_warps<C3>(m, static_cast<int16_t*>(dl), dist + b.dist_off, b.w, rows, gw, 4);
         }
-        __syncthreads();
+        sync();
     }
 }
 
@@ -1074,25 +714,23 @@ void launch_batch_sdf(const void* items, const int* order, int n, const uint32_t
                       int* counter, cudaStream_t st)
 {
     ProfScope ps("batch_sdf", st);
-    // rows up to 1024 cells: 4 cells x 256 threads, or 8 cells x 128 threads
-    const bool eight = tune_get(kTuneBatch, 1024) == 8;
-    const int threads = eight ? 128 : 256;
-    int per_sm = 0;
-    if (eight)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_sdf<8>, threads, 0);
+    // 16 warps per CTA, or 8
+    auto run = [&](auto kern, int warps) {
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBatchSmem);
+        int per_sm = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, kBatchSmem);
+        if (per_sm < 1) per_sm = 1;
+        int grid = per_sm * g_num_sms;
+        if (grid > n) grid = n;
+        if (grid < 1) grid = 1;
+        cudaMemsetAsync(counter, 0, 2 * sizeof(int), st);   // the queue heads; counter[2] (nv) stays
+        kern<<<grid, 32 * warps, kBatchSmem, st>>>(static_cast<const BatchItemDev*>(items), order, n, masks,
+                                                   static_cast<unsigned char*>(deltas), dist, counter);
+    };
+    if (tune_get(kTuneBatch, 1024) == 8)
+        run(k_batch_sdf<8>, 8);
     else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_sdf<4>, threads, 0);
-    if (per_sm < 1) per_sm = 1;
-    int grid = per_sm * g_num_sms;
-    if (grid > n) grid = n;
-    if (grid < 1) grid = 1;
-    cudaMemsetAsync(counter, 0, 2 * sizeof(int), st);   // the queue heads; counter[2] (nv) stays
-    if (eight)
-        k_batch_sdf<8><<<grid, threads, 0, st>>>(static_cast<const BatchItemDev*>(items), order, n, masks,
-                                                 static_cast<unsigned char*>(deltas), dist, counter);
-    else
-        k_batch_sdf<4><<<grid, threads, 0, st>>>(static_cast<const BatchItemDev*>(items), order, n, masks,
-                                                 static_cast<unsigned char*>(deltas), dist, counter);
+        run(k_batch_sdf<16>, 16);
 }
 
 }  // namespace dolk
