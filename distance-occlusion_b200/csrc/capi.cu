@@ -523,8 +523,10 @@ dol_status dol_fastsweep_3d(int w, int h, int d, dol_delta3* deltas, int cw, voi
     if (w > kMaxSweepWidth3) return fail(DOL_ERR_UNSUPPORTED, "3D FastSweep rows are limited to %d cells", kMaxSweepWidth3);
     DOL_TRY(check_dev_ptr(deltas, "deltas"));
     Workspace ws;
-    DOL_TRY(get_workspace(ws, workspace, workspace_bytes, fastsweep3_workspace_bytes(w, h, d), S(stream)));
-    launch_fastsweep_3d(deltas, w, h, d, cw, ws.ptr, ds->err_dev, S(stream));
+    size_t got;
+    DOL_TRY(get_workspace_between(ws, workspace, workspace_bytes, fastsweep3_workspace_bytes(w, h, d),
+                                  fastsweep3_workspace_bytes_min(w, h, d), &got, S(stream)));
+    launch_fastsweep_3d(deltas, w, h, d, cw, ws.ptr, got, ds->err_dev, S(stream));
     return launched("fastsweep_3d");
 }
 
@@ -730,6 +732,12 @@ dol_status dol_voxelize_triangles(int tri_count, const int* indices, const float
 
 static size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
+// what FastSweep 3D asks for above what it can run on
+static size_t fastsweep3_spare(int w, int h, int d)
+{
+    return align256(fastsweep3_workspace_bytes(w, h, d)) - align256(fastsweep3_workspace_bytes_min(w, h, d));
+}
+
 size_t dol_sdf_workspace_size(int w, int h, int d, int method)
 {
     const int dim = d > 1 ? 3 : 2;
@@ -772,7 +780,13 @@ static dol_status sdf_common(int dim, int w, int h, int d, const uint32_t* mask,
         launch_edt_mask(ed, mask, dist, w, h, d, DOL_EDT_SIGNED, ws.ptr, got, ds->err_dev, st);
         return launched("sdf (felzenszwalb)");
     }
-    DOL_TRY(get_workspace(ws, workspace, workspace_bytes, dol_sdf_workspace_size(w, h, dim == 3 ? d : 1, method), st));
+    // FastSweep 3D runs on less than it asks for
+    const size_t need = dol_sdf_workspace_size(w, h, dim == 3 ? d : 1, method);
+    const size_t spare = method == DOL_FASTSWEEP && dim == 3 && d > 1 ? fastsweep3_spare(w, h, d) : 0;
+    size_t got;
+    DOL_TRY(get_workspace_between(ws, workspace, workspace_bytes, need, need - spare, &got, st));
+    const size_t fs3_bytes = spare && got < need ? fastsweep3_workspace_bytes_min(w, h, d)
+                                                 : fastsweep3_workspace_bytes(w, h, d);
     const size_t cells = (size_t)w * h * (dim == 3 ? d : 1);
     const size_t cb = dim == 3 ? sizeof(dol_delta3) : sizeof(dol_delta2);
     char* p = static_cast<char*>(ws.ptr);
@@ -786,7 +800,7 @@ static dol_status sdf_common(int dim, int w, int h, int d, const uint32_t* mask,
         if (dim == 2)
             launch_fastsweep_2d(dl, w, h, 2, st);
         else
-            launch_fastsweep_3d(dl, w, h, d, 2, p, ds->err_dev, st);
+            launch_fastsweep_3d(dl, w, h, d, 2, p, fs3_bytes, ds->err_dev, st);
     } else {
         launch_jumpflood(dim, dl, p, w, h, d, 2, st);
     }
@@ -842,7 +856,12 @@ static dol_status sdf_two_pass_common(int dim, int w, int h, int d, const uint32
     cudaStream_t st = S(stream);
     const int dd = dim == 3 ? d : 1;
     Workspace ws;
-    DOL_TRY(get_workspace(ws, workspace, workspace_bytes, dol_sdf_two_pass_workspace_size(w, h, dd, method), st));
+    const size_t need = dol_sdf_two_pass_workspace_size(w, h, dd, method);
+    const size_t spare = method == DOL_FASTSWEEP && dd > 1 ? fastsweep3_spare(w, h, d) : 0;
+    size_t got;
+    DOL_TRY(get_workspace_between(ws, workspace, workspace_bytes, need, need - spare, &got, st));
+    const size_t fs3_bytes = spare && got < need ? fastsweep3_workspace_bytes_min(w, h, d)
+                                                 : fastsweep3_workspace_bytes(w, h, d);
     const size_t cells = (size_t)w * h * dd;
     const size_t cb = dim == 3 ? sizeof(dol_delta3) : sizeof(dol_delta2);
     char* p = static_cast<char*>(ws.ptr);
@@ -860,7 +879,7 @@ static dol_status sdf_two_pass_common(int dim, int w, int h, int d, const uint32
             if (dim == 2)
                 launch_fastsweep_2d(dl, w, h, 1, st);
             else
-                launch_fastsweep_3d(dl, w, h, d, 1, p, ds->err_dev, st);
+                launch_fastsweep_3d(dl, w, h, d, 1, p, fs3_bytes, ds->err_dev, st);
         } else {
             launch_jumpflood(dim, dl, p, w, h, dd, 1, st);
         }

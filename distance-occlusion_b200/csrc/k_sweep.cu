@@ -413,15 +413,24 @@ void launch_fastsweep_2d(void* deltas, int w, int h, int cw, cudaStream_t st)
 
 size_t fastsweep3_workspace_bytes(int w, int h, int d)
 {
+    const size_t pipe = fastsweep3_pipe_bytes(w, h, d), rows = fastsweep3_workspace_bytes_min(w, h, d);
+    return pipe > rows ? pipe : rows;
+}
+
+size_t fastsweep3_workspace_bytes_min(int w, int h, int d)
+{
     (void)w;
     size_t flags = (size_t)h * d * sizeof(int);
     size_t diag = (size_t)(h + d + 2) * sizeof(int);
     return ((flags + 255) & ~(size_t)255) + ((diag + 255) & ~(size_t)255) + 256;
 }
 
-void launch_fastsweep_3d(void* deltas, int w, int h, int d, int cw, void* ws, int* err, cudaStream_t st)
+void launch_fastsweep_3d(void* deltas, int w, int h, int d, int cw, void* ws, size_t ws_bytes, int* err,
+                         cudaStream_t st)
 {
     if (h < 2 || d < 2) return;   // no row is ever updated (:2208, :2214 start at 1)
+    if (launch_fastsweep_3d_pipe(deltas, w, h, d, cw, ws, ws_bytes, err, st)) return;
+    cudaGetLastError();
     char* p = static_cast<char*>(ws);
     int* flags = reinterpret_cast<int*>(p);
     p += (((size_t)h * d * sizeof(int)) + 255) & ~(size_t)255;

@@ -117,11 +117,18 @@ size_t danielsson_workspace_bytes(int dim, int w, int h, int d);
 bool run_danielsson(int dim, void* deltas, int w, int h, int d, int cw, void* ws, size_t ws_bytes, int* err,
                     cudaStream_t st);
 void launch_fastsweep_2d(void* deltas, int w, int h, int cw, cudaStream_t st);
+// the _min form holds the engines of rows too wide for a warp
 size_t fastsweep3_workspace_bytes(int w, int h, int d);
+size_t fastsweep3_workspace_bytes_min(int w, int h, int d);
 // batched signed Danielsson; items: device array of dol_batch_item (40 bytes)
 void launch_batch_sdf(const void* items, const int* order, int n, const uint32_t* masks, void* deltas, float* dist,
                       int* counter, cudaStream_t st);
-void launch_fastsweep_3d(void* deltas, int w, int h, int d, int cw, void* ws, int* err, cudaStream_t st);
+void launch_fastsweep_3d(void* deltas, int w, int h, int d, int cw, void* ws, size_t ws_bytes, int* err,
+                         cudaStream_t st);
+// k_fastsweep3.cu -- rows of up to 256 cells; false when it does not apply
+size_t fastsweep3_pipe_bytes(int w, int h, int d);
+bool launch_fastsweep_3d_pipe(void* deltas, int w, int h, int d, int cw, void* ws, size_t ws_bytes, int* err,
+                              cudaStream_t st);
 
 // k_chamfer.cu -- Chamfer 3-4 on int16 / int32 fields
 template <typename T>

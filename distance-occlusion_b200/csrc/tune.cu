@@ -264,7 +264,7 @@ DOL_API dol_status dol_autotune(int kind, int w, int h, int d, void* stream)
                 break;
             case kTuneFs3:
                 launch_init_border(3, static_cast<uint32_t*>(dm), dl, tw, th, td, st);
-                launch_fastsweep_3d(dl, tw, th, td, 2, ws, err, st);
+                launch_fastsweep_3d(dl, tw, th, td, 2, ws, ws_bytes, err, st);
                 break;
             case kTuneJfa2:
             case kTuneJfa3:
