@@ -680,7 +680,7 @@ dol_status dol_occlusion_sweep_2d(int w, int h, float* dirW, void* stream)
     DOL_TRY(device_state(&ds));
     DOL_TRY(occ_checks(w, h, 1));
     DOL_TRY(check_dev_ptr(dirW, "dirW"));
-    launch_occlusion_sweep(2, dirW, nullptr, w, h, 1, S(stream));
+    launch_occlusion_sweep(2, dirW, nullptr, w, h, 1, ds->err_dev, g_workspace_limit.load(), S(stream));
     return launched("occlusion_sweep_2d");
 }
 
@@ -690,7 +690,7 @@ dol_status dol_occlusion_sweep_3d(int w, int h, int d, float* dirW, void* stream
     DOL_TRY(device_state(&ds));
     DOL_TRY(occ_checks(w, h, d));
     DOL_TRY(check_dev_ptr(dirW, "dirW"));
-    launch_occlusion_sweep(3, dirW, nullptr, w, h, d, S(stream));
+    launch_occlusion_sweep(3, dirW, nullptr, w, h, d, ds->err_dev, g_workspace_limit.load(), S(stream));
     return launched("occlusion_sweep_3d");
 }
 
@@ -702,7 +702,7 @@ dol_status dol_occlusion_sweep_3d_io(int w, int h, int d, const float* in, float
     DOL_TRY(check_dev_ptr(in, "in"));
     DOL_TRY(check_dev_ptr(out, "out"));
     if (in == out) return fail(DOL_ERR_INVALID_ARG, "the in/out occlusion sweep needs distinct in and out fields");
-    launch_occlusion_sweep(3, out, in, w, h, d, S(stream));
+    launch_occlusion_sweep(3, out, in, w, h, d, ds->err_dev, g_workspace_limit.load(), S(stream));
     return launched("occlusion_sweep_3d_io");
 }
 

@@ -387,6 +387,271 @@ __global__ void __launch_bounds__(32 * BY, 1024 / (32 * BY))
     }
 }
 
+// ---- pipelined block wavefront (3D, in place) ---------------------------------------------
+//
+// The same blocks without a launch per diagonal: persistent CTAs take blocks from
+// a counter in the order of their diagonals (all 8 planes side by side) and wait
+// for the flags of the three blocks before theirs.  A block is taken only by a
+// running CTA, after every block it waits for, so the earliest unfinished one
+// always proceeds; the waits are bounded.
+//
+// A block (32 columns x kWaveY rows x kWaveZ slices) is staged in shared memory by
+// whole rows -- the skewed order touches a different row in every lane, which
+// straight from global memory was a sector per lane and access -- while its CTA
+// waits for the blocks before it.  A lane owns kWaveM adjacent rows of one
+// column: at step s it updates slice s - i - j of row j.  "back" is its own value
+// of the step before, "left" its neighbour lane's (a shuffle), "up" its own of
+// the row before, or, for its first row, the value the warp before put into the
+// block a step earlier; one barrier per step.  The slice index falls with the
+// lane, so the 32 lanes of an access fall in 32 banks.
+//
+// What bounds it: the steps' latency (shuffle, shared load, ten dependent float
+// operations) and lanes that wait for their first slice (32 of 66 steps each).
+// 256^3, 8 planes: 1.73 ms with a launch per diagonal, 0.77 ms.
+constexpr int kWaveY = 16, kWaveZ = 32, kWaveM = 4;
+constexpr int kWaveThreads = 32 * kWaveY / kWaveM;
+
+struct OccWave {
+    float* planes;
+    unsigned* counter;   // blocks taken
+    unsigned* done;      // per plane and block
+    int* err;
+    int w, h, d, nbx, nby, nbz;
+};
+
+struct WaveBlock {
+    int plane, bx, by, bz;
+};
+
+// Block number t in the order of diagonals, planes side by side.  diag[l]: the
+// blocks of one plane on diagonals before l.
+__device__ __forceinline__ WaveBlock wave_block(const OccWave& p, const int* diag, int t)
+{
+    WaveBlock b;
+    b.plane = t & 7;
+    int r = t >> 3, l = 0;
+    const int nd = p.nbx + p.nby + p.nbz - 2;
+    int step = 1;
+    while (step < nd) step <<= 1;
+    for (; step > 0; step >>= 1)
+        if (l + step < nd && diag[l + step] <= r) l += step;
+    r -= diag[l];
+    for (b.bz = max(0, l - (p.nbx - 1) - (p.nby - 1));; b.bz++) {   // by: lo .. hi on this diagonal
+        const int m = l - b.bz, lo = max(0, m - (p.nbx - 1)), hi = min(p.nby - 1, m);
+        if (r <= hi - lo) {
+            b.by = lo + r;
+            b.bx = m - b.by;
+            return b;
+        }
+        r -= hi - lo + 1;
+    }
+}
+
+__global__ void __launch_bounds__(kWaveThreads) k_occlusion_wave3(OccWave p)
+{
+    extern __shared__ __align__(16) float smem_f[];
+    float* T = smem_f;                            // [kWaveZ][kWaveY][32], x in memory order
+    float* U = T + kWaveZ * kWaveY * 32;          // [kWaveZ][32]: row j = -1
+    float* F = U + kWaveZ * 32;                   // [kWaveZ][kWaveY]: column i = -1
+    int* diag = reinterpret_cast<int*>(F + kWaveZ * kWaveY);
+    __shared__ int s_item;
+    const int t = threadIdx.x, i = t & 31, wi = t >> 5;
+    const int nd = p.nbx + p.nby + p.nbz - 2, nb = p.nbx * p.nby * p.nbz;
+    for (int l = t; l < nd; l += blockDim.x) {   // blocks on diagonal l
+        int c = 0;
+        for (int z = 0; z < p.nbz; z++) {
+            const int m = l - z;
+            if (m < 0) break;
+            c += max(0, min(p.nby - 1, m) - max(0, m - (p.nbx - 1)) + 1);
+        }
+        diag[l] = c;
+    }
+    __syncthreads();
+    if (t == 0) {
+        int sum = 0;
+        for (int l = 0; l < nd; l++) {
+            const int c = diag[l];
+            diag[l] = sum;
+            sum += c;
+        }
+    }
+    const int w = p.w, h = p.h, d = p.d;
+    const long long wh = (long long)w * h, n = wh * d;
+    bool up_ok = true;   // thread 0: no wait has given up
+    for (;;) {
+        __syncthreads();   // the block before is stored, its shared memory free
+        if (t == 0) s_item = (int)atomicAdd(p.counter, 1u);
+        __syncthreads();
+        if (s_item >= 8 * nb) return;
+        const WaveBlock b = wave_block(p, diag, s_item);
+        const int sx = b.plane & 1, sy = (b.plane >> 1) & 1, sz = (b.plane >> 2) & 1;
+        float* out = p.planes + b.plane * n;
+        const int i0 = b.bx * 32, j0 = b.by * kWaveY, k0 = b.bz * kWaveZ;
+        const int ni = min(32, w - i0), nj = min(kWaveY, h - j0), nk = min(kWaveZ, d - k0);
+        // row (j, k) of the block in memory order: its cells lie at row + 0 .. ni - 1
+        const int xm = sx ? w - i0 - ni : i0;
+        auto row_at = [&](int j, int k) -> float* {
+            return out + ((long long)(sz ? d - 1 - k : k) * h + (sy ? h - 1 - j : j)) * w + xm;
+        };
+        // column i's place in a staged row
+        auto place = [&](int c) { return sx ? ni - 1 - c : c; };
+        // stage the block; only this CTA writes these cells
+        const bool vec = ni == 32 && ((uintptr_t)row_at(j0, k0) & 15) == 0 && (w & 3) == 0;
+        if (vec) {
+            for (int r = t; r < nj * nk * 8; r += blockDim.x) {
+                const int q = r & 7, row = r >> 3, k = row / nj, j = row - k * nj;
+                const float* src = row_at(j0 + j, k0 + k) + 4 * q;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                                 (uint32_t)__cvta_generic_to_shared(T + (k * kWaveY + j) * 32 + 4 * q)),
+                             "l"(src)
+                             : "memory");
+            }
+        } else {
+            for (int row = wi; row < nj * nk; row += kWaveThreads / 32) {
+                const int k = row / nj, j = row - k * nj;
+                if (i < ni)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                                     (uint32_t)__cvta_generic_to_shared(T + (k * kWaveY + j) * 32 + i)),
+                                 "l"(row_at(j0 + j, k0 + k) + i)
+                                 : "memory");
+            }
+        }
+        // the three blocks before this one
+        if (t == 0) {
+            const unsigned* f = p.done + (long long)b.plane * nb + ((long long)b.bz * p.nby + b.by) * p.nbx + b.bx;
+            const unsigned* pre[3] = {b.bx ? f - 1 : nullptr, b.by ? f - p.nbx : nullptr,
+                                      b.bz ? f - (long long)p.nbx * p.nby : nullptr};
+            for (int a = 0; a < 3; a++) {
+                if (!pre[a]) continue;
+                for (unsigned polls = 0;; polls++) {
+                    unsigned v;
+                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(pre[a]) : "memory");
+                    if (v) break;
+                    if (!up_ok || polls >= (1u << 22)) {
+                        if (up_ok) atomicExch(p.err, 1);
+                        up_ok = false;
+                        break;
+                    }
+                    __nanosleep(32);
+                }
+            }
+        }
+        __syncthreads();
+        // their faces: L2-coherent loads
+        for (int r = wi; r < nk; r += kWaveThreads / 32)
+            U[r * 32 + i] = j0 && i < ni ? __ldcg(row_at(j0 - 1, k0 + r) + place(i)) : 0.0f;
+        for (int r = t; r < nk * kWaveY; r += blockDim.x) {
+            const int k = r / kWaveY, j = r - k * kWaveY;
+            F[r] = i0 && j < nj ? __ldcg(row_at(j0 + j, k0 + k) + (sx ? ni : -1)) : 0.0f;
+        }
+        float v[kWaveM];   // the value of the step before, at first "back" of slice 0
+#pragma unroll
+        for (int m = 0; m < kWaveM; m++) {
+            const int j = wi * kWaveM + m;
+            v[m] = k0 && i < ni && j < nj ? __ldcg(row_at(j0 + j, k0 - 1) + place(i)) : 0.0f;
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        const int S = nk + ni - 1 + nj - 1;
+        const int my_rows = i < ni ? min(kWaveM, nj - wi * kWaveM) : 0;
+        // row m's cell of slice k at cell[k * kPitch + m * 32]; its left
+        // neighbour in the block, or, for lane 0, in the face beside it; the
+        // first row's upper neighbour likewise
+        constexpr int kPitch = kWaveY * 32;
+        const int me = place(i < ni ? i : 0);
+        float* cell = T + wi * kWaveM * 32 + me;
+        const float* leftc = i ? cell + (sx ? 1 : -1) : F + wi * kWaveM;
+        const int left_pitch = i ? kPitch : kWaveY, left_row = i ? 32 : 1;
+        const float* upc = wi ? cell - 32 : U + (i < ni ? i : 0);
+        const int up_pitch = wi ? kPitch : 32;
+        int first_k = 0;
+        if (i0 + j0 + k0 == 0 && t == 0) {   // the plane's starting cell keeps its value
+            v[0] = *cell;
+            first_k = 1;
+        }
+        float left[kWaveM], own[kWaveM], u0 = 0.0f;
+#pragma unroll
+        for (int m = 0; m < kWaveM; m++) left[m] = own[m] = 0.0f;
+        int k = -i - wi * kWaveM;   // the slice of row 0; row m is m slices behind
+        cell += k * kPitch;
+        leftc += k * left_pitch;
+        upc += k * up_pitch;
+        for (int s = 0; s < S; s++) {
+            // all loads of the step before any of its stores: the rows are
+            // independent within a step
+            bool on[kWaveM];
+#pragma unroll
+            for (int m = 0; m < kWaveM; m++) {
+                on[m] = m < my_rows && (m ? (unsigned)(k - m) < (unsigned)nk
+                                          : (unsigned)(k - first_k) < (unsigned)(nk - first_k));
+                if (on[m]) {
+                    own[m] = cell[m * (32 - kPitch)];
+                    left[m] = leftc[m * (left_row - left_pitch)];
+                }
+            }
+            if (on[0]) u0 = *upc;
+#pragma unroll
+            for (int m = kWaveM - 1; m >= 0; m--) {
+                const float nv = occ_update(own[m], oct_combine(left[m], m ? v[m > 0 ? m - 1 : 0] : u0, v[m]));
+                if (on[m]) {
+                    cell[m * (32 - kPitch)] = nv;
+                    v[m] = nv;
+                }
+            }
+            k++;
+            cell += kPitch;
+            leftc += left_pitch;
+            upc += up_pitch;
+            __syncthreads();
+        }
+        if (vec) {
+            for (int r = t; r < nj * nk * 8; r += blockDim.x) {
+                const int q = r & 7, row = r >> 3, k = row / nj, j = row - k * nj;
+                *reinterpret_cast<float4*>(row_at(j0 + j, k0 + k) + 4 * q) =
+                    *reinterpret_cast<const float4*>(T + (k * kWaveY + j) * 32 + 4 * q);
+            }
+        } else {
+            for (int row = wi; row < nj * nk; row += kWaveThreads / 32) {
+                const int k = row / nj, j = row - k * nj;
+                if (i < ni) row_at(j0 + j, k0 + k)[i] = T[(k * kWaveY + j) * 32 + i];
+            }
+        }
+        __syncthreads();
+        if (t == 0) {
+            __threadfence();
+            asm volatile("st.release.gpu.global.u32 [%0], 1;" ::"l"(
+                             p.done + (long long)b.plane * nb + ((long long)b.bz * p.nby + b.by) * p.nbx + b.bx)
+                         : "memory");
+        }
+    }
+}
+
+static bool occ_wave3(float* dirw, int w, int h, int d, int* err, size_t cap, cudaStream_t st)
+{
+    OccWave p{dirw, nullptr, nullptr, err, w, h, d, (w + 31) / 32, (h + kWaveY - 1) / kWaveY, (d + kWaveZ - 1) / kWaveZ};
+    const long long nb = (long long)p.nbx * p.nby * p.nbz;
+    const int nd = p.nbx + p.nby + p.nbz - 2;
+    const size_t smem = ((size_t)kWaveZ * kWaveY * 32 + kWaveZ * 32 + kWaveZ * kWaveY + nd) * 4;
+    if (8 * nb > (1 << 28) || smem > 220 * 1024) return false;
+    const size_t bytes = 256 + (size_t)nb * 8 * sizeof(unsigned);
+    if (cap && bytes > cap) return false;
+    cudaFuncSetAttribute(k_occlusion_wave3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(k_occlusion_wave3, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_occlusion_wave3, kWaveThreads, smem) != cudaSuccess ||
+        per_sm < 1)
+        return false;
+    void* scratch = nullptr;
+    if (cudaMallocAsync(&scratch, bytes, st) != cudaSuccess) return false;
+    p.counter = static_cast<unsigned*>(scratch);
+    p.done = p.counter + 64;
+    cudaMemsetAsync(scratch, 0, bytes, st);
+    const long long grid = min((long long)per_sm * g_num_sms, 8 * nb);
+    k_occlusion_wave3<<<(int)grid, kWaveThreads, smem, st>>>(p);
+    cudaFreeAsync(scratch, st);
+    return true;
+}
+
 void launch_init_dirw(int dim, const uint32_t* mask, float* dirw, int w, int h, int d, cudaStream_t st)
 {
     const long long rows = (long long)h * (dim == 3 ? d : 1);
@@ -452,7 +717,8 @@ static void occ_blocks3(float* dirw, const float* in, int w, int h, int d, int b
         k_occlusion_blocks3<IO, BY><<<grid, block, 0, st>>>(dirw, in, w, h, d, bzs, nb, ax0, ax1, L);
 }
 
-void launch_occlusion_sweep(int dim, float* dirw, const float* in, int w, int h, int d, cudaStream_t st)
+void launch_occlusion_sweep(int dim, float* dirw, const float* in, int w, int h, int d, int* err, size_t scratch_cap,
+                            cudaStream_t st)
 {
     ProfScope ps(in ? "occlusion_sweep_io" : "occlusion_sweep", st);
     const int t = tune_get(kTuneOcc, w);
@@ -460,7 +726,10 @@ void launch_occlusion_sweep(int dim, float* dirw, const float* in, int w, int h,
         occ_planes(dim, dirw, in, w, h, d, st);
     } else if (dim == 2) {
         occ_tiles2(dirw, w, h, st);
+    } else if (t == 0 && !in && occ_wave3(dirw, w, h, d, err, scratch_cap, st)) {
+        // one launch
     } else {
+        cudaGetLastError();
         // t > 1: slices per block (t % 1000); t >= 1000: blocks of 32 rows instead of 16
         const int bzs = t > 1 && t % 1000 ? min(t % 1000, 1024) : (d >= 256 ? 64 : kOccSlicesPerBlock);
         const bool rows32 = t >= 1000;

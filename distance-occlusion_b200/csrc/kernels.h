@@ -145,7 +145,8 @@ void launch_init_dirw(int dim, const uint32_t* mask, float* dirw, int w, int h, 
 // that many slices, plus 1000 = blocks of 32 x 32 columns
 constexpr int kOccSlicesPerBlock = 32;
 constexpr int kOccPlaneMaxWidth = 4096;
-void launch_occlusion_sweep(int dim, float* dirw, const float* in, int w, int h, int d, cudaStream_t st);
+void launch_occlusion_sweep(int dim, float* dirw, const float* in, int w, int h, int d, int* err, size_t scratch_cap,
+                            cudaStream_t st);
 
 // k_voxel.cu -- triangles to bitmask (ORed into mask); bbox: min xyz, max xyz (host)
 void launch_voxelize(int tri_count, const int* indices, const float* verts, const float bbox[6], int w, int h, int d,
