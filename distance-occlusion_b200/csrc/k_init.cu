@@ -65,13 +65,16 @@ __global__ void k_init_deltas(const uint32_t* __restrict__ mask, void* __restric
     long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
     for (long long base = warp * 32; base < nwords; base += nwarps * 32) {
         uint32_t mine = base + lane < nwords ? (mask[base + lane] ^ invert) : 0u;
+        // each lane finds its own word's cells (a division), the others get them by shuffle
+        long long my_first;
+        int my_n;
+        word_cells(base + lane, w, ws, &my_first, &my_n);
         for (int q = 0; q < 32; q++) {
             long long wid = base + q;
             if (wid >= nwords) break;
             uint32_t word = __shfl_sync(0xFFFFFFFFu, mine, q);
-            long long first;
-            int n;
-            word_cells(wid, w, ws, &first, &n);
+            const long long first = __shfl_sync(0xFFFFFFFFu, my_first, q);
+            const int n = __shfl_sync(0xFFFFFFFFu, my_n, q);
             if (lane < n) {
                 bool on = (word >> lane) & 1u;
                 long long c = first + lane;
@@ -108,6 +111,9 @@ __global__ void __launch_bounds__(256) k_init_border(const uint32_t* __restrict_
     long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
     for (long long base = warp * 32; base < nwords; base += nwarps * 32) {
         long long wid = base + lane;
+        long long my_first;
+        int my_n;
+        word_cells(wid, w, ws, &my_first, &my_n);
         if (wid < nwords) {
             long long row = wid / ws;
             int k = (int)(wid - row * ws);
@@ -127,9 +133,8 @@ __global__ void __launch_bounds__(256) k_init_border(const uint32_t* __restrict_
         for (int q = 0; q < 32; q++) {
             long long wq = base + q;
             if (wq >= nwords) break;
-            long long first;
-            int n;
-            word_cells(wq, w, ws, &first, &n);
+            const long long first = __shfl_sync(0xFFFFFFFFu, my_first, q);
+            const int n = __shfl_sync(0xFFFFFFFFu, my_n, q);
             if (lane < n) {
                 const uint32_t* s = planes[wib][q];
                 if (kDim == 2) {

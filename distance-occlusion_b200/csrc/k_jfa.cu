@@ -6,7 +6,10 @@
 // exactly.  The driver keeps the reference's pass schedule: steps from
 // FloorPow2(max dim - 1) halving to 1, plus one extra step-1 pass back into the
 // caller's buffer when the last result sits in the ping-pong buffer.
+#include <limits.h>
+
 #include "common.cuh"
+#include "grid_barrier.cuh"
 #include "kernels.h"
 
 namespace dolk {
@@ -198,6 +201,180 @@ __global__ void __launch_bounds__(512) k_jfa3z(const void* __restrict__ in, void
     }
 }
 
+// ---- packed 3D passes ---------------------------------------------------------------------
+//
+// A neighbour's candidate is its delta plus the offset to it, that is, the
+// distance from this cell to the neighbour's site; cells at max (25000) are
+// skipped and so stay as they are.  So a pass can keep sites instead of deltas:
+// one 32-bit word per cell, the site's position in units of the cell width
+// (cw * cell + delta, plus 1: border deltas reach one unit outside), 10 + 10 + 11
+// bits, or kNoSite for a cell at max.  The squared length of a candidate is then
+// exact integer arithmetic on positions with no int16 in between.
+//
+// Fields whose sides stay within kSiteSpan units qualify; there a site is less
+// than 2^21 away in square and kNoSite's position more, so a cell without a
+// site loses to any real one without a test.  Initial deltas always have this
+// form; the caller's own are checked by the conversion (k_jfa3_pack), and if
+// one does not, the packed passes do nothing and k_jfa3_general runs the
+// passes on the cells as they are.
+//
+// What bounds a pass: integer instructions.  Walking z (as k_jfa3z) a neighbour
+// is unpacked once for the three cells that read it; each of them costs a
+// multiply-add and a share of a three-way min of length * 256 + order, the order being
+// the reference's (own cell first, z outermost, x innermost), so that ties fall
+// as there, and the winner's word is read again at the end.  256^3, a pass:
+// 0.30 ms on 8-byte deltas with a compare and five selects per candidate,
+// 0.16 ms.
+constexpr int kSiteSpan = 600;
+constexpr uint32_t kNoSite = 0xFFFFFFFFu;   // at (1023, 1023, 2047)
+
+__device__ __forceinline__ uint32_t pack_site(int x, int y, int z)
+{
+    return (uint32_t)x | ((uint32_t)y << 10) | ((uint32_t)z << 21);
+}
+
+// deltas -> sites; *odd is set when a cell has no site in range and is not at max
+__global__ void __launch_bounds__(256) k_jfa3_pack(const int16_t* __restrict__ in, uint32_t* __restrict__ out, int w,
+                                                   int h, int d, int cw, int* __restrict__ odd)
+{
+    bool bad = false;
+    const int rows = h * d, lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
+    for (int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < rows; row += nw) {
+        const int z = row / h, y = row - z * h;
+        for (int x = lane; x < w; x += 32) {
+            const int i = row * w + x;
+            const C3 c = load3(in, i);
+            const int px = c.x + cw * x + 1, py = c.y + cw * y + 1, pz = c.z + cw * z + 1;
+            const bool none = c.x == kMax3 && c.y == kMax3 && c.z == kMax3;
+            if (!none)
+                bad |= (unsigned)px > (unsigned)(cw * (w - 1) + 2) || (unsigned)py > (unsigned)(cw * (h - 1) + 2) ||
+                       (unsigned)pz > (unsigned)(cw * (d - 1) + 2);
+            out[i] = none ? kNoSite : pack_site(px & 1023, py & 1023, pz & 1023);
+        }
+    }
+    if (odd && __any_sync(0xFFFFFFFFu, bad) && lane == 0) *odd = 1;
+}
+
+template <bool kLast>
+__global__ void __launch_bounds__(512) k_jfa3p(const uint32_t* __restrict__ in, void* __restrict__ out, int w, int h,
+                                               int d, int s, int cw, int nchunk, const int* __restrict__ odd)
+{
+    if (odd && *odd) return;
+    const int x = blockIdx.x * 32 + (threadIdx.x & 31);
+    const int y = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (x >= w || y >= h) return;
+    const int r = blockIdx.z / nchunk, chunk = blockIdx.z % nchunk;
+    const int m = (d - r + s - 1) / s;   // cells r + i s < d
+    const int i0 = chunk * kJfaChunk, i1 = min(m, i0 + kJfaChunk);
+    if (i0 >= i1) return;
+    const int plane = w * h;
+    const int col = y * w + x;
+    const int cx = cw * x + 1, cy = cw * y + 1;
+    // the slice's nine neighbours; one outside the field stands for the middle
+    // one, a candidate anyway
+    const int oy[3] = {y - s >= 0 ? -s * w : 0, 0, y + s < h ? s * w : 0};
+    const int ox[3] = {x - s >= 0 ? -s : 0, 0, x + s < w ? s : 0};
+    __shared__ int s_off[9][512];
+#pragma unroll
+    for (int n = 0; n < 9; n++) s_off[n][threadIdx.x] = oy[n / 3] + ox[n % 3];
+    // a cell's best so far: length * 256 + order (0: its own site)
+    int kA = INT_MAX, kB = INT_MAX, kC = INT_MAX;
+    // the cells s slices away from this slice's: (d +- t)^2 = d^2 +- 2 t d + t^2, in units of 1/16
+    const int t = 16 * cw * s, t2 = t * t;
+    for (int j = i0 - 1; j <= i1; j++) {
+        kC = INT_MAX;   // cell j + 1 starts here
+        if (j >= 0 && j < m) {
+            const uint32_t* slice = in + ((r + j * s) * plane + col);
+            const int zB = 16 * (cw * (r + j * s) + 1);
+            int vA[9], vB[9], vC[9];   // cells j - 1, j, j + 1 (A, C less t2)
+#pragma unroll
+            for (int n = 0; n < 9; n++) {
+                const uint32_t p = __ldg(slice + (oy[n / 3] + ox[n % 3]));
+                const int dx = (int)(p & 1023u) * 16 - 16 * cx, dy = (int)((p >> 10) & 1023u) * 16 - 16 * cy;
+                const int dz = (int)(p >> 21) * 16 - zB;
+                const int b = dz * dz + (dy * dy + (dx * dx + n));
+                vA[n] = dz * (2 * t) + b;
+                vB[n] = b;
+                vC[n] = dz * (-2 * t) + b;
+            }
+            auto min9 = [](const int (&v)[9]) {
+                return __vimin3_s32(__vimin3_s32(v[0], v[1], v[2]), __vimin3_s32(v[3], v[4], v[5]),
+                                    __vimin3_s32(v[6], v[7], v[8]));
+            };
+            const int own = vB[4] & ~255;
+            kC = min9(vC) + t2 + 1;                              // orders 1 .. 9: the slice below
+            vB[4] = vB[3];
+            kB = __vimin3_s32(kB, min9(vB) + 10, own);           // 10 .. 18: its own slice
+            kA = min(kA, min9(vA) + t2 + 19);                    // 19 .. 27: the slice above
+        }
+        if (j - 1 >= i0) {   // cell j - 1 has seen its three slices
+            const int z = r + (j - 1) * s, idx = z * plane + col;
+            const int o = (kA & 255) - 1;    // -1: its own
+            int from = idx;
+            if (o >= 0) {
+                const int sl = (o * 57) >> 9;      // o / 9
+                from = idx + (sl - 1) * (s * plane) + s_off[o - 9 * sl][threadIdx.x];
+            }
+            const uint32_t p = __ldg(in + from);
+            if (kLast) {
+                const C3 c = p == kNoSite ? C3{kMax3, kMax3, kMax3}
+                                          : C3{(int)(p & 1023u) - cx, (int)((p >> 10) & 1023u) - cy,
+                                               (int)(p >> 21) - (cw * z + 1)};
+                store3(static_cast<int16_t*>(out), idx, c);
+            } else {
+                static_cast<uint32_t*>(out)[idx] = p;
+            }
+        }
+        kA = kB;
+        kB = kC;
+    }
+}
+
+// All passes on the cells as they are, between the caller's array and one buffer
+// (the schedule has an even number of passes), in one cooperative launch, when
+// the conversion found a cell that the packed passes cannot hold.
+struct JfaSteps {
+    int n, s[40];
+};
+__global__ void __launch_bounds__(256) k_jfa3_general(int16_t* cells, uint2* buf, int w, int h, int d, int cw,
+                                                      JfaSteps st, const int* odd, unsigned* count, int* err)
+{
+    if (!*odd) return;
+    const long long plane = (long long)w * h, n = plane * d;
+    unsigned passed = 0;
+    for (int pass = 0; pass < st.n; pass++) {
+        const int s = st.s[pass];
+        const bool out = (pass & 1) == 0;   // to the buffer
+        auto ld = [&](long long i) -> C3 {
+            if (out) return C3{__ldcg(cells + 3 * i), __ldcg(cells + 3 * i + 1), __ldcg(cells + 3 * i + 2)};
+            const uint2 u = __ldcg(buf + i);
+            return C3{(int)(int16_t)(u.x & 0xFFFFu), (int)(int16_t)(u.x >> 16), (int)(int16_t)(u.y & 0xFFFFu)};
+        };
+        for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+            const int z = (int)(i / plane), y = (int)((i - z * plane) / w), x = (int)(i - z * plane - (long long)y * w);
+            C3 best = ld(i);
+            int32_t bl = len(best);
+            for (int iz = -1; iz <= 1; iz++)
+                for (int iy = -1; iy <= 1; iy++)
+                    for (int ix = -1; ix <= 1; ix++) {
+                        const int nz = z + iz * s, ny = y + iy * s, nx = x + ix * s;
+                        if (nz < 0 || nz >= d || ny < 0 || ny >= h || nx < 0 || nx >= w) continue;
+                        const C3 c = ld(nz * plane + (long long)ny * w + nx);
+                        if (c.x == kMax3) continue;
+                        const C3 cand = add(c, cw * s * ix, cw * s * iy, cw * s * iz);
+                        const int32_t cl = len(cand);
+                        if (bl > cl) {
+                            best = cand;
+                            bl = cl;
+                        }
+                    }
+            if (out) store3w(buf, i, best);
+            else store3(cells, i, best);
+        }
+        if (pass + 1 < st.n && !grid_barrier(count, passed, err)) return;
+    }
+}
+
 size_t jumpflood_workspace_bytes(int dim, int w, int h, int d)
 {
     const size_t cells = (size_t)w * h * (dim == 3 ? d : 1);
@@ -215,7 +392,56 @@ static int floor_pow2(int v)
     return (v + 1) >> 1;
 }
 
-void launch_jumpflood(int dim, void* deltas, void* temp, int w, int h, int d, int cw, cudaStream_t st)
+// The packed passes in the workspace of the 8-byte ones: their two buffers take
+// the first half, the check's flag and the general passes' barrier the start of
+// the second.
+static bool run_packed(void* deltas, void* temp, size_t half, int w, int h, int d, int cw, const int* steps, int np,
+                       int ry, bool checked, int* err, cudaStream_t st)
+{
+    const size_t cells = (size_t)w * h * d;
+    uint32_t* pb[2] = {static_cast<uint32_t*>(temp), static_cast<uint32_t*>(temp) + cells};
+    unsigned* words = reinterpret_cast<unsigned*>(static_cast<char*>(temp) + half);   // the second buffer's start
+    int* odd = checked ? nullptr : reinterpret_cast<int*>(words);
+    JfaSteps js;
+    js.n = np;
+    for (int i = 0; i < np; i++) js.s[i] = steps[i];
+    int per_sm = 0;
+    if (!checked) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_jfa3_general, 256, 0) != cudaSuccess || per_sm < 1)
+            return false;
+        cudaMemsetAsync(odd, 0, 2 * sizeof(unsigned), st);
+    }
+    const int warps = h * d;
+    k_jfa3_pack<<<min((warps + 7) / 8, g_num_sms * 16), 256, 0, st>>>(static_cast<const int16_t*>(deltas), pb[0], w, h, d,
+                                                                     cw, odd);
+    for (int i = 0; i < np; i++) {
+        ProfScope ps("jumpflood_pass", st);
+        const int sv = steps[i], nres = sv < d ? sv : d;
+        const int nchunk = ((d + sv - 1) / sv + kJfaChunk - 1) / kJfaChunk;
+        const dim3 gz((w + 31) / 32, (h + ry - 1) / ry, (unsigned)(nres * nchunk));
+        if (i == np - 1)
+            k_jfa3p<true><<<gz, 32 * ry, 0, st>>>(pb[i & 1], deltas, w, h, d, sv, cw, nchunk, odd);
+        else
+            k_jfa3p<false><<<gz, 32 * ry, 0, st>>>(pb[i & 1], pb[(i & 1) ^ 1], w, h, d, sv, cw, nchunk, odd);
+    }
+    if (!checked) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)min((long long)per_sm * g_num_sms, (long long)(cells + 255) / 256));
+        cfg.blockDim = dim3(256);
+        cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        cudaLaunchKernelEx(&cfg, k_jfa3_general, static_cast<int16_t*>(deltas), static_cast<uint2*>(temp), w, h, d, cw, js,
+                           (const int*)odd, words + 1, err);
+    }
+    return true;
+}
+
+void launch_jumpflood(int dim, void* deltas, void* temp, int w, int h, int d, int cw, bool initial, int* err,
+                      cudaStream_t st)
 {
     int m = w > h ? w : h;
     if (dim == 3 && d > m) m = d;
@@ -243,8 +469,13 @@ void launch_jumpflood(int dim, void* deltas, void* temp, int w, int h, int d, in
         }
         return;
     }
-    // 3D: the caller's 6-byte cells -> 8-byte ping-pong buffers -> the caller's cells
     const size_t cells = (size_t)w * h * d;
+    const size_t half = ((cells * sizeof(uint2)) + 255) & ~(size_t)255;
+    // sites in 32 bits: sides within the packed positions' range
+    if (!per_cell && np > 0 && (long long)cw * (m - 1) + 2 <= kSiteSpan && ((uintptr_t)temp & 7) == 0 &&
+        run_packed(deltas, temp, half, w, h, d, cw, steps, np, ry, initial, err, st))
+        return;
+    // 3D: the caller's 6-byte cells -> 8-byte ping-pong buffers -> the caller's cells
     uint2* wb[2] = {static_cast<uint2*>(temp),
                     reinterpret_cast<uint2*>(static_cast<char*>(temp) + (((cells * sizeof(uint2)) + 255) & ~(size_t)255))};
     const dim3 grid((w + 31) / 32, (h + ry - 1) / ry, d);
@@ -278,44 +509,102 @@ void launch_jumpflood(int dim, void* deltas, void* temp, int w, int h, int d, in
 
 // ---- deltas -> distances (DistanceOcclusionTool.cpp:46-61, sign :1262/:1392) ----
 
-template <int kDim>
+// A warp takes 256 cells of a row, eight at a time per lane in flight (a division
+// per 256 cells instead of one per cell, and the sign bits of 32 cells are one
+// word).  256^3: 76 us with a flat index and a division per cell, 60 us.
+template <int kDim, bool kHalve>
 __global__ void __launch_bounds__(256) k_deltas_to_dist(const void* __restrict__ deltas, int cw,
                                                         const uint32_t* __restrict__ sign_mask, float* __restrict__ out,
-                                                        int w, long long rows)
+                                                        int w, long long items, int segs)
 {
-    const int ws = words_per_row(w);
-    const long long n = rows * w;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        int32_t l;
-        if (kDim == 2) {
-            l = len(unpack2(__ldg(static_cast<const uint32_t*>(deltas) + i)));
-        } else {
-            l = len(load3(static_cast<const int16_t*>(deltas), i));
+    const int ws = words_per_row(w), lane = threadIdx.x & 31;
+    const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
+    for (long long it = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < items; it += warps) {
+        const long long row = items < (1LL << 31) ? (long long)((unsigned)it / (unsigned)segs) : it / segs;
+        const int x0 = (int)(it - row * segs) * 256;
+        const long long first = row * w + x0;
+        int32_t l[8];
+        uint32_t sign[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const int x = 32 * u + lane;
+            l[u] = 0;
+            sign[u] = 0;
+            if (x0 + x < w) {
+                if (kDim == 2) l[u] = len(unpack2(__ldg(static_cast<const uint32_t*>(deltas) + first + x)));
+                else l[u] = len(load3(static_cast<const int16_t*>(deltas), first + x));
+                if (sign_mask) sign[u] = (__ldg(sign_mask + row * ws + (x0 >> 5) + u) >> lane) << 31;
+            }
         }
-        float r = sqrtf((float)l);
-        if (cw != 1) r = __fdiv_rn(r, (float)cw);
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const int x = 32 * u + lane;
+            float r = sqrtf((float)l[u]);
+            // half of a square root of an integer is exact: the division by 2 in one multiplication
+            if (kHalve) r = __fmul_rn(r, 0.5f);
+            else if (cw != 1) r = __fdiv_rn(r, (float)cw);
+            if (x0 + x < w) out[first + x] = __uint_as_float(__float_as_uint(r) ^ sign[u]);
+        }
+    }
+}
+
+// The same for volumes of rows of whole fours at 8- and 16-byte aligned arrays: a
+// lane takes four cells as three 8-byte loads and stores them as one float4
+// (256^3: 60 us with 2-byte loads, 35 us).
+template <bool kHalve>
+__global__ void __launch_bounds__(256) k_deltas_to_dist4(const uint2* __restrict__ deltas, int cw,
+                                                         const uint32_t* __restrict__ sign_mask,
+                                                         float4* __restrict__ out, int w4, long long n4)
+{
+    const int ws = words_per_row(4 * w4);
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
+        const uint2 a = __ldg(deltas + 3 * i), b = __ldg(deltas + 3 * i + 1), c = __ldg(deltas + 3 * i + 2);
+        auto lo = [](uint32_t v) { return (int)(int16_t)v; };
+        auto hi = [](uint32_t v) { return (int)v >> 16; };
+        const int32_t l[4] = {len(C3{lo(a.x), hi(a.x), lo(a.y)}), len(C3{hi(a.y), lo(b.x), hi(b.x)}),
+                              len(C3{lo(b.y), hi(b.y), lo(c.x)}), len(C3{hi(c.x), lo(c.y), hi(c.y)})};
+        uint32_t sign = 0;
         if (sign_mask) {
-            long long row = i / w;
-            int x = (int)(i - row * w);
-            if ((__ldg(sign_mask + row * ws + (x >> 5)) >> (x & 31)) & 1u) r = -r;
+            const unsigned row = n4 < (1LL << 31) ? (unsigned)i / (unsigned)w4 : (unsigned)(i / w4);
+            const unsigned x = (unsigned)(i - (long long)row * w4) * 4;
+            sign = __ldg(sign_mask + (long long)row * ws + (x >> 5)) >> (x & 31);
         }
-        out[i] = r;
+        float r[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            r[u] = sqrtf((float)l[u]);
+            if (kHalve) r[u] = __fmul_rn(r[u], 0.5f);
+            else if (cw != 1) r[u] = __fdiv_rn(r[u], (float)cw);
+            r[u] = __uint_as_float(__float_as_uint(r[u]) ^ (sign >> u << 31));
+        }
+        out[i] = make_float4(r[0], r[1], r[2], r[3]);
     }
 }
 
 void launch_deltas_to_dist(int dim, const void* deltas, int cw, const uint32_t* sign_mask, float* out, int w, int h,
                            int d, cudaStream_t st)
 {
-    long long rows = (long long)h * (dim == 3 ? d : 1);
-    long long n = rows * w;
-    long long blocks = (n + 255) / 256;
-    long long cap = (long long)g_num_sms * 32;
-    int grid = (int)(blocks < cap ? blocks : cap);
+    const int segs = (w + 255) / 256;
+    const long long items = (long long)h * (dim == 3 ? d : 1) * segs;
+    const long long blocks = (items + 7) / 8, cap = (long long)g_num_sms * 32;
+    const int grid = (int)(blocks < cap ? blocks : cap);
     ProfScope ps("deltas_to_dist", st);
-    if (dim == 2)
-        k_deltas_to_dist<2><<<grid, 256, 0, st>>>(deltas, cw, sign_mask, out, w, rows);
-    else
-        k_deltas_to_dist<3><<<grid, 256, 0, st>>>(deltas, cw, sign_mask, out, w, rows);
+    if (dim == 3 && w % 4 == 0 && ((uintptr_t)deltas & 7) == 0 && ((uintptr_t)out & 15) == 0) {
+        const long long n4 = (long long)(w / 4) * h * d, b4 = (n4 + 255) / 256;
+        const int g4 = (int)(b4 < cap ? b4 : cap);
+        const uint2* in = static_cast<const uint2*>(deltas);
+        float4* o = reinterpret_cast<float4*>(out);
+        if (cw == 2) k_deltas_to_dist4<true><<<g4, 256, 0, st>>>(in, cw, sign_mask, o, w / 4, n4);
+        else k_deltas_to_dist4<false><<<g4, 256, 0, st>>>(in, cw, sign_mask, o, w / 4, n4);
+        return;
+    }
+    if (dim == 2) {
+        if (cw == 2) k_deltas_to_dist<2, true><<<grid, 256, 0, st>>>(deltas, cw, sign_mask, out, w, items, segs);
+        else k_deltas_to_dist<2, false><<<grid, 256, 0, st>>>(deltas, cw, sign_mask, out, w, items, segs);
+    } else {
+        if (cw == 2) k_deltas_to_dist<3, true><<<grid, 256, 0, st>>>(deltas, cw, sign_mask, out, w, items, segs);
+        else k_deltas_to_dist<3, false><<<grid, 256, 0, st>>>(deltas, cw, sign_mask, out, w, items, segs);
+    }
 }
 
 // ---- two-pass signed distance: Dist(exterior) - Dist(interior) ----

@@ -269,7 +269,7 @@ DOL_API dol_status dol_autotune(int kind, int w, int h, int d, void* stream)
             case kTuneJfa2:
             case kTuneJfa3:
                 launch_init_border(dim, static_cast<uint32_t*>(dm), dl, tw, th, td, st);
-                launch_jumpflood(dim, dl, tmp, tw, th, td, 2, st);
+                launch_jumpflood(dim, dl, tmp, tw, th, td, 2, true, err, st);
                 break;
             case kTuneEdt:
                 launch_edt_mask(3, static_cast<uint32_t*>(dm), static_cast<float*>(dl), tw, th, td, DOL_EDT_SIGNED, ws,
