@@ -89,14 +89,24 @@ def sync(stream=None) -> None:
 
 # ---- helpers ----------------------------------------------------------------------------------
 
+_torch_module = None
+
+
 def _torch():
-    import torch
-    return torch
+    global _torch_module
+    if _torch_module is None:
+        import torch
+        _torch_module = torch
+    return _torch_module
 
 
 def _stream(stream=None):
     if stream is None:
         torch = _torch()
+        if torch.cuda.is_initialized():
+            # the current stream's handle without a Stream object around it: a
+            # small call spends more time in this layer than on its launches
+            return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
         if not torch.cuda.is_available():
             return None
         stream = torch.cuda.current_stream()
@@ -114,7 +124,7 @@ def _ptr(t):
 
 
 def _ints(*xs):
-    return [C.c_int(int(x)) for x in xs]
+    return [int(x) for x in xs]   # (ctypes passes a Python int as a C int)
 
 
 def mask_words(w, h, d=1):
