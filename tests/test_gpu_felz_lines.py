@@ -25,3 +25,28 @@ def test_lines_match_oracle(dol, O, cuda, dims, kind):
     want = O.felzenszwalb(f, dims)
     got = dol.felzenszwalb(cuda.from_numpy(f.copy()).cuda(), dims).cpu().numpy()
     assert np.array_equal(got.view(np.uint32), np.asarray(want, np.float32).view(np.uint32))
+
+
+@pytest.mark.parametrize("dims", [(5, 33), (64, 97), (3, 1500), (33, 260)])
+@pytest.mark.parametrize("kind", ["line", "integers", "near", "bend", "few"])
+def test_lines_with_ties_match_oracle(dol, O, cuda, dims, kind):
+    """Fields whose envelopes tie or nearly tie: collinear heights, small
+    integers, rounding noise on a line, long slightly bent runs, whole lines
+    without a site."""
+    rng = np.random.default_rng(dims[0] * 7 + dims[1])
+    shape = (dims[1], dims[0])
+    y, x = np.mgrid[:shape[0], :shape[1]].astype(np.float64)
+    if kind == "line":         # heights along both passes on one line: everything pops
+        f = 3 * y - y * y
+    elif kind == "integers":
+        f = rng.integers(0, 60, shape) * 1.0
+    elif kind == "near":       # the line plus noise of a unit in the last place
+        f = 0.1 * y + 1000.3 - y * y
+    elif kind == "bend":       # convex by a little, in runs
+        f = 1e-4 * (y % 40) ** 2 - y * y
+    else:
+        f = np.where((rng.random(shape) < 0.02) & (x % 5 < 2), rng.random(shape), np.finfo(np.float32).max)
+    f = f.astype(np.float32)
+    want = O.felzenszwalb(f, dims)
+    got = dol.felzenszwalb(cuda.from_numpy(f.copy()).cuda(), dims).cpu().numpy()
+    assert np.array_equal(got.view(np.uint32), np.asarray(want, np.float32).view(np.uint32))
