@@ -160,7 +160,12 @@ dol_status get_workspace_between(Workspace& ws, void* user, size_t user_bytes, s
         if (cap && need > cap) want = least;
     }
     *bytes = want;
-    return get_workspace(ws, user, user_bytes, want, st);
+    dol_status s = get_workspace(ws, user, user_bytes, want, st);
+    if (s == DOL_ERR_NO_MEMORY && want > least) {   // the device has no room for it either
+        *bytes = least;
+        s = get_workspace(ws, user, user_bytes, least, st);
+    }
+    return s;
 }
 
 inline cudaStream_t S(void* s) { return static_cast<cudaStream_t>(s); }

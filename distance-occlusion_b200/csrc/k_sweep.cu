@@ -9,9 +9,9 @@
 // current one is scanned.  A row of up to 256 cells is one warp's (nothing
 // crosses a barrier), wider rows take one warp per 256 cells.
 //
-// FastSweep 3D (:2186-2260) has more parallelism: row (y, z) of an octant
-// sweep needs only row (y-1, z) and row (y, z-1) of the same sweep, so rows on
-// an anti-diagonal y+z = c are independent.  k_fastsweep3 runs one octant per
+// FastSweep 3D (:2186-2260) runs in k_fastsweep3.cu; here are the forms that need
+// little scratch.  Row (y, z) of an octant sweep needs only row (y-1, z) and row
+// (y, z-1) of the same sweep, so rows on an anti-diagonal y+z = c are independent.  k_fastsweep3 runs one octant per
 // launch with persistent CTAs that claim rows in anti-diagonal order from an
 // atomic counter and wait (bounded) on per-row ready flags.  A row is only
 // claimed by a running CTA and every row it waits on was claimed earlier, so
@@ -413,8 +413,8 @@ void launch_fastsweep_2d(void* deltas, int w, int h, int cw, cudaStream_t st)
 
 size_t fastsweep3_workspace_bytes(int w, int h, int d)
 {
-    const size_t pipe = fastsweep3_pipe_bytes(w, h, d), rows = fastsweep3_workspace_bytes_min(w, h, d);
-    return pipe > rows ? pipe : rows;
+    const size_t columns = fastsweep3_columns_bytes(w, h, d), rows = fastsweep3_workspace_bytes_min(w, h, d);
+    return columns > rows ? columns : rows;
 }
 
 size_t fastsweep3_workspace_bytes_min(int w, int h, int d)
@@ -429,7 +429,7 @@ void launch_fastsweep_3d(void* deltas, int w, int h, int d, int cw, void* ws, si
                          cudaStream_t st)
 {
     if (h < 2 || d < 2) return;   // no row is ever updated (:2208, :2214 start at 1)
-    if (launch_fastsweep_3d_pipe(deltas, w, h, d, cw, ws, ws_bytes, err, st)) return;
+    if (launch_fastsweep_3d_columns(deltas, w, h, d, cw, ws, ws_bytes, err, st)) return;
     cudaGetLastError();
     char* p = static_cast<char*>(ws);
     int* flags = reinterpret_cast<int*>(p);

@@ -127,10 +127,10 @@ void launch_batch_sdf(const void* items, const int* order, int n, const uint32_t
                       int* counter, cudaStream_t st);
 void launch_fastsweep_3d(void* deltas, int w, int h, int d, int cw, void* ws, size_t ws_bytes, int* err,
                          cudaStream_t st);
-// k_fastsweep3.cu -- rows of up to 256 cells; false when it does not apply
-size_t fastsweep3_pipe_bytes(int w, int h, int d);
-bool launch_fastsweep_3d_pipe(void* deltas, int w, int h, int d, int cw, void* ws, size_t ws_bytes, int* err,
-                              cudaStream_t st);
+// k_fastsweep3.cu -- columns streaming along z; false when the workspace is too small
+size_t fastsweep3_columns_bytes(int w, int h, int d);
+bool launch_fastsweep_3d_columns(void* deltas, int w, int h, int d, int cw, void* ws, size_t ws_bytes, int* err,
+                                 cudaStream_t st);
 
 // k_chamfer.cu -- Chamfer 3-4 on int16 / int32 fields
 template <typename T>

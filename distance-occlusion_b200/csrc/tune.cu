@@ -80,10 +80,12 @@ static std::vector<int> candidates(int kind, int w)
             if (w <= (kind == kTuneDan3 ? 256 : 512)) c.push_back(32);
             return c;
         }
-        case kTuneFs3: {   // the slice pipeline, then the anti-diagonal wavefront (negative)
+        case kTuneFs3: {   // streaming columns, then the anti-diagonal wavefront (negative)
             std::vector<int> c;
-            for (int s : {1, 2, 4, 8})
-                if ((w + s - 1) / s <= 256) c.push_back(s);
+            // (any positive value: the cells per thread of the slices that take over on little scratch)
+            for (int most : {128, 256})
+                for (int s : {1, 2, 4, 8})
+                    if (c.empty() && (w + s - 1) / s <= most) c.push_back(s);
             for (int s : {1, 2, 4, 8})
                 if ((w + s - 1) / s <= 256) c.push_back(-s);
             return c;
