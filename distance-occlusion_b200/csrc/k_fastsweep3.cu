@@ -480,7 +480,7 @@ static __device__ void fs3_compute(const Fs3& p, const Fs3Column& c, Fs3Smem& sm
             end = c.chunk_end(p, next++);
         }
         int e = min(steps, smem_wait<20>(&sm.faces, s + 1, sm, p.err));
-        e = min(e, s < p.d ? end : s + kChunk);
+        e = max(s + 1, min(e, s < p.d ? end : s + kChunk));   // (max: a wait gave up)
         if (!wraps)
             fs3_steps<false>(q, v, slice, s, e);
         else
