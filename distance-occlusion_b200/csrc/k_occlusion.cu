@@ -405,10 +405,14 @@ __global__ void __launch_bounds__(32 * BY, 1024 / (32 * BY))
 // block a step earlier; one barrier per step.  The slice index falls with the
 // lane, so the 32 lanes of an access fall in 32 banks.
 //
-// What bounds it: the steps' latency (shuffle, shared load, ten dependent float
-// operations) and lanes that wait for their first slice (32 of 66 steps each).
-// 256^3, 8 planes: 1.73 ms with a launch per diagonal, 0.77 ms.
-constexpr int kWaveY = 16, kWaveZ = 32, kWaveM = 4;
+// What bounds it: the steps' latency (shared loads, ten dependent float
+// operations, a barrier) and lanes that wait for their first slice (46 of 94
+// steps).  256^3, 8 planes: 1.73 ms with a launch per diagonal; 0.77 ms as blocks
+// of 16 rows x 32 slices with 4 rows per lane (12 warps per SM), 0.57 ms with 2,
+// 0.61 ms with 1; 0.57 ms as 16 x 48 with 1 (32 warps per SM), which is ahead of
+// 16 x 32 with 2 on other shapes: 100 x 60 x 300 0.25 against 0.30 ms, 400 x 400 x
+// 30 0.52 against 0.62 ms.  8 x 64: 0.75 ms, 32 x 16: 0.82 ms.
+constexpr int kWaveY = 16, kWaveZ = 48, kWaveM = 1;
 constexpr int kWaveThreads = 32 * kWaveY / kWaveM;
 
 struct OccWave {

@@ -10,7 +10,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dims", [(1, 1, 1), (1, 40, 3), (31, 17, 33), (32, 16, 32), (33, 16, 32), (64, 15, 65),
-                                  (36, 50, 9), (100, 3, 70), (7, 90, 90), (130, 35, 34)])
+                                  (36, 50, 9), (100, 3, 70), (7, 90, 90), (130, 35, 34),
+                                  (32, 16, 48), (33, 17, 49), (5, 16, 97)])
 @pytest.mark.parametrize("kind", ["mask", "weights"])
 def test_wave_matches_oracle(dol, O, cuda, dims, kind):
     rng = np.random.default_rng(sum(dims))
