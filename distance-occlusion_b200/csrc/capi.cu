@@ -362,9 +362,9 @@ static dol_status chamfer_common(int w, int h, void* dist, bool wide, int* multi
     DOL_TRY(check_sweep_width(w));
     DOL_TRY(check_dev_ptr(dist, "dist"));
     if (wide)
-        launch_chamfer_2d<int32_t>(static_cast<int32_t*>(dist), w, h, ds->err_dev, S(stream));
+        launch_chamfer_2d<int32_t>(static_cast<int32_t*>(dist), w, h, ds->err_dev, g_workspace_limit.load(), S(stream));
     else
-        launch_chamfer_2d<int16_t>(static_cast<int16_t*>(dist), w, h, ds->err_dev, S(stream));
+        launch_chamfer_2d<int16_t>(static_cast<int16_t*>(dist), w, h, ds->err_dev, g_workspace_limit.load(), S(stream));
     if (multiplier) *multiplier = 3;
     return launched(wide ? "chamfer_2d_i32" : "chamfer_2d_i16");
 }

@@ -211,7 +211,8 @@ __global__ void __launch_bounds__(1024) k_chamfer2(T* __restrict__ dist, int w, 
 // What bounds it: the barrier and shuffle latency of the 4 R rows a CTA walks
 // and the scan's grid barriers.  1024 x 1024 int16: 0.47 ms when one CTA
 // carried the rows from block to block and each cell searched its window;
-// 0.11 ms now.
+// 0.10 ms now; with blocks of 4, 6, 12 or 16 rows 0.11 - 0.12 ms.  2048 x 2048
+// int32: 0.26 ms (2.87 ms).
 constexpr int kChamferBlockRows = 8;
 
 template <typename K>
@@ -328,15 +329,15 @@ int chamfer_threads(int w)
 }
 
 template <typename T>
-void launch_chamfer_2d(T* dist, int w, int h, int* err, cudaStream_t st)
+void launch_chamfer_2d(T* dist, int w, int h, int* err, size_t scratch_cap, cudaStream_t st)
 {
     using K = typename ChamferKey<T>::K;
     const int threads = chamfer_threads(w);
     ProfScope ps("chamfer_2d", st);
     if (h >= 2 * kChamferBlockRows) {
         const size_t smem = 3 * (size_t)w * sizeof(K);
-        if (smem > 48 * 1024)
-            cudaFuncSetAttribute(k_chamfer_coop<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        // (always: the static shared memory counts towards the 48 KB that need no asking)
+        cudaFuncSetAttribute(k_chamfer_coop<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         int per_sm = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_chamfer_coop<T>, threads, smem);
         // every block's CTA has to be resident: longer blocks for taller fields
@@ -346,7 +347,8 @@ void launch_chamfer_2d(T* dist, int w, int h, int* err, cudaStream_t st)
         const int nb = (h + R - 1) / R;
         void* scratch = nullptr;
         const size_t rows = 2 * (size_t)nb * w * sizeof(K);
-        if (resident > 0 && nb >= 2 && cudaMallocAsync(&scratch, rows + 256, st) == cudaSuccess) {
+        if (resident > 0 && nb >= 2 && (!scratch_cap || rows + 256 <= scratch_cap) &&
+            cudaMallocAsync(&scratch, rows + 256, st) == cudaSuccess) {
             ChamferCoop<K> p{static_cast<K*>(scratch), reinterpret_cast<unsigned*>(static_cast<char*>(scratch) + rows),
                              err, w, h, R, nb};
             cudaMemsetAsync(p.ctl, 0, sizeof(unsigned), st);
@@ -378,8 +380,8 @@ void launch_init_distances_int(const uint32_t* mask, T* dist, int w, long long r
     k_init_distances_int<T><<<(int)(blocks < cap ? blocks : cap), 256, 0, st>>>(mask, dist, w, rows, max_d);
 }
 
-template void launch_chamfer_2d<int16_t>(int16_t*, int, int, int*, cudaStream_t);
-template void launch_chamfer_2d<int32_t>(int32_t*, int, int, int*, cudaStream_t);
+template void launch_chamfer_2d<int16_t>(int16_t*, int, int, int*, size_t, cudaStream_t);
+template void launch_chamfer_2d<int32_t>(int32_t*, int, int, int*, size_t, cudaStream_t);
 template void launch_init_distances_int<int16_t>(const uint32_t*, int16_t*, int, long long, int16_t, cudaStream_t);
 template void launch_init_distances_int<int32_t>(const uint32_t*, int32_t*, int, long long, int32_t, cudaStream_t);
 

@@ -134,7 +134,7 @@ bool launch_fastsweep_3d_columns(void* deltas, int w, int h, int d, int cw, void
 
 // k_chamfer.cu -- Chamfer 3-4 on int16 / int32 fields
 template <typename T>
-void launch_chamfer_2d(T* dist, int w, int h, int* err, cudaStream_t st);
+void launch_chamfer_2d(T* dist, int w, int h, int* err, size_t scratch_cap, cudaStream_t st);
 template <typename T>
 void launch_init_distances_int(const uint32_t* mask, T* dist, int w, long long rows, T max_d, cudaStream_t st);
 
