@@ -485,9 +485,16 @@ int dan_blocks_rows(int dim, int w, int h, int d)
 {
     const int tv = tune_get(kTuneDanRows, w);
     if (tv > 0) return tv >= kDanSerial ? kDanSerial : min(tv, kBlkMaxRows);
-    // tiny fields: the serial engine's launch is cheaper than the rounds
+    // tiny fields: the serial engine's launch is cheaper than the rounds.  Small
+    // images: a row takes the serial engine 0.8 - 1.5 us, the blocks need up to 20
+    // rounds where single shapes fill the image (value noise, lattice 51 | 20, and
+    // 40 points: 64 x 64 76 | 121, 119 us serial, 157 | 156, 105 us in blocks; 64 x
+    // 128 158 | 236, 205 and 285 | 135, 121; 128 x 64 160 | 147, 119 and 156 | 145,
+    // 109; 256 x 32 82 | 100, 88 and 179 | 146, 131; 96 x 96 280 | 346, 252 and
+    // 285 | 219, 146)
     const long long cells = (long long)w * h * (dim == 3 ? d : 1);
     if (cells < 1024 || w > kBlkMaxWidth) return kDanSerial;
+    if (dim == 2 && ((w <= 256 && h <= 32) || (w <= 128 && h <= 64) || (w <= 64 && h <= 128))) return kDanSerial;
     // 8 rows; tall images of several x blocks 16 (1024^2, 100 points: 0.51
     // against 0.62 ms; 501 x 700 noise: 0.53 against 0.43); volumes whose
     // blocks of 4 rows do not outnumber the resident warps by much 4 (101 x 77
@@ -496,15 +503,17 @@ int dan_blocks_rows(int dim, int w, int h, int d)
     return cells <= (1 << 21) ? 4 : 8;
 }
 
-// Cells per lane.  Images of at most 256 columns take one x block (250 x 180
-// noise: 0.22 ms, 0.27 as two), wider ones blocks of 128 (1024^2, 100 points:
+// Cells per lane.  Images of up to 512 columns take x blocks of 64 (256^2 noise,
+// lattice 51: 0.32 ms, 0.35 with 128, 0.44 as one block; 96 x 192 0.37 against
+// 0.49; 400 x 256 0.36 either way), but 128 columns one block (128 x 256 noise,
+// lattice 20: 0.16 against 0.18 ms); wider ones blocks of 128 (1024^2, 100 points:
 // 0.51 ms, 0.64 with 256); volumes blocks of 64 (256^3 boxes and spheres: 8.8
 // ms, 9.4 with 128 and 11.8 with 256), from 512 columns on 128.
 static int dan_blocks_s(int dim, int w)
 {
     int s = tune_get(dim == 2 ? kTuneDan2 : kTuneDan3, w);
     if (s != 2 && s != 4 && s != 8) {
-        if (dim == 2) s = w <= 64 ? 2 : (w <= 128 ? 4 : (w <= 256 ? 8 : 4));
+        if (dim == 2) s = w <= 512 && (w <= 112 || w > 128) ? 2 : 4;
         else s = w < 512 ? 2 : 4;
     }
     return s;

@@ -363,19 +363,22 @@ static int threads_for(int w, int s)
 }
 
 // Cells per lane and warps of a row: 256 cells per warp, fewer per lane for
-// rows that one warp holds with fewer.  Tuning values 4 and 8 set the cells
+// rows that one warp holds with fewer (one for an image's rows of up to 32).
+// Tuning values 4 and 8 set the cells
 // per lane (any other: this rule).
 static void row_shape(int kind, int w, int* s, int* nw)
 {
     const int tv = tune_get(kind, w);
     *s = tv == 4 || tv == 8 ? tv : (w <= 64 ? 2 : (w <= 128 ? 4 : 8));
     if (*s < 8 && w > 32 * *s * 16) *s = 8;
+    if (w <= 32 && tv != 4 && tv != 8 && kind != kTuneDan3) *s = 1;
     const int need = (w + 32 * *s - 1) / (32 * *s);
     *nw = 1;
     while (*nw < need) *nw *= 2;
 }
 
-// every shape row_shape gives, up to 4096 cells: f(S, NW)
+// every shape row_shape gives for images and volumes, up to 4096 cells: f(S, NW);
+// (1, 1) is an image's alone
 #define DOL_ROW_SHAPES(f) \
     f(2, 1) f(4, 1) f(4, 2) f(4, 4) f(4, 8) f(4, 16) f(8, 1) f(8, 2) f(8, 4) f(8, 8) f(8, 16)
 
@@ -397,6 +400,7 @@ void launch_danielsson(int dim, void* deltas, int w, int h, int d, int cw, cudaS
     }
     DOL_ROW_SHAPES(DOL_DAN_CASE)
 #undef DOL_DAN_CASE
+    if (s == 1) run(k_dan_serial<2, 1, 1>, 1, SerialIO<2, 1>::kBytes);
 }
 
 void launch_fastsweep_2d(void* deltas, int w, int h, int cw, cudaStream_t st)
@@ -408,6 +412,7 @@ void launch_fastsweep_2d(void* deltas, int w, int h, int cw, cudaStream_t st)
     if (s == SV && nw == NWV)  \
         k_fastsweep2<SV, NWV><<<1, 32 * NWV, NWV * SerialIO<2, SV>::kBytes, st>>>(deltas, w, h, cw);
     DOL_ROW_SHAPES(DOL_FS_CASE)
+    DOL_FS_CASE(1, 1)
 #undef DOL_FS_CASE
 }
 
@@ -626,14 +631,100 @@ __device__ __noinline__ void batch_item_warp(const BatchItemDev& b, const uint32
 // items with rows over 256 cells, then the narrow images.  A CTA (one per SM)
 // takes queue A items while there are any, the slices' rows in parallel chunks
 // (dan_slices.cuh), or, where a slice does not fit in shared memory, warp 0
-// walking it serially.  Then each group of 4 warps turns to queue B by itself
-// (its own barrier): items with wide rows take the group; the first narrow
-// image it draws switches it to per-warp draining.
-// 4096 images and 64 volumes: 98 ms with every volume walked serially by one
-// warp, 55 ms.
+// walking it serially.  Then it turns to queue B; items with wide rows come
+// first, the first narrow image drawn switches to per-warp draining.
+//   * up to kBatchFew items per CTA: 8 warps take one wide item at a time, 4 cells
+//     per thread (2.7 us a row step: a wide image is a chain of steps, and the
+//     largest ones decide when the batch ends);
+//   * more: each group of 4 warps takes items by itself (its own barrier), 11 us
+//     a step but four images at a time.
+// Milliseconds, 8 warps | groups (images only, sides up to 1024 x 2047): 16 images
+// 5.3 | 8.1 (5.6 with 256 threads per item and as many CTAs as fit), 200 15 | 32
+// (16.4), 900 16 | 42 (17.9), 2000 37 | 43 (39), 4096 71 | 50 (75); 16 warps per
+// item: 20 at 200, 93 at 4096.  4096 images and 64 volumes: 98 ms with every
+// volume walked serially by one warp, 55 ms.
 // counter: [0] queue B, [1] queue A, [2] nv (written by dol_batch_prepare).
 constexpr size_t kBatchSmem = 216 * 1024;
+constexpr int kBatchFew = 16;
 constexpr int kBatchStrip = (int)SerialIO<3, 8>::kBytes;   // a warp's strips in queue B, the widest
+
+// Danielsson of an image with rows of at most S cells per thread by the whole CTA
+// (scan.cuh): a few cells per thread, the next row loaded during this one, each
+// pass posting what the next one needs.
+template <int S>
+__device__ __noinline__ void batch_dan_cta(uint32_t* __restrict__ dl, int w, int h, int cw, ScanShared<C2>& sh)
+{
+    const int t = threadIdx.x;
+    const int nseg = (w + S - 1) / S;
+    const bool active = t < nseg;
+    const int n = active ? min(S, w - t * S) : 0;
+    const long long x0 = (long long)t * S;
+    if (h < 2) return;
+    const int steps = 2 * (h - 1);
+    auto row_of = [&](int i) { return i < h - 1 ? i + 1 : 2 * h - 3 - i; };
+    auto dy_of = [&](int i) { return i < h - 1 ? -cw : cw; };
+    C2 P[S], C[S], V[S], R[S], D[S];
+#pragma unroll
+    for (int s = 0; s < S; s++) P[s] = C[s] = V[s] = R[s] = D[s] = C2{0, 0};
+
+    load_row<C2, S>(P, dl, x0, n);
+    load_row<C2, S>(C, dl, (long long)row_of(0) * w + x0, n);
+#pragma unroll
+    for (int s = 0; s < S; s++) V[s] = closer(C[s], add(P[s], 0, dy_of(0)));
+    int g = 0;
+    if (active) sh.guess[g][t] = seg_edge<C2, S, +1>(V, n);
+    __syncthreads();
+    for (int i = 0; i < steps; i++) {
+        const int y = row_of(i);
+        const bool more = i + 1 < steps;
+        const int dyn = more ? dy_of(i + 1) : 0;
+        if (more) load_row<C2, S>(C, dl, (long long)row_of(i + 1) * w + x0, n);
+        const C2 in0 = (active && t > 0) ? sh.guess[g][t - 1] : V[0];
+        row_pass<C2, S, false, +1>(R, V, t, nseg, n, cw, sh, D, in0, [&](const C2 (&X)[S]) {
+            if (active) sh.guess[g ^ 1][t] = X[0];
+        });
+        g ^= 1;
+        const C2 in1 = (active && t + 1 < nseg) ? sh.guess[g][t + 1] : R[0];
+        row_pass<C2, S, false, -1>(P, R, t, nseg, n, cw, sh, D, in1, [&](const C2 (&X)[S]) {
+            if (more && active)
+                sh.guess[g ^ 1][t] = closer(seg_edge<C2, S, +1>(C, n), add(seg_edge<C2, S, +1>(X, n), 0, dyn));
+        });
+        g ^= 1;
+        store_row<C2, S>(dl, (long long)y * w + x0, P, n);
+        if (more) {
+#pragma unroll
+            for (int s = 0; s < S; s++) V[s] = closer(C[s], add(P[s], 0, dyn));
+        }
+    }
+}
+
+// an item of queue B with rows of more than 256 cells, by the CTA's 8 warps
+__device__ __noinline__ void batch_item_cta(const BatchItemDev& b, const uint32_t* masks, unsigned char* deltas, float* dist,
+                                            unsigned char* smem, RowShared<4>& group)
+{
+    const int warp = threadIdx.x >> 5;
+    const uint32_t* m = masks + b.mask_off;
+    void* dl = deltas + b.delta_off;
+    if (b.d <= 1) {
+        border_warps<2>(m, dl, b.w, b.h, 1, warp, 8);
+        __syncthreads();
+        batch_dan_cta<4>(static_cast<uint32_t*>(dl), b.w, b.h, 2, *reinterpret_cast<ScanShared<C2>*>(smem));
+        __syncthreads();
+        if (dist && b.dist_off >= 0)
+            signed_dist_warps<C2>(m, static_cast<uint32_t*>(dl), dist + b.dist_off, b.w, b.h, warp, 8);
+    } else {
+        border_warps<3>(m, dl, b.w, b.h, b.d, warp, 8);
+        __syncthreads();
+        if (warp < 4) {
+            unsigned char* strip = smem + warp * kBatchStrip;
+            if (b.w <= 512) batch_dan_group<3, 4>(dl, b.w, b.h, b.d, strip, group);
+            else batch_dan_group<3, 8>(dl, b.w, b.h, b.d, strip, group);
+        }
+        __syncthreads();
+        if (dist && b.dist_off >= 0)
+            signed_dist_warps<C3>(m, static_cast<int16_t*>(dl), dist + b.dist_off, b.w, b.h * b.d, warp, 8);
+    }
+}
 
 template <int NW>
 __global__ void __launch_bounds__(32 * NW) k_batch_sdf(const BatchItemDev* __restrict__ items,
@@ -667,9 +758,36 @@ __global__ void __launch_bounds__(32 * NW) k_batch_sdf(const BatchItemDev* __res
             signed_dist_warps<C3>(m, dl, dist + b.dist_off, b.w, b.h * b.d, warp, NW);
         __syncthreads();
     }
+    unsigned char* strip = smem + warp * kBatchStrip;
+    if (n - nv <= kBatchFew * (int)gridDim.x) {
+        if (warp >= 8) return;   // (barriers count the threads that are left)
+        if (threadIdx.x == 0) sh[0].bar = 1;
+        for (;;) {
+            __syncthreads();
+            if (threadIdx.x == 0) s_item[0] = nv + atomicAdd(counter, 1);
+            __syncthreads();
+            const int it = s_item[0];
+            if (it >= n) return;
+            const BatchItemDev b = items[order[it]];
+            if (b.w <= 256) {
+                // narrow images from here on: the first warp takes this item, every warp then drains the queue
+                int mine = warp == 0 ? it : -1;
+                for (;;) {
+                    if (mine < 0) {
+                        int v = 0;
+                        if (lane == 0) v = nv + atomicAdd(counter, 1);
+                        mine = __shfl_sync(0xFFFFFFFFu, v, 0);
+                        if (mine >= n) return;
+                    }
+                    batch_item_warp(items[order[mine]], masks, deltas, dist, strip);
+                    mine = -1;
+                }
+            }
+            batch_item_cta(b, masks, deltas, dist, smem, sh[0]);
+        }
+    }
     const int group = warp >> 2, gw = warp & 3;
     RowShared<4>& gsh = sh[group];
-    unsigned char* strip = smem + warp * kBatchStrip;
     if ((threadIdx.x & 127) == 0) gsh.bar = 1 + group;
     auto sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); };
     for (;;) {
