@@ -489,12 +489,14 @@ int dan_blocks_rows(int dim, int w, int h, int d)
     // images: a row takes the serial engine 0.8 - 1.5 us, the blocks need up to 20
     // rounds where single shapes fill the image (value noise, lattice 51 | 20, and
     // 40 points: 64 x 64 76 | 121, 119 us serial, 157 | 156, 105 us in blocks; 64 x
-    // 128 158 | 236, 205 and 285 | 135, 121; 128 x 64 160 | 147, 119 and 156 | 145,
+    // 128 158 | 236, 205 and 285 | 135, 121; 20 x 400 0.40 and 0.94 ms with lattice
+    // 51; 128 x 64 160 | 147, 119 and 156 | 145,
     // 109; 256 x 32 82 | 100, 88 and 179 | 146, 131; 96 x 96 280 | 346, 252 and
     // 285 | 219, 146)
     const long long cells = (long long)w * h * (dim == 3 ? d : 1);
     if (cells < 1024 || w > kBlkMaxWidth) return kDanSerial;
-    if (dim == 2 && ((w <= 256 && h <= 32) || (w <= 128 && h <= 64) || (w <= 64 && h <= 128))) return kDanSerial;
+    if (dim == 2 && ((w <= 256 && h <= 32) || (w <= 128 && h <= 64) || (w <= 64 && h <= 200) || (w <= 32 && h <= 512)))
+        return kDanSerial;
     // 8 rows; tall images of several x blocks 16 (1024^2, 100 points: 0.51
     // against 0.62 ms; 501 x 700 noise: 0.53 against 0.43); volumes whose
     // blocks of 4 rows do not outnumber the resident warps by much 4 (101 x 77
