@@ -122,7 +122,7 @@ DOL_API dol_status dol_init_border_3d(int w, int h, int d, const uint32_t* mask,
 /* ---- delta propagation (in place) ------------------------------------------------- */
 /* Danielsson (DistanceOcclusionLib.cpp:702-778, :2348-2394).  Large fields
    run as an exact block schedule that needs scratch of
-   dol_danielsson_workspace_size() bytes (about 2.2x the field for volumes);
+   dol_danielsson_workspace_size() bytes (about 2.5x the field for volumes);
    the plain entries allocate it stream-ordered, the _ws entries take the
    caller's (NULL: allocate; too small: DOL_ERR_INVALID_ARG).  Without it --
    the allocation failed or is above the dol_set_workspace_limit cap -- the
@@ -141,14 +141,17 @@ DOL_API dol_status dol_danielsson_3d_ws(int w, int h, int d, dol_delta3* deltas,
 DOL_API int        dol_last_engine(void);
 /* FastSweep (DistanceOcclusionLib.cpp:633-697, :2186-2260) */
 DOL_API dol_status dol_fastsweep_2d(int w, int h, dol_delta2* deltas, int cw, void* stream);
+/* 3D: about 1.2x the field (a copy in tiles and the words that columns hand on);
+   with less -- a caller's workspace, or the dol_set_workspace_limit cap -- down to
+   4 (h d + h + d) bytes and some, the slices run instead: same deltas, slower */
 DOL_API size_t     dol_fastsweep_3d_workspace_size(int w, int h, int d);
 DOL_API dol_status dol_fastsweep_3d(int w, int h, int d, dol_delta3* deltas, int cw,
                             void* workspace, size_t workspace_bytes, void* stream);
 /* JumpFlood (DistanceOcclusionLib.cpp:887-908, :2450-2472); the workspace
    stands for the reference's internal ping-pong buffer: one 4-byte cell per
-   cell in 2D; in 3D two buffers of 8-byte cells (one aligned load per
-   neighbour), the caller's 6-byte cells being read by the first pass and
-   written by the last */
+   cell in 2D; in 3D room for two buffers of 8-byte cells, of which sites packed
+   into 4 bytes take half (sides up to about 1000 cells), the caller's 6-byte
+   cells being read by the first pass and written by the last */
 DOL_API size_t     dol_jumpflood_2d_workspace_size(int w, int h);
 DOL_API size_t     dol_jumpflood_3d_workspace_size(int w, int h, int d);
 DOL_API dol_status dol_jumpflood_2d(int w, int h, dol_delta2* deltas, int cw,
@@ -321,17 +324,18 @@ DOL_API dol_status dol_sites_backward(int dim, int w, int h, int d, int n_sites,
    device and per size bucket (ceil(log2(w))); 0 = the built-in heuristic.
    dol_autotune times every candidate on a synthetic problem of the given shape
    (blocking; it allocates its own scratch) and keeps the fastest. */
-#define DOL_TUNE_DANIELSSON_2D 0   /* CTA engine with 1, 2, 4, 8 cells per thread; 32 = single-warp engine */
+#define DOL_TUNE_DANIELSSON_2D 0   /* cells per lane of a block's rows: 2, 4, 8 (serial rows: 4, 8); others: by width */
 #define DOL_TUNE_DANIELSSON_3D 1
-#define DOL_TUNE_FASTSWEEP_2D  2
-#define DOL_TUNE_FASTSWEEP_3D  3   /* cells per thread 1, 2, 4, 8: the slice pipeline (one CTA per slice in turn);
-                                      -1, -2, -4, -8: the anti-diagonal wavefront of rows */
-#define DOL_TUNE_JUMPFLOOD_2D  4   /* rows per CTA: 2, 4, 8, 16 */
+#define DOL_TUNE_FASTSWEEP_2D  2   /* cells per lane: 4, 8; others: by width */
+#define DOL_TUNE_FASTSWEEP_3D  3   /* positive: streaming columns, and 1, 2, 4, 8 cells per thread of the slices
+                                      that run on little scratch; -1, -2, -4, -8: the anti-diagonal wavefront of
+                                      rows */
+#define DOL_TUNE_JUMPFLOOD_2D  4   /* rows per CTA of a launch per pass: 2, 4, 8, 16; 0: up to 2^22 cells one launch */
 #define DOL_TUNE_JUMPFLOOD_3D  5   /* rows per CTA 2, 4, 8, 16 of the z walk; negative: one thread per cell */
-#define DOL_TUNE_BATCH         6   /* cells per thread: 4 (256 threads) or 8 (128 threads) */
+#define DOL_TUNE_BATCH         6   /* 8: 8 warps per CTA; others: 16 */
 #define DOL_TUNE_EDT           7   /* threads per CTA of the line passes: 256 or 512 */
 #define DOL_TUNE_DANIELSSON_ROWS 8 /* Danielsson block schedule: rows per block (1..4096);
-                                      65536 = the serial single-CTA engine */
+                                      65536 = the serial engine; at most 16 are used */
 #define DOL_TUNE_DANIELSSON_SLICES 9 /* Danielsson block schedule: slices per block (3D) */
 #define DOL_TUNE_EDT_HULL     10   /* EDT line passes, by line length: the percentage of a tile's cells with no
                                       other-state cell on their lower-dimension lines at which the tile takes the
@@ -340,9 +344,10 @@ DOL_API dol_status dol_sites_backward(int dim, int w, int h, int d, int n_sites,
                                       their cells 128 or more from the other state in their plane take the
                                       block-pruned search, 101 = for every tile not on the envelope path, 102 =
                                       never */
-#define DOL_TUNE_OCCLUSION    11   /* occlusion sweeps, by row length: 0 = block wavefront (3D blocks of 32 x 16
-                                      columns x 32 slices, 64 from 256 slices on), 1 = one CTA per plane (rows
-                                      up to 4096 cells), 2..999 = 3D blocks of that many slices, plus 1000 =
+#define DOL_TUNE_OCCLUSION    11   /* occlusion sweeps, by row length: 0 = block wavefront (3D in place: one launch,
+                                      blocks of 32 x 16 columns x 48 slices; in/out, or without scratch: a launch
+                                      per diagonal, 32 slices, 64 from 256 on), 1 = one CTA per plane (rows up to
+                                      4096 cells), 2..999 = 3D blocks of that many slices, plus 1000 =
                                       blocks of 32 x 32 columns */
 DOL_API dol_status dol_autotune(int kind, int w, int h, int d, void* stream);
 DOL_API int        dol_tune_get(int kind, int w);
@@ -351,14 +356,13 @@ DOL_API void       dol_tune_set(int kind, int w, int value);
 /* ---- failure-detection test hook (no reference counterpart; the reference
    has no error reporting, DistanceOcclusionLib.cpp:14-18 asserts only) ---------------
    For tests of the timeout path only; process-wide, affects later launches.
-   The 3D FastSweep wavefront (dol_fastsweep_3d, dol_sdf_3d with FastSweep)
-   waits, per row, for the rows it depends on; each wait gives up after
-   `limit` polls (about 128 ns apart; 0 = the default, 2^22), marks the call
-   failed and lets the row go on, so the launch always ends and the next
+   The 3D FastSweep columns and rows (dol_fastsweep_3d, dol_sdf_3d with
+   FastSweep) wait for those they depend on; each wait gives up after `limit`
+   polls (some hundred ns apart; 0 = the default, 2^22), marks the call failed
+   and lets the column or row go on, so the launch always ends and the next
    dol_sync() on the stream returns DOL_ERR_TIMEOUT (that call's deltas are
-   then invalid).  stall_sweep 0..7 makes that sweep's rows wait for a flag
-   value no row writes, so every such wait runs out; -1 restores normal
-   operation. */
+   then invalid).  stall_sweep 0..7 makes that sweep wait for a value nobody
+   writes, so every such wait runs out; -1 restores normal operation. */
 DOL_API void       dol_test_wait_hooks(int stall_sweep, unsigned limit);
 
 /* ---- synthetic inputs (no reference counterpart) --------------------------------------

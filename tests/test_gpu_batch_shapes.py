@@ -54,3 +54,40 @@ def test_engine_edges(dol, O, cuda, warps):
         np.testing.assert_array_equal(g, want, err_msg=f"{dm}")
         f = O.deltas_to_dist(want, dm, 2, masks[i])
         assert np.array_equal(got_f[items[i].dist_offset:][:n].view(np.uint32), f.reshape(-1).view(np.uint32)), dm
+
+
+def test_many_items(dol, O, cuda):
+    """More items per CTA than it takes one at a time: wide images by groups of
+    warps, then narrow ones warp by warp."""
+    torch = cuda
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    rng = np.random.default_rng(4)
+    wide = [(257, 5), (300, 33), (512, 9), (513, 20), (1024, 7), (700, 2)]
+    narrow = [(5, 4), (33, 6), (64, 3), (200, 5), (256, 9)]
+    kinds = [(d, O.bool_to_mask(rng.random((d[1], d[0])) < p)) for d in wide + narrow for p in (0.02, 0.4)]
+    which = [i % len(kinds) if i < 300 else len(kinds) - 10 + i % 10 for i in range(16 * sms + 300)]
+    items = (Item * len(which))()
+    masks, words, dbytes, cells = [], 0, 0, 0
+    for i, k in enumerate(which):
+        (w, h), m = kinds[k]
+        masks.append(m)
+        items[i] = Item(w, h, 1, 0, words, dbytes, cells)
+        words += len(m)
+        dbytes += (w * h * 4 + 15) // 16 * 16
+        cells += w * h
+    md = torch.from_numpy(np.concatenate(masks).view(np.int32)).cuda()
+    deltas = torch.zeros(dbytes, dtype=torch.uint8, device="cuda")
+    dist = torch.zeros(cells, dtype=torch.float32, device="cuda")
+    dol.check(dol.lib().dol_batch_sdf(len(which), items, C.c_void_p(md.data_ptr()), C.c_void_p(deltas.data_ptr()),
+                                      C.c_void_p(dist.data_ptr()), None, C.c_size_t(0), None))
+    dol.sync()
+    torch.cuda.synchronize()
+    got_d, got_f = deltas.cpu().numpy(), dist.cpu().numpy()
+    want = [(O.propagate("danielsson", O.border_init(m, d), d, 2), m, d) for d, m in kinds]
+    want = [(x.reshape(-1), O.deltas_to_dist(x, d, 2, m).reshape(-1)) for x, m, d in want]
+    for i, k in enumerate(which):
+        d, f = want[k]
+        n = items[i].w * items[i].h
+        g = got_d[items[i].delta_byte_offset:][:4 * n].view(np.int16)
+        assert np.array_equal(g, d.view(np.int16).reshape(-1)), (i, kinds[k][0])
+        assert np.array_equal(got_f[items[i].dist_offset:][:n].view(np.uint32), f.view(np.uint32)), (i, kinds[k][0])
