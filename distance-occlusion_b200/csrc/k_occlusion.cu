@@ -20,9 +20,10 @@
 // parallelism is the wavefront: cell (i, j, k) needs (i-1, j, k), (i, j-1, k)
 // and (i, j, k-1), so any order that visits those three first gives the
 // reference's values.  Two engines:
-//   * the block wavefront (default): each plane is cut into blocks, the
-//     blocks of one anti-diagonal run as one launch (k_occlusion_tiles2,
-//     k_occlusion_blocks3), cells inside a block in a skewed wavefront;
+//   * the block wavefront (default): each plane is cut into blocks, cells
+//     inside a block in a skewed wavefront; 3D in place one launch in which
+//     blocks wait for those before them (k_occlusion_wave3), else a launch per
+//     anti-diagonal of blocks (k_occlusion_tiles2, k_occlusion_blocks3);
 //   * one CTA per plane (k_occlusion_sweep, k_occlusion_sweep1): thread t
 //     owns C adjacent columns and walks the (slice, row) items in order,
 //     skewed one step behind thread t-1, whose last column it takes from
