@@ -292,7 +292,8 @@ __global__ void __launch_bounds__(256) k_jfa3_pack(const int16_t* __restrict__ i
 
 template <bool kLast>
 __global__ void __launch_bounds__(512) k_jfa3p(const uint32_t* __restrict__ in, void* __restrict__ out, int w, int h,
-                                               int d, int s, int cw, int nchunk, const int* __restrict__ odd)
+                                               int d, int s, int cw, int len, int nchunk,
+                                               const int* __restrict__ odd)
 {
     if (odd && *odd) return;
     const int x = blockIdx.x * 32 + (threadIdx.x & 31);
@@ -300,7 +301,7 @@ __global__ void __launch_bounds__(512) k_jfa3p(const uint32_t* __restrict__ in, 
     if (x >= w || y >= h) return;
     const int r = blockIdx.z / nchunk, chunk = blockIdx.z % nchunk;
     const int m = (d - r + s - 1) / s;   // cells r + i s < d
-    const int i0 = chunk * kJfaChunk, i1 = min(m, i0 + kJfaChunk);
+    const int i0 = chunk * len, i1 = min(m, i0 + len);
     if (i0 >= i1) return;
     const int plane = w * h;
     const int col = y * w + x;
@@ -483,15 +484,19 @@ static bool run_packed(void* deltas, void* temp, size_t half, int w, int h, int 
     const int warps = h * d;
     k_jfa3_pack<<<min((warps + 7) / 8, g_num_sms * 16), 256, 0, st>>>(static_cast<const int16_t*>(deltas), pb[0], w, h, d,
                                                                      cw, odd);
+    // cells a thread walks: a chunk of n loads n + 2 slices, but small volumes need
+    // the threads (whole calls with 8 | 16 | 32 cells: 64^3 78 | 96 | 116 us, 128^3 247 |
+    // 253 | 275, 400 x 300 x 100 2342 | 2309 | 2345, 256^3 1511 | 1442 | 1442)
+    const int len = (long long)w * h * d <= (1 << 20) ? 8 : 16;
     for (int i = 0; i < np; i++) {
         ProfScope ps("jumpflood_pass", st);
         const int sv = steps[i], nres = sv < d ? sv : d;
-        const int nchunk = ((d + sv - 1) / sv + kJfaChunk - 1) / kJfaChunk;
+        const int nchunk = ((d + sv - 1) / sv + len - 1) / len;
         const dim3 gz((w + 31) / 32, (h + ry - 1) / ry, (unsigned)(nres * nchunk));
         if (i == np - 1)
-            k_jfa3p<true><<<gz, 32 * ry, 0, st>>>(pb[i & 1], deltas, w, h, d, sv, cw, nchunk, odd);
+            k_jfa3p<true><<<gz, 32 * ry, 0, st>>>(pb[i & 1], deltas, w, h, d, sv, cw, len, nchunk, odd);
         else
-            k_jfa3p<false><<<gz, 32 * ry, 0, st>>>(pb[i & 1], pb[(i & 1) ^ 1], w, h, d, sv, cw, nchunk, odd);
+            k_jfa3p<false><<<gz, 32 * ry, 0, st>>>(pb[i & 1], pb[(i & 1) ^ 1], w, h, d, sv, cw, len, nchunk, odd);
     }
     if (!checked) {
         cudaLaunchConfig_t cfg = {};

@@ -8,7 +8,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("dims", [(1, 1, 2), (2, 1, 1), (5, 3, 2), (33, 9, 70), (64, 32, 16), (300, 5, 4), (4, 301, 5),
+@pytest.mark.parametrize("dims", [(1, 1, 2), (2, 1, 1), (5, 3, 2), (33, 9, 70), (6, 4, 8), (7, 5, 17), (128, 130, 67), (64, 32, 16), (300, 5, 4), (4, 301, 5),
                                   (6, 4, 598), (600, 3, 2), (37, 41, 43)])
 @pytest.mark.parametrize("p", [0.0, 0.002, 0.4])
 def test_packed_matches_oracle(dol, O, cuda, dims, p):
