@@ -43,6 +43,7 @@
 // rounds, each closed by one grid barrier (bounded waits).  With a warp for
 // every block a block that changed marks its dependents for the next round;
 // larger fields take blocks from a work list.
+#include "dan_rounds.h"
 #include "dan_serial.cuh"
 #include "grid_barrier.cuh"
 #include "kernels.h"
@@ -572,7 +573,7 @@ static bool run_phase(DanBlk& p, void* dl, cudaStream_t st)
     p.Z = Z;
     p.nk = (p.nchain + Z - 1) / Z;
     p.nblocks = p.nk * p.nc * p.nx;
-    p.max_rounds = 4 * p.nblocks + 8;
+    p.max_rounds = dan_max_rounds(p.nchain, p.h, p.nx);
     k_dan_blocks_init<<<min((p.nblocks + 255) / 256, g_num_sms * 8), 256, 0, st>>>(p);
     // a warp per CTA while that spreads the blocks over more SMs
     const int warps = p.nblocks <= 2 * g_num_sms ? 1 : kBlkWarps;
