@@ -522,7 +522,10 @@ static int dan_blocks_s(int dim, int w)
     return s;
 }
 
-// bytes of the pieces of the workspace
+// Bytes of the pieces of the workspace.  The control words need 32 of the last
+// piece's; the rest lets the first piece start at a 16-byte boundary whatever the
+// caller's workspace is aligned to (side cells move 8 bytes at a time).
+constexpr size_t kCtlBytes = 256, kWsAlign = 16;
 struct DanSizes {
     size_t field, down, side, flag, list, total;
 };
@@ -538,7 +541,7 @@ static DanSizes dan_sizes(int dim, int w, int h, int d, int R)
     z.side = nx > 1 ? al256(nd * h * 2 * nx * sizeof(uint2)) : 0;
     z.flag = al256(nc * nd * nx);
     z.list = al256(nc * nd * nx * sizeof(int));
-    z.total = 2 * z.field + 2 * z.down + 4 * z.side + 2 * z.flag + 4 * z.list + 256;
+    z.total = 2 * z.field + 2 * z.down + 4 * z.side + 2 * z.flag + 4 * z.list + kCtlBytes;
     return z;
 }
 
@@ -600,7 +603,8 @@ template <int kDim, int S>
 static bool run_all(int w, int h, int d, int cw, int R, void* deltas, void* ws, int* err, cudaStream_t st)
 {
     const DanSizes z = dan_sizes(kDim, w, h, d, R);
-    char* q = static_cast<char*>(ws);
+    static_assert(8 * sizeof(unsigned) + kWsAlign <= kCtlBytes, "the control words follow the shifted pieces");
+    char* q = reinterpret_cast<char*>(((uintptr_t)ws + kWsAlign - 1) & ~(uintptr_t)(kWsAlign - 1));
     auto take = [&](size_t bytes) {
         char* r = q;
         q += bytes;
