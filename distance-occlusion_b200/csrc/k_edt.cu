@@ -27,6 +27,7 @@
 #include <float.h>
 
 #include "common.cuh"
+#include "edt_layout.h"
 #include "hull.cuh"
 #include "kernels.h"
 #include "tma.cuh"
@@ -993,16 +994,6 @@ bool encode_map_3d(CUtensorMap* map, const void* base, CUtensorMapDataType type,
     return r == CUDA_SUCCESS;
 }
 
-// scratch of the mask EDT with rows `pitch` cells apart
-static size_t edt_bytes(int dim, int pitch, int h, int d)
-{
-    size_t cells = (size_t)pitch * h * (dim == 3 ? d : 1);
-    size_t b = cells * sizeof(uint16_t);
-    b = (b + 255) & ~(size_t)255;
-    if (dim == 3) b += cells * sizeof(uint32_t);
-    return b;
-}
-
 size_t edt_workspace_bytes(int dim, int w, int h, int d) { return edt_bytes(dim, padded_pitch(w), h, d); }
 size_t edt_workspace_bytes_min(int dim, int w, int h, int d) { return edt_bytes(dim, w, h, d); }
 
@@ -1032,7 +1023,7 @@ void launch_edt_mask(int dim, const uint32_t* mask, float* out, int w, int h, in
         ProfScope ps("edt_y_final", st);
         line_pass<uint16_t, true>(vx, out, w, pitch, h, 1, 0, form, err, st);
     } else {
-        const size_t off = edt_bytes(2, pitch, h * d, 1);
+        const size_t off = edt_x_bytes(pitch, (long long)h * d);
         uint32_t* ey = reinterpret_cast<uint32_t*>(static_cast<char*>(ws) + off);
         const bool blk = blocked_layout_ok(vx, ey, pitch, h, d);
         {
@@ -1057,7 +1048,7 @@ void launch_edt_mask_3d_chunked(const uint32_t* mask, float* out, int w, int h, 
     const int pitch = edt_pitch(3, w, h, d, ws_bytes);
     const int words = words_per_row(w);
     uint16_t* vx = static_cast<uint16_t*>(ws);
-    const size_t off = edt_bytes(2, pitch, h * d, 1);
+    const size_t off = edt_x_bytes(pitch, (long long)h * d);
     uint32_t* ey = reinterpret_cast<uint32_t*>(static_cast<char*>(ws) + off);
     const bool blk = blocked_layout_ok(vx, ey, pitch, h, d);
     slabs = slabs < 1 ? 1 : (slabs > d ? d : slabs);
