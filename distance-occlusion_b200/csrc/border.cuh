@@ -25,6 +25,17 @@
 
 namespace dolk {
 
+// number of live cells in global word `wid`, and the index of its first cell (64
+// bits: a batched volume may have more than 2^31 cells)
+DOL_HD void word_cells(long long wid, int w, int ws, long long* first, int* n)
+{
+    long long row = wid / ws;
+    int k = (int)(wid - row * ws);
+    *first = row * (long long)w + 32 * k;
+    int m = w - 32 * k;
+    *n = m < 32 ? m : 32;
+}
+
 // ---------------------------------------------------------------- 2D ----
 
 struct Planes2 {

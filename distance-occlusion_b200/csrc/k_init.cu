@@ -12,16 +12,6 @@
 
 namespace dolk {
 
-// number of live cells in global word `wid`, and the index of its first cell
-__device__ __forceinline__ void word_cells(long long wid, int w, int ws, long long* first, int* n)
-{
-    long long row = wid / ws;
-    int k = (int)(wid - row * ws);
-    *first = row * (long long)w + 32 * k;
-    int m = w - 32 * k;
-    *n = m < 32 ? m : 32;
-}
-
 // ---- byte mask -> bitmask ---------------------------------------------------
 // One warp per 32 words: for each word, lane b reads byte 32k+b of the row
 // (a coalesced 32-byte load) and a ballot forms the word.

@@ -543,26 +543,29 @@ __device__ __forceinline__ void border_warps(const uint32_t* mask, void* dl, int
 {
     const int lane = threadIdx.x & 31;
     const int ws = words_per_row(w);
-    const int words = ws * h * d;
-    for (int base = 32 * u; base < words; base += 32 * nu) {
-        const int wid = min(base + lane, words - 1);
-        const int row = wid / ws, k = wid - row * ws;
+    const long long words = (long long)ws * h * d;
+    for (long long base = 32 * u; base < words; base += 32 * nu) {
+        const long long wid = min(base + lane, words - 1);
+        const long long row = wid / ws;
+        const int k = (int)(wid - row * ws);
+        long long first;
+        int live;
+        word_cells(wid, w, ws, &first, &live);
         uint32_t pl[7];
         if (DIM == 2) {
-            const Planes2 p = border2_word(w, h, mask, row, k);
+            const Planes2 p = border2_word(w, h, mask, (int)row, k);
             pl[0] = p.mx; pl[1] = p.xn; pl[2] = p.xs; pl[3] = p.yn; pl[4] = p.ys; pl[5] = pl[6] = 0;
         } else {
-            const int z = row / h;
-            const Planes3 p = border3_word(w, h, d, mask, z, row - z * h, k);
+            const int z = (int)(row / h);
+            const Planes3 p = border3_word(w, h, d, mask, z, (int)(row - (long long)z * h), k);
             pl[0] = p.mx; pl[1] = p.xn; pl[2] = p.xs; pl[3] = p.yn; pl[4] = p.ys; pl[5] = p.zn; pl[6] = p.zs;
         }
-        const int first = row * w + 32 * k, live = min(32, w - 32 * k);
-        const int n = min(32, words - base);
+        const int n = (int)min(32LL, words - base);
         for (int q = 0; q < n; q++) {
             uint32_t b[7];
 #pragma unroll
             for (int i = 0; i < (DIM == 2 ? 5 : 7); i++) b[i] = __shfl_sync(0xFFFFFFFFu, pl[i], q);
-            const int at = __shfl_sync(0xFFFFFFFFu, first, q) + lane;
+            const long long at = __shfl_sync(0xFFFFFFFFu, first, q) + lane;
             const int nq = __shfl_sync(0xFFFFFFFFu, live, q);
             if (lane < nq) {
                 if (DIM == 2)
@@ -576,16 +579,16 @@ __device__ __forceinline__ void border_warps(const uint32_t* mask, void* dl, int
 }
 
 template <class Cell, class P>
-__device__ __forceinline__ void signed_dist_warps(const uint32_t* mask, const P* dl, float* out, int w, int rows, int u,
+__device__ __forceinline__ void signed_dist_warps(const uint32_t* mask, const P* dl, float* out, int w, long long rows, int u,
                                                   int nu)
 {
     const int lane = threadIdx.x & 31;
     const int ws = words_per_row(w);
-    for (int row = u; row < rows; row += nu) {
-        const long long first = (long long)row * w;
+    for (long long row = u; row < rows; row += nu) {
+        const long long first = row * w;
         for (int x = lane; x < w; x += 32) {
             float r = __fdiv_rn(sqrtf((float)len(cell_load(dl, first + x))), 2.0f);
-            if ((mask[(long long)row * ws + (x >> 5)] >> lane) & 1u) r = -r;
+            if ((mask[row * ws + (x >> 5)] >> lane) & 1u) r = -r;
             out[first + x] = r;
         }
     }
@@ -722,7 +725,7 @@ __device__ __noinline__ void batch_item_cta(const BatchItemDev& b, const uint32_
         }
         __syncthreads();
         if (dist && b.dist_off >= 0)
-            signed_dist_warps<C3>(m, static_cast<int16_t*>(dl), dist + b.dist_off, b.w, b.h * b.d, warp, 8);
+            signed_dist_warps<C3>(m, static_cast<int16_t*>(dl), dist + b.dist_off, b.w, (long long)b.h * b.d, warp, 8);
     }
 }
 
@@ -755,7 +758,7 @@ __global__ void __launch_bounds__(32 * NW) k_batch_sdf(const BatchItemDev* __res
         else if (warp == 0) batch_dan_warp<3>(dl, b.w, b.h, b.d, smem);
         __syncthreads();
         if (dist && b.dist_off >= 0)
-            signed_dist_warps<C3>(m, dl, dist + b.dist_off, b.w, b.h * b.d, warp, NW);
+            signed_dist_warps<C3>(m, dl, dist + b.dist_off, b.w, (long long)b.h * b.d, warp, NW);
         __syncthreads();
     }
     unsigned char* strip = smem + warp * kBatchStrip;
@@ -813,7 +816,7 @@ __global__ void __launch_bounds__(32 * NW) k_batch_sdf(const BatchItemDev* __res
         }
         const uint32_t* m = masks + b.mask_off;
         void* dl = deltas + b.delta_off;
-        const int rows = b.h * b.d;
+        const long long rows = (long long)b.h * b.d;
         if (b.d <= 1) {
             border_warps<2>(m, dl, b.w, b.h, 1, gw, 4);
             sync();

@@ -20,6 +20,18 @@ def host(tmp_path_factory):
     return L
 
 
+@pytest.mark.parametrize("w,h,d", [(1024, 2048, 1025), (37, 70000, 3000), (1, 50000, 50000), (8, 4, 3)])
+def test_cells_of_a_mask_word(host, w, h, d):
+    ws = (w + 31) // 32
+    words = ws * h * d
+    for wid in (0, 1, ws, words // 2, words - ws, words - 1):
+        first, n = C.c_longlong(), C.c_int()
+        host.host_word_cells(C.c_longlong(wid), w, C.byref(first), C.byref(n))
+        row, k = divmod(wid, ws)
+        assert (first.value, n.value) == (row * w + 32 * k, min(32, w - 32 * k))
+    assert first.value + n.value == w * h * d
+
+
 @pytest.mark.parametrize("w,h,d", [(1, 46341, 46341), (3, 60000, 60000), (1024, 1024, 1024), (7, 5, 3)])
 def test_fields_of_the_mask_edt(host, w, h, d):
     up = lambda b: (b + 255) // 256 * 256
