@@ -743,17 +743,23 @@ static size_t fastsweep3_spare(int w, int h, int d)
     return align256(fastsweep3_workspace_bytes(w, h, d)) - align256(fastsweep3_workspace_bytes_min(w, h, d));
 }
 
+// dim: of the entry; a one-slice volume holds 3D cells
+static size_t sdf_bytes(int dim, int w, int h, int d, int method)
+{
+    const size_t cells = (size_t)w * h * d;
+    const size_t cb = dim == 3 ? sizeof(dol_delta3) : sizeof(dol_delta2);
+    if (method == DOL_FELZENSZWALB) return edt_workspace_bytes(d > 1 ? dim : 2, w, h, d);
+    size_t b = align256(cells * cb);                       // deltas, when the caller passes none
+    if (method == DOL_JUMPFLOOD) b += align256(jumpflood_workspace_bytes(dim, w, h, d));
+    if (method == DOL_FASTSWEEP && dim == 3) b += align256(fastsweep3_workspace_bytes(w, h, d));
+    if (method == DOL_DANIELSSON) b += align256(danielsson_workspace_bytes(dim, w, h, d));
+    return b;
+}
+
 size_t dol_sdf_workspace_size(int w, int h, int d, int method)
 {
-    const int dim = d > 1 ? 3 : 2;
-    const size_t cells = (size_t)w * h * (dim == 3 ? d : 1);
-    const size_t cb = dim == 3 ? sizeof(dol_delta3) : sizeof(dol_delta2);
-    if (method == DOL_FELZENSZWALB) return edt_workspace_bytes(dim, w, h, d);
-    size_t b = align256(cells * cb);                       // deltas, when the caller passes none
-    if (method == DOL_JUMPFLOOD) b += align256(jumpflood_workspace_bytes(dim, w, h, dim == 3 ? d : 1));
-    if (method == DOL_FASTSWEEP && dim == 3) b += align256(fastsweep3_workspace_bytes(w, h, d));
-    if (method == DOL_DANIELSSON) b += align256(danielsson_workspace_bytes(dim, w, h, dim == 3 ? d : 1));
-    return b;
+    // one slice: enough for the 2D entry and for the 3D entry
+    return d > 1 ? sdf_bytes(3, w, h, d, method) : std::max(sdf_bytes(2, w, h, 1, method), sdf_bytes(3, w, h, 1, method));
 }
 
 static dol_status sdf_common(int dim, int w, int h, int d, const uint32_t* mask, int method, void* deltas, float* dist,
@@ -786,8 +792,8 @@ static dol_status sdf_common(int dim, int w, int h, int d, const uint32_t* mask,
         return launched("sdf (felzenszwalb)");
     }
     // FastSweep 3D runs on less than it asks for
-    const size_t need = dol_sdf_workspace_size(w, h, dim == 3 ? d : 1, method);
-    const size_t spare = method == DOL_FASTSWEEP && dim == 3 && d > 1 ? fastsweep3_spare(w, h, d) : 0;
+    const size_t need = sdf_bytes(dim, w, h, dim == 3 ? d : 1, method);
+    const size_t spare = method == DOL_FASTSWEEP && dim == 3 ? fastsweep3_spare(w, h, d) : 0;
     size_t got;
     DOL_TRY(get_workspace_between(ws, workspace, workspace_bytes, need, need - spare, &got, st));
     const size_t fs3_bytes = spare && got < need ? fastsweep3_workspace_bytes_min(w, h, d)
@@ -827,16 +833,21 @@ dol_status dol_sdf_3d(int w, int h, int d, const uint32_t* mask, int method, dol
 
 // ---- two-pass signed fields (the tool's -S path) --------------------------------------------------
 
-size_t dol_sdf_two_pass_workspace_size(int w, int h, int d, int method)
+static size_t two_pass_bytes(int dim, int w, int h, int d, int method)
 {
-    const int dim = d > 1 ? 3 : 2;
-    const size_t cells = (size_t)w * h * (dim == 3 ? d : 1);
+    const size_t cells = (size_t)w * h * d;
     const size_t cb = dim == 3 ? sizeof(dol_delta3) : sizeof(dol_delta2);
     size_t b = 2 * align256(cells * cb);                    // exterior / interior deltas the caller does not keep
-    if (method == DOL_JUMPFLOOD) b += align256(jumpflood_workspace_bytes(dim, w, h, dim == 3 ? d : 1));
+    if (method == DOL_JUMPFLOOD) b += align256(jumpflood_workspace_bytes(dim, w, h, d));
     if (method == DOL_FASTSWEEP && dim == 3) b += align256(fastsweep3_workspace_bytes(w, h, d));
-    if (method == DOL_DANIELSSON) b += align256(danielsson_workspace_bytes(dim, w, h, dim == 3 ? d : 1));
+    if (method == DOL_DANIELSSON) b += align256(danielsson_workspace_bytes(dim, w, h, d));
     return b;
+}
+
+size_t dol_sdf_two_pass_workspace_size(int w, int h, int d, int method)
+{
+    return d > 1 ? two_pass_bytes(3, w, h, d, method)
+                 : std::max(two_pass_bytes(2, w, h, 1, method), two_pass_bytes(3, w, h, 1, method));
 }
 
 static dol_status sdf_two_pass_common(int dim, int w, int h, int d, const uint32_t* mask, int method, void* ext,
@@ -861,8 +872,8 @@ static dol_status sdf_two_pass_common(int dim, int w, int h, int d, const uint32
     cudaStream_t st = S(stream);
     const int dd = dim == 3 ? d : 1;
     Workspace ws;
-    const size_t need = dol_sdf_two_pass_workspace_size(w, h, dd, method);
-    const size_t spare = method == DOL_FASTSWEEP && dd > 1 ? fastsweep3_spare(w, h, d) : 0;
+    const size_t need = two_pass_bytes(dim, w, h, dd, method);
+    const size_t spare = method == DOL_FASTSWEEP && dim == 3 ? fastsweep3_spare(w, h, d) : 0;
     size_t got;
     DOL_TRY(get_workspace_between(ws, workspace, workspace_bytes, need, need - spare, &got, st));
     const size_t fs3_bytes = spare && got < need ? fastsweep3_workspace_bytes_min(w, h, d)

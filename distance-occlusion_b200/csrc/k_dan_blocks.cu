@@ -648,6 +648,7 @@ static bool run_all(int w, int h, int d, int cw, int R, void* deltas, void* ws, 
 
 size_t danielsson_workspace_bytes(int dim, int w, int h, int d)
 {
+    if (dim == 3 && d < 2) return 0;   // nothing to sweep
     const int R = dan_blocks_rows(dim, w, h, d);
     if (R >= kDanSerial || w > kBlkMaxWidth) return 0;
     return dan_blocks_workspace_bytes(dim, w, h, d, R);
