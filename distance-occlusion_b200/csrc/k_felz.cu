@@ -12,14 +12,21 @@
 // can be built in parallel.  So, one warp per line:
 //   1. each lane builds the hull of a word of 32 positions (a bit per vertex),
 //      and the words' hulls merge pairwise (felz_merge);
-//   2. every position is checked against its neighbours on that hull: a vertex
-//      whose right boundary is above its left one, or another point with them
-//      the other way round, by more than kFelzClear of their size is clear.  If
-//      the rest are off by at most kFelzOff, and the vertices that turn the
-//      wrong way by that are few (kFelzTurns), then every point is above the
-//      hull's edges and every boundary above or below the hull's next one to
-//      within (kFelzTurns + 1) kFelzOff < kFelzClear / 2 of its size, and the
-//      reference's rounding (2^-23 of a boundary's size) is far smaller still.
+//   2. every position is checked against its neighbours on that hull, by the
+//      boundaries with them.  e = 2^-24; a boundary computed from heights (a
+//      difference and a division, each correctly rounded) is off by at most 2 e
+//      of its size, the difference of two, the gap, by 6 e of the larger one's.
+//      A vertex whose right boundary is above its left one, or another point
+//      with them the other way round, by more than kFelzClear = 128 e of their
+//      size is clear (in truth: by 122 e).  If no point is off by more than
+//      kFelzOff = 2 e (8 e), and the vertices whose gap is not surely above zero
+//      (kFelzSure) are at most kFelzTurns = 4, then along the hull boundaries
+//      fall back by at most 4 x 8 e, and a point lies above an edge's line to
+//      within 8 e more: from a clear vertex every later point is seen at or above
+//      its right boundary, every earlier one at or below its left one, each
+//      to within 40 e, so that the two stay 122 - 80 = 42 e apart, and the
+//      reference, whose two boundaries are off by 2 e each, decides as on
+//      exact numbers.
 //      So a clear vertex is never popped, and a clear other point between two
 //      clear vertices is popped at the latest by the second.
 //   3. what is not clear -- ties of integer fields, now and then a near tie -- is
@@ -28,7 +35,9 @@
 //      first, and nothing later reaches back over the second;
 //   4. boundaries by neighbouring vertices, a binary search per cell.
 // A line that step 2 finds worse than that (not finite, say) is built serially as
-// a whole; step 1 so needs no bound on its rounding.
+// a whole; step 1 so needs no bound on its rounding.  (Input that is not finite
+// has no defined result: the reference leaves its stack there.  Here the bottom
+// of the stack stays, whatever compares.)
 //
 // What bounds it: latency of the dependent steps of a warp (an SM holds one to
 // three warps per scheduler).  1024 x 1024 heights, both passes: 3.47 ms with one
@@ -45,8 +54,9 @@ namespace dolk {
 constexpr int kFelzMaxLines = 8;
 constexpr size_t kFelzSmemLimit = 224 * 1024;
 constexpr float kFelzClear = 0x1p-17f;
-constexpr float kFelzOff = 0x1p-21f;
-constexpr int kFelzTurns = 6;
+constexpr float kFelzOff = 0x1p-23f;
+constexpr float kFelzSure = 0x1p-21f;
+constexpr int kFelzTurns = 4;
 
 // Shared memory of a line of n cells: values, heights (value + position^2; a word
 // of padding per 32, so that lanes a word apart fall in different banks),
@@ -265,14 +275,14 @@ __global__ void __launch_bounds__(32 * kFelzMaxLines) k_felz_lines(const float* 
             }
             const float hq = l.height(q);
             if (q > 0 && q < n - 1) {   // the ends are vertices of any build
-                const float s1 = __fdividef(hq - hp, (float)(2 * (q - p)));
-                const float s2 = __fdividef(hx - hq, (float)(2 * (x - q)));
+                const float s1 = __fdiv_rn(hq - hp, (float)(2 * (q - p)));
+                const float s2 = __fdiv_rn(hx - hq, (float)(2 * (x - q)));
                 const float gap = vertex ? s2 - s1 : s1 - s2;
                 const float size = fmaxf(fabsf(s1), fabsf(s2));
                 if (!(gap > __fmaf_rn(kFelzClear, size, FLT_MIN))) {
                     doubt |= 1u << b;
                     if (!(gap >= -kFelzOff * size)) bad += kFelzTurns + 1;
-                    if (vertex && gap < 0.0f) bad++;
+                    if (vertex && !(gap > kFelzSure * size)) bad++;
                 }
             }
             if (vertex) {
