@@ -486,17 +486,27 @@ int dan_blocks_rows(int dim, int w, int h, int d)
 {
     const int tv = tune_get(kTuneDanRows, w);
     if (tv > 0) return tv >= kDanSerial ? kDanSerial : min(tv, kBlkMaxRows);
-    // tiny fields: the serial engine's launch is cheaper than the rounds.  Small
-    // images: a row takes the serial engine 0.8 - 1.5 us, the blocks need up to 20
-    // rounds where single shapes fill the image (value noise, lattice 51 | 20, and
-    // 40 points: 64 x 64 76 | 121, 119 us serial, 157 | 156, 105 us in blocks; 64 x
-    // 128 158 | 236, 205 and 285 | 135, 121; 20 x 400 0.40 and 0.94 ms with lattice
-    // 51; 128 x 64 160 | 147, 119 and 156 | 145,
-    // 109; 256 x 32 82 | 100, 88 and 179 | 146, 131; 96 x 96 280 | 346, 252 and
-    // 285 | 219, 146)
+    // Fields of a short chain go to the serial engine: the blocks take some 20
+    // rounds and three launches however short it is.  Images (noise of lattice 51
+    // | 20, and 40 points, us serial against blocks): 64 x 64 76 | 121, 119 against
+    // 157 | 156, 105; 64 x 128 158 | 236, 205 against 285 | 135, 121; 128 x 64 160 |
+    // 147, 119 against 156 | 145, 109; 256 x 32 82 | 100, 88 against 179 | 146, 131;
+    // 96 x 96 280 | 346, 252 against 285 | 219, 146; lattice 20 and 30 points: 400 x 16
+    // 101, 92 against 114, 101; 700 x 16 123, 93 against 138, 124; 700 x 24 184, 134
+    // against 177, 148).  Volumes: a row step takes the serial engine about 0.5 us
+    // and 2 ns a cell; blocks from 4 (h - 1) (d - 1) steps that sum to 140 us,
+    // 220 where slices outnumber rows, each a step of the rounds' chain (the same
+    // contents: 64 x 4 x 16 137, 137 against 229, 208; 64 x 8 x 16 311, 285
+    // against 295, 265; 16 x 16 x 4 132, 118 against 168, 122; 16 x 16 x 8 295, 257
+    // against 212, 182; 256 x 8 x 4 119, 116 against 172, 156; 256 x 16 x 4 244, 224
+    // against 228, 197; 1000 x 4 x 6 257, 231 against 254, 233; 32 x 3
+    // x 40 234, 206 against 336, 234); one row per slice has
+    // no passes at all (64 x 1 x 40 0.04 against 0.27 ms).
     const long long cells = (long long)w * h * (dim == 3 ? d : 1);
     if (cells < 1024 || w > kBlkMaxWidth) return kDanSerial;
-    if (dim == 2 && ((w <= 256 && h <= 32) || (w <= 128 && h <= 64) || (w <= 64 && h <= 200) || (w <= 32 && h <= 512)))
+    if (dim == 3 && (h == 1 || 4LL * (h - 1) * (d - 1) * (250 + w) < (d > h ? 110000 : 70000))) return kDanSerial;
+    if (dim == 2 && ((w <= 256 && h <= 32) || (w <= 128 && h <= 64) || (w <= 64 && h <= 200) || (w <= 32 && h <= 512) ||
+                     h < 24))
         return kDanSerial;
     // 8 rows; tall images of several x blocks 16 (1024^2, 100 points: 0.51
     // against 0.62 ms; 501 x 700 noise: 0.53 against 0.43); volumes whose

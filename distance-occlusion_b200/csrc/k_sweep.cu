@@ -18,29 +18,15 @@
 // the earliest unfinished row can always proceed.
 #include <limits.h>
 
+#include "dan_scan.cuh"
 #include "dan_serial.cuh"
 #include "dan_slices.cuh"
 #include "kernels.h"
-#include "scan.cuh"
 
 namespace dolk {
 
 // ---------------------------------------------------------------- helpers ----
 
-template <class Cell, int S, class P>
-__device__ __forceinline__ void load_row(Cell (&dst)[S], const P* base, long long row_first, int n)
-{
-#pragma unroll
-    for (int s = 0; s < S; s++)
-        if (s < n) dst[s] = cell_load(base, row_first + s);
-}
-template <class Cell, int S, class P>
-__device__ __forceinline__ void store_row(P* base, long long row_first, const Cell (&src)[S], int n)
-{
-#pragma unroll
-    for (int s = 0; s < S; s++)
-        if (s < n) cell_store(base, row_first + s, src[s]);
-}
 // L2-coherent loads for rows written by other CTAs of the same launch
 __device__ __forceinline__ C3 cell_load_cg(const int16_t* p, long long i)
 {
@@ -387,6 +373,8 @@ void launch_danielsson(int dim, void* deltas, int w, int h, int d, int cw, cudaS
     int s, nw;
     row_shape(dim == 2 ? kTuneDan2 : kTuneDan3, w, &s, &nw);
     ProfScope ps("danielsson", st);
+    const int tv = tune_get(dim == 2 ? kTuneDan2 : kTuneDan3, w);
+    if (tv != 4 && tv != 8 && launch_danielsson_scan(dim, deltas, w, h, dim == 2 ? 1 : d, cw, st)) return;
     auto run = [&](auto kern, int warps, size_t strips) {
         if (strips > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)strips);
         kern<<<1, 32 * warps, strips, st>>>(deltas, w, h, dim == 2 ? 1 : d, cw);
@@ -408,11 +396,12 @@ void launch_fastsweep_2d(void* deltas, int w, int h, int cw, cudaStream_t st)
     int s, nw;
     row_shape(kTuneFs2, w, &s, &nw);
     ProfScope ps("fastsweep_2d", st);
+    const int tv = tune_get(kTuneFs2, w);
+    if (tv != 4 && tv != 8 && launch_fastsweep_2d_scan(deltas, w, h, cw, st)) return;
 #define DOL_FS_CASE(SV, NWV) \
     if (s == SV && nw == NWV)  \
         k_fastsweep2<SV, NWV><<<1, 32 * NWV, NWV * SerialIO<2, SV>::kBytes, st>>>(deltas, w, h, cw);
     DOL_ROW_SHAPES(DOL_FS_CASE)
-    DOL_FS_CASE(1, 1)
 #undef DOL_FS_CASE
 }
 
@@ -651,54 +640,10 @@ constexpr size_t kBatchSmem = 216 * 1024;
 constexpr int kBatchFew = 16;
 constexpr int kBatchStrip = (int)SerialIO<3, 8>::kBytes;   // a warp's strips in queue B, the widest
 
-// Danielsson of an image with rows of at most S cells per thread by the whole CTA
-// (scan.cuh): a few cells per thread, the next row loaded during this one, each
-// pass posting what the next one needs.
-template <int S>
-__device__ __noinline__ void batch_dan_cta(uint32_t* __restrict__ dl, int w, int h, int cw, ScanShared<C2>& sh)
+// an image with rows of at most 1024 cells by 8 warps, 4 cells per thread
+__device__ __noinline__ void batch_dan_image(uint32_t* dl, int w, int h, ScanShared<C2>& sh)
 {
-    const int t = threadIdx.x;
-    const int nseg = (w + S - 1) / S;
-    const bool active = t < nseg;
-    const int n = active ? min(S, w - t * S) : 0;
-    const long long x0 = (long long)t * S;
-    if (h < 2) return;
-    const int steps = 2 * (h - 1);
-    auto row_of = [&](int i) { return i < h - 1 ? i + 1 : 2 * h - 3 - i; };
-    auto dy_of = [&](int i) { return i < h - 1 ? -cw : cw; };
-    C2 P[S], C[S], V[S], R[S], D[S];
-#pragma unroll
-    for (int s = 0; s < S; s++) P[s] = C[s] = V[s] = R[s] = D[s] = C2{0, 0};
-
-    load_row<C2, S>(P, dl, x0, n);
-    load_row<C2, S>(C, dl, (long long)row_of(0) * w + x0, n);
-#pragma unroll
-    for (int s = 0; s < S; s++) V[s] = closer(C[s], add(P[s], 0, dy_of(0)));
-    int g = 0;
-    if (active) sh.guess[g][t] = seg_edge<C2, S, +1>(V, n);
-    __syncthreads();
-    for (int i = 0; i < steps; i++) {
-        const int y = row_of(i);
-        const bool more = i + 1 < steps;
-        const int dyn = more ? dy_of(i + 1) : 0;
-        if (more) load_row<C2, S>(C, dl, (long long)row_of(i + 1) * w + x0, n);
-        const C2 in0 = (active && t > 0) ? sh.guess[g][t - 1] : V[0];
-        row_pass<C2, S, false, +1>(R, V, t, nseg, n, cw, sh, D, in0, [&](const C2 (&X)[S]) {
-            if (active) sh.guess[g ^ 1][t] = X[0];
-        });
-        g ^= 1;
-        const C2 in1 = (active && t + 1 < nseg) ? sh.guess[g][t + 1] : R[0];
-        row_pass<C2, S, false, -1>(P, R, t, nseg, n, cw, sh, D, in1, [&](const C2 (&X)[S]) {
-            if (more && active)
-                sh.guess[g ^ 1][t] = closer(seg_edge<C2, S, +1>(C, n), add(seg_edge<C2, S, +1>(X, n), 0, dyn));
-        });
-        g ^= 1;
-        store_row<C2, S>(dl, (long long)y * w + x0, P, n);
-        if (more) {
-#pragma unroll
-            for (int s = 0; s < S; s++) V[s] = closer(C[s], add(P[s], 0, dyn));
-        }
-    }
+    danielsson2_cta<4>(dl, w, h, 2, sh);
 }
 
 // an item of queue B with rows of more than 256 cells, by the CTA's 8 warps
@@ -711,7 +656,7 @@ __device__ __noinline__ void batch_item_cta(const BatchItemDev& b, const uint32_
     if (b.d <= 1) {
         border_warps<2>(m, dl, b.w, b.h, 1, warp, 8);
         __syncthreads();
-        batch_dan_cta<4>(static_cast<uint32_t*>(dl), b.w, b.h, 2, *reinterpret_cast<ScanShared<C2>*>(smem));
+        batch_dan_image(static_cast<uint32_t*>(dl), b.w, b.h, *reinterpret_cast<ScanShared<C2>*>(smem));
         __syncthreads();
         if (dist && b.dist_off >= 0)
             signed_dist_warps<C2>(m, static_cast<uint32_t*>(dl), dist + b.dist_off, b.w, b.h, warp, 8);

@@ -119,6 +119,9 @@ size_t danielsson_workspace_bytes(int dim, int w, int h, int d);
 bool run_danielsson(int dim, void* deltas, int w, int h, int d, int cw, void* ws, size_t ws_bytes, int* err,
                     cudaStream_t st);
 void launch_fastsweep_2d(void* deltas, int w, int h, int cw, cudaStream_t st);
+// k_scan.cu -- rows in registers; false: the walk by warps is faster
+bool launch_danielsson_scan(int dim, void* deltas, int w, int h, int d, int cw, cudaStream_t st);
+bool launch_fastsweep_2d_scan(void* deltas, int w, int h, int cw, cudaStream_t st);
 // the _min form holds the engines of rows too wide for a warp
 size_t fastsweep3_workspace_bytes(int w, int h, int d);
 size_t fastsweep3_workspace_bytes_min(int w, int h, int d);

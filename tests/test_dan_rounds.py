@@ -63,10 +63,24 @@ def test_limit_of_large_fields(model):
         assert 1 << 27 < f(*args) < 1 << 28
 
 
+@pytest.fixture
+def tune_rows(dol):
+    set_ = []
+
+    def put(w, rows):
+        set_.append(w)
+        dol.lib().dol_tune_set(8, w, rows)   # DOL_TUNE_DANIELSSON_ROWS
+    yield put
+    for w in set_:
+        dol.lib().dol_tune_set(8, w, 0)
+
+
 @pytest.mark.gpu
+@pytest.mark.parametrize("rows", [0, 4])   # the engine that the shape gets; blocks of 4 rows
 @pytest.mark.parametrize("dims", SHAPES)
-def test_callers_deltas(dol, O, cuda, dims):
+def test_callers_deltas(dol, O, cuda, tune_rows, dims, rows):
     d = dims[2]
+    tune_rows(dims[0], rows)
     odims = dims if d > 1 else dims[:2]
     for i, f in enumerate(fields(dims, 100 + sum(dims), 48)):
         cw = 1 + i % 2
