@@ -574,13 +574,15 @@ static bool run_phase(DanBlk& p, void* dl, cudaStream_t st)
         return false;
     const int resident = per_sm * g_num_sms * kBlkWarps;   // warps
     // slices per block: 2 while that gives at most two blocks per resident warp
-    // (101 x 77 x 90: 1.6 ms, 1.8 with 4), else 4, more where there would be
-    // over 8 blocks per resident warp, at most 16
+    // (101 x 77 x 90: 1.6 ms, 1.8 with 4), 1 for up to 16 slices then (noise | 30
+    // points: 64 x 400 x 8 0.45 | 0.94 ms, 0.52 | 1.44 with 2; 200 x 400 x 4 0.43 | 0.95,
+    // 0.54 | 1.32; but 8 x 400 x 100 1.45 | 3.26, 1.29 | 3.60), else 4, more where there
+    // would be over 8 blocks per resident warp, at most 16
     int Z = tune_get(kTuneDanSlices, p.w);
     if (Z < 1) {
         Z = (int)((long long)p.nchain * p.nc * p.nx / (8LL * resident));
         const bool few = (long long)p.nchain * p.nc * p.nx <= 4LL * resident;
-        Z = max(few ? 2 : 4, min(Z, 16));
+        Z = max(few ? (p.nchain <= 16 ? 1 : 2) : 4, min(Z, 16));
     }
     if (Z > p.nchain) Z = p.nchain;
     p.Z = Z;
