@@ -948,7 +948,7 @@ dol_status dol_batch_prepare(int n, const dol_batch_item* items, void* workspace
         work[i] = it.d > 1 ? 4.0 * it.d * it.h + 1e-3 * it.w * it.h * it.d : 2.0 * it.h + 1e-3 * it.w * it.h;
         order[i] = i;
     }
-    // queue A: volumes with rows of at most 256 cells (one warp each); queue B:
+    // queue A: volumes with rows of at most 256 cells (a CTA each); queue B:
     // items with wider rows (one CTA each), then the narrow images; each group
     // by decreasing work
     auto group = [&](int i) { return items[i].w > 256 ? 1 : (items[i].d > 1 ? 0 : 2); };
