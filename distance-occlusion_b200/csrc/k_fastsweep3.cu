@@ -582,9 +582,22 @@ static Fs3Layout fs3_layout(int w, int h, int d)
     return l;
 }
 
+// Volumes of few rows and slices go to the slices (k_sweep.cu, a CTA per slice that
+// walks its rows): those take a row's time for each row and slice of each sweep,
+// some 1.3 us and 4.5 ns a cell, whatever the width, while x turns round with
+// every sweep, so that the eight sweeps cross the columns of a row one after
+// another, some 6 us each.  Columns against slices, us: 256 x 4 x 4 749, 142; 256 x 8 x
+// 32 812, 707; 256 x 32 x 32 846, 1148; 2000 x 2 x 2 5709, 133; 2000 x 32 x 32 5995, 4816;
+// 2000 x 128 x 8 5839, 10462; 64 x 8 x 8 216, 194; 64 x 8 x 32 251, 561.
+bool fastsweep3_by_slices(int w, int h, int d)
+{
+    return (h + d - 2.0) * (10.4 + 0.036 * w) < 50.0 * ((w + kTX - 1) / kTX);
+}
+
 size_t fastsweep3_columns_bytes(int w, int h, int d)
 {
-    if (h < 2 || d < 2 || tune_get(kTuneFs3, w) < 0) return 0;
+    const int tuned = tune_get(kTuneFs3, w);   // positive: columns, negative: the anti-diagonal wavefront
+    if (h < 2 || d < 2 || tuned < 0 || (tuned == 0 && fastsweep3_by_slices(w, h, d))) return 0;
     const Fs3Layout l = fs3_layout(w, h, d);
     if (8 * l.cols > (1 << 28) || l.nch > 65535) return 0;
     return l.bytes;

@@ -130,7 +130,9 @@ void launch_batch_sdf(const void* items, const int* order, int n, const uint32_t
                       int* counter, cudaStream_t st);
 void launch_fastsweep_3d(void* deltas, int w, int h, int d, int cw, void* ws, size_t ws_bytes, int* err,
                          cudaStream_t st);
-// k_fastsweep3.cu -- columns streaming along z; false when the workspace is too small
+// k_fastsweep3.cu -- columns streaming along z; false when the workspace is too small,
+// or the slices are faster (fastsweep3_by_slices)
+bool fastsweep3_by_slices(int w, int h, int d);
 size_t fastsweep3_columns_bytes(int w, int h, int d);
 bool launch_fastsweep_3d_columns(void* deltas, int w, int h, int d, int cw, void* ws, size_t ws_bytes, int* err,
                                  cudaStream_t st);

@@ -143,7 +143,9 @@ DOL_API int        dol_last_engine(void);
 DOL_API dol_status dol_fastsweep_2d(int w, int h, dol_delta2* deltas, int cw, void* stream);
 /* 3D: about 1.2x the field (a copy in tiles and the words that columns hand on);
    with less -- a caller's workspace, or the dol_set_workspace_limit cap -- down to
-   4 (h d + h + d) bytes and some, the slices run instead: same deltas, slower */
+   4 (h d + h + d) bytes and some, the slices run instead: same deltas, slower
+   (and on volumes of few rows and slices for their width, where they are faster
+   and the size is theirs) */
 DOL_API size_t     dol_fastsweep_3d_workspace_size(int w, int h, int d);
 DOL_API dol_status dol_fastsweep_3d(int w, int h, int d, dol_delta3* deltas, int cw,
                             void* workspace, size_t workspace_bytes, void* stream);
