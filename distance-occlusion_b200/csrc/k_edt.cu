@@ -805,6 +805,11 @@ __global__ void __launch_bounds__(512) k_edt_line_tma(const __grid_constant__ CU
 
 constexpr size_t kStageLimit = 200 * 1024;   // largest staged line tile of the plain form
 constexpr size_t kTileLimit = 200 * 1024;    // largest tile of the TMA form
+// Lines of up to this many cells take the plain form: a TMA tile of so few positions
+// costs its CTA more than the search (whole calls on value noise, TMA against
+// plain: 900 x 3 x 250 83 against 28 us, 900 x 16 x 250 104 against 84, 900 x 24 x 250 123
+// against 135, 100 x 16 x 250 32 against 26, 900 x 16 images 13 either way)
+constexpr int kShortLine = 16;
 
 // set_attr = false: the caller raised the staged kernel's shared-memory limit
 // to kStageLimit beforehand (prepare_edt_mask_2d_plain)
@@ -852,7 +857,7 @@ static bool line_map(CUtensorMap* map, const TIn* in, int w, int h, int d, int a
 // [y][pitch/8][z][8] array: 8 | pitch, both line tiles fit, both maps encode.
 static bool blocked_layout_ok(const uint16_t* vx, const uint32_t* ey, int pitch, int h, int d)
 {
-    if (pitch % 8 != 0 || d > 65535) return false;
+    if (pitch % 8 != 0 || d > 65535 || h <= kShortLine || d <= kShortLine) return false;
     if (tma_tile_bytes<uint16_t, 16>(h) > kTileLimit || tma_tile_bytes<uint32_t, 8>(d) > kTileLimit) return false;
     if ((long long)(pitch / 8) * h > 0x7FFFFFFFLL) return false;
     if (((uintptr_t)vx % 16) != 0 || ((uintptr_t)ey % 16) != 0) return false;
@@ -940,7 +945,7 @@ static void line_pass(const TIn* in, void* out, int w, int pitch, int h, int d, 
                                            outer0, st);
         return;
     }
-    if (aligned && outer <= 65535) {
+    if (aligned && outer <= 65535 && n > kShortLine) {
         // grid.z CTAs search one tile while the tiles alone would leave SMs
         // idle (an image: w / 16 tiles), each at least 64 positions
         auto parts = [&](int tx) {
@@ -994,13 +999,22 @@ bool encode_map_3d(CUtensorMap* map, const void* base, CUtensorMapDataType type,
     return r == CUDA_SUCCESS;
 }
 
-size_t edt_workspace_bytes(int dim, int w, int h, int d) { return edt_bytes(dim, padded_pitch(w), h, d); }
+// padded rows where a pass of the TMA form reads them; else they only spread the
+// plain form's loads (1 x 16000: 5.4 ms packed, 5.8 padded)
+static int wanted_pitch(int dim, int w, int h, int d)
+{
+    const bool y = h > kShortLine && tma_tile_bytes<uint16_t, 8>(h) <= kTileLimit;
+    const bool z = dim == 3 && d > kShortLine && tma_tile_bytes<uint32_t, 8>(d) <= kTileLimit;
+    return y || z ? padded_pitch(w) : w;
+}
+
+size_t edt_workspace_bytes(int dim, int w, int h, int d) { return edt_bytes(dim, wanted_pitch(dim, w, h, d), h, d); }
 size_t edt_workspace_bytes_min(int dim, int w, int h, int d) { return edt_bytes(dim, w, h, d); }
 
 // padded rows whenever the scratch holds them
 static int edt_pitch(int dim, int w, int h, int d, size_t ws_bytes)
 {
-    return ws_bytes >= edt_workspace_bytes(dim, w, h, d) ? padded_pitch(w) : w;
+    return ws_bytes >= edt_workspace_bytes(dim, w, h, d) ? wanted_pitch(dim, w, h, d) : w;
 }
 
 static void run_edt_x(const uint32_t* mask, uint16_t* vx, int w, int pitch, long long rows, int sms, cudaStream_t st)
