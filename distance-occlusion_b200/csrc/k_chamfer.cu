@@ -17,9 +17,9 @@
 // A CTA walks a run of rows (each row needs the one before); a thread owns 4
 // consecutive cells, so rows of up to 4096 cells.  The previous row stays in
 // registers, its neighbours across threads come by shuffle, across warps from
-// the row's own scan, so a row costs one barrier.  Fields of 16 rows or more
-// run in blocks of 8 rows, all blocks at once (see below); smaller ones, or
-// when the small boundary scratch cannot be had, in one CTA.
+// the row's own scan, so a row costs one barrier.  Fields of more than a few rows
+// (chamfer_block_rows) run in blocks of 8 rows, all blocks at once (see below);
+// smaller ones, or when the small boundary scratch cannot be had, in one CTA.
 #include <limits.h>
 
 #include <type_traits>
@@ -328,13 +328,19 @@ int chamfer_threads(int w)
     return ((t + 31) / 32) * 32;
 }
 
+// Rows from which the blocks are faster than one CTA's walk: their scan costs some
+// 20 - 30 us, a row 0.5 - 3 us by its width (one CTA against blocks, us, int16: 250
+// x 16 19, 33; 250 x 32 33, 41; 1000 x 20 36, 41; 1000 x 24 42, 40; 2000 x 18 45, 47; 2000 x
+// 20 51, 47; 4096 x 16 69, 58; int32 250 x 32 50, 55; 2000 x 18 72, 74)
+static int chamfer_block_rows(int w) { return w <= 512 ? 33 : w <= 1024 ? 24 : w <= 2048 ? 20 : 16; }
+
 template <typename T>
 void launch_chamfer_2d(T* dist, int w, int h, int* err, size_t scratch_cap, cudaStream_t st)
 {
     using K = typename ChamferKey<T>::K;
     const int threads = chamfer_threads(w);
     ProfScope ps("chamfer_2d", st);
-    if (h >= 2 * kChamferBlockRows) {
+    if (h >= chamfer_block_rows(w)) {
         const size_t smem = 3 * (size_t)w * sizeof(K);
         // (always: the static shared memory counts towards the 48 KB that need no asking)
         cudaFuncSetAttribute(k_chamfer_coop<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
