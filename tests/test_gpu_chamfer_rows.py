@@ -7,7 +7,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dtype", ["int16", "int32"])
-@pytest.mark.parametrize("w,rows", [(1, 33), (250, 33), (512, 33), (513, 24), (1024, 24), (1025, 20), (2048, 20), (2049, 16),
+@pytest.mark.parametrize("w,rows", [(2, 33), (250, 33), (512, 33), (513, 24), (1024, 24), (1025, 20), (2048, 20), (2049, 16),
                                     (4096, 16)])
 def test_rows(dol, O, cuda, dtype, w, rows):
     rng = np.random.default_rng(w + rows)
