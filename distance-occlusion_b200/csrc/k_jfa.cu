@@ -167,22 +167,28 @@ __global__ void __launch_bounds__(512) k_jfa3(const void* __restrict__ in, void*
 // values per cell instead of 27.
 constexpr int kJfaChunk = 32;
 
-template <bool kWideIn>
+// kSame: the pass before ran in the same launch (no read-only loads; the grid
+// barrier between them orders plain ones)
+template <bool kWideIn, bool kSame>
 __device__ __forceinline__ C3 jfa_ld(const void* in, long long i)
 {
-    return kWideIn ? load3w(static_cast<const uint2*>(in), i) : load3(static_cast<const int16_t*>(in), i);
+    if (!kSame) return kWideIn ? load3w(static_cast<const uint2*>(in), i) : load3(static_cast<const int16_t*>(in), i);
+    if (kWideIn) {
+        const uint2 u = static_cast<const uint2*>(in)[i];
+        return C3{(int)(int16_t)(u.x & 0xFFFFu), (int)(int16_t)(u.x >> 16), (int)(int16_t)(u.y & 0xFFFFu)};
+    }
+    const int16_t* c = static_cast<const int16_t*>(in) + 3 * i;
+    return C3{c[0], c[1], c[2]};
 }
 
-template <bool kWideIn, bool kWideOut>
-__global__ void __launch_bounds__(512) k_jfa3z(const void* __restrict__ in, void* __restrict__ out, int w, int h, int d,
-                                               int s, int cw, int nchunk)
+template <bool kWideIn, bool kWideOut, bool kSame>
+__device__ __forceinline__ void jfa3z_column(const void* in, void* out, int w, int h, int d, int s, int cw, int run,
+                                             int nchunk, int x, int y, int rc)
 {
-    const int x = blockIdx.x * 32 + (threadIdx.x & 31);
-    const int y = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (x >= w || y >= h) return;
-    const int r = blockIdx.z / nchunk, chunk = blockIdx.z % nchunk;
+    const int r = rc / nchunk, chunk = rc % nchunk;
     const int m = (d - r + s - 1) / s;   // cells r + i s < d
-    const int i0 = chunk * kJfaChunk, i1 = min(m, i0 + kJfaChunk);
+    const int i0 = chunk * run, i1 = min(m, i0 + run);
     if (i0 >= i1) return;
     const long long plane = (long long)w * h;
     const long long col = (long long)y * w + x;
@@ -201,7 +207,7 @@ __global__ void __launch_bounds__(512) k_jfa3z(const void* __restrict__ in, void
     for (int j = i0 - 1; j <= i1; j++) {
         const bool hasA = j - 1 >= i0, hasB = j >= i0 && j < i1, hasC = j + 1 < i1;
         if (hasC) {   // cell j + 1 starts from its own value
-            bC = jfa_ld<kWideIn>(in, (long long)(r + (j + 1) * s) * plane + col);
+            bC = jfa_ld<kWideIn, kSame>(in, (long long)(r + (j + 1) * s) * plane + col);
             lC = len(bC);
         }
         if (j >= 0 && j < m) {   // slice r + j s exists: its 9 neighbours of the column
@@ -213,7 +219,7 @@ __global__ void __launch_bounds__(512) k_jfa3z(const void* __restrict__ in, void
                 for (int ix = -1; ix <= 1; ix++) {
                     const bool vx = ix == 0 || (ix < 0 ? xlo : xhi);
                     if (!(vy && vx)) continue;
-                    const C3 c = jfa_ld<kWideIn>(in, base + (long long)iy * s * w + ix * s);
+                    const C3 c = jfa_ld<kWideIn, kSame>(in, base + (long long)iy * s * w + ix * s);
                     if (c.x == kMax3) continue;
                     const int cx = trunc16(c.x + o * ix), cy = trunc16(c.y + o * iy);
                     if (hasC) consider(bC, lC, C3{cx, cy, trunc16(c.z - o)});
@@ -234,6 +240,14 @@ __global__ void __launch_bounds__(512) k_jfa3z(const void* __restrict__ in, void
         bB = bC;
         lB = lC;
     }
+}
+
+template <bool kWideIn, bool kWideOut>
+__global__ void __launch_bounds__(512) k_jfa3z(const void* __restrict__ in, void* __restrict__ out, int w, int h, int d,
+                                               int s, int cw, int nchunk)
+{
+    jfa3z_column<kWideIn, kWideOut, false>(in, out, w, h, d, s, cw, kJfaChunk, nchunk, blockIdx.x * 32 + (threadIdx.x & 31),
+                                           blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5), blockIdx.z);
 }
 
 // ---- packed 3D passes ---------------------------------------------------------------------
@@ -366,43 +380,28 @@ __global__ void __launch_bounds__(512) k_jfa3p(const uint32_t* __restrict__ in, 
     }
 }
 
-// All passes on the cells as they are, between the caller's array and one buffer
-// (the schedule has an even number of passes), in one cooperative launch, when
-// the conversion found a cell that the packed passes cannot hold.
+// All passes on the cells as they are, in one cooperative launch, when the
+// conversion found a cell that the packed passes cannot hold: the z walk, between
+// the caller's array and one buffer (the schedule has an even number of passes;
+// the second buffer's start holds the flag and the barrier).  256^3 with one such
+// cell: 5.68 ms with a cell per thread and 27 loads, 2.97 now (2.47 as launches of
+// the z walk between two buffers, which only the host could choose); 64^3 0.16 ms,
+// 0.13 (0.22).
 __global__ void __launch_bounds__(256) k_jfa3_general(int16_t* cells, uint2* buf, int w, int h, int d, int cw,
-                                                      JfaSteps st, const int* odd, unsigned* count, int* err)
+                                                      JfaSteps st, int len, const int* odd, unsigned* count, int* err)
 {
     if (!*odd) return;
-    const long long plane = (long long)w * h, n = plane * d;
+    const int tx = (w + 31) / 32, ty = (h + 7) / 8;
     unsigned passed = 0;
     for (int pass = 0; pass < st.n; pass++) {
         const int s = st.s[pass];
-        const bool out = (pass & 1) == 0;   // to the buffer
-        auto ld = [&](long long i) -> C3 {
-            if (out) return C3{__ldcg(cells + 3 * i), __ldcg(cells + 3 * i + 1), __ldcg(cells + 3 * i + 2)};
-            const uint2 u = __ldcg(buf + i);
-            return C3{(int)(int16_t)(u.x & 0xFFFFu), (int)(int16_t)(u.x >> 16), (int)(int16_t)(u.y & 0xFFFFu)};
-        };
-        for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-            const int z = (int)(i / plane), y = (int)((i - z * plane) / w), x = (int)(i - z * plane - (long long)y * w);
-            C3 best = ld(i);
-            int32_t bl = len(best);
-            for (int iz = -1; iz <= 1; iz++)
-                for (int iy = -1; iy <= 1; iy++)
-                    for (int ix = -1; ix <= 1; ix++) {
-                        const int nz = z + iz * s, ny = y + iy * s, nx = x + ix * s;
-                        if (nz < 0 || nz >= d || ny < 0 || ny >= h || nx < 0 || nx >= w) continue;
-                        const C3 c = ld(nz * plane + (long long)ny * w + nx);
-                        if (c.x == kMax3) continue;
-                        const C3 cand = add(c, cw * s * ix, cw * s * iy, cw * s * iz);
-                        const int32_t cl = len(cand);
-                        if (bl > cl) {
-                            best = cand;
-                            bl = cl;
-                        }
-                    }
-            if (out) store3w(buf, i, best);
-            else store3(cells, i, best);
+        const int nchunk = ((d + s - 1) / s + len - 1) / len;
+        const int items = tx * ty * min(s, d) * nchunk;
+        for (int t = blockIdx.x; t < items; t += gridDim.x) {
+            const int rc = t / (tx * ty), tile = t - rc * (tx * ty), by = tile / tx;
+            const int x = (tile - by * tx) * 32 + (threadIdx.x & 31), y = by * 8 + (threadIdx.x >> 5);
+            if (pass & 1) jfa3z_column<true, false, true>(buf, cells, w, h, d, s, cw, len, nchunk, x, y, rc);
+            else jfa3z_column<false, true, true>(cells, buf, w, h, d, s, cw, len, nchunk, x, y, rc);
         }
         if (pass + 1 < st.n && !grid_barrier(count, passed, err)) return;
     }
@@ -499,6 +498,9 @@ static bool run_packed(void* deltas, void* temp, size_t half, int w, int h, int 
             k_jfa3p<false><<<gz, 32 * ry, 0, st>>>(pb[i & 1], pb[(i & 1) ^ 1], w, h, d, sv, cw, len, nchunk, odd);
     }
     if (!checked) {
+        // as `len` above (2 | 4 | 8 | 16 | 32 cells: 64^3 129 | 167 | 225 | 322 | 456 us,
+        // 128^3 622 | 514 | 578 | 562 | 841, 256^3 4048 | 3354 | 3107 | 2974 | 2918)
+        const int glen = cells <= (1 << 19) ? 2 : cells <= (1 << 21) ? 4 : 16;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)min((long long)per_sm * g_num_sms, (long long)(cells + 255) / 256));
         cfg.blockDim = dim3(256);
@@ -509,7 +511,7 @@ static bool run_packed(void* deltas, void* temp, size_t half, int w, int h, int 
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         cudaLaunchKernelEx(&cfg, k_jfa3_general, static_cast<int16_t*>(deltas), static_cast<uint2*>(temp), w, h, d, cw, js,
-                           (const int*)odd, words + 1, err);
+                           glen, (const int*)odd, words + 1, err);
     }
     return true;
 }
