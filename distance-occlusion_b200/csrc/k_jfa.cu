@@ -588,13 +588,64 @@ void launch_jumpflood(int dim, void* deltas, void* temp, int w, int h, int d, in
 
 // ---- deltas -> distances (DistanceOcclusionTool.cpp:46-61, sign :1262/:1392) ----
 
-// A warp takes 256 cells of a row, eight at a time per lane in flight (a division
-// per 256 cells instead of one per cell, and the sign bits of 32 cells are one
-// word).  256^3: 76 us with a flat index and a division per cell, 60 us.
-template <int kDim, bool kHalve>
+// Cells in order, four per thread in flight; a thread finds its first cell's row, for
+// the sign, by a division and steps from there.  Whole calls without | with signs,
+// us: 1501 x 400 x 300 393 | 525 (446 | 694 with a division per cell, 604 | 607 with a
+// warp for 256 cells of a row), 1 x 1000 x 1000 16 | 16 (26 | 25, 179 | 180), 257 x 400
+// x 300 69 | 99 (87 | 131, 171 | 172).
+template <int kDim, bool kHalve, bool kSigned>
 __global__ void __launch_bounds__(256) k_deltas_to_dist(const void* __restrict__ deltas, int cw,
                                                         const uint32_t* __restrict__ sign_mask, float* __restrict__ out,
-                                                        int w, long long items, int segs)
+                                                        int w, long long n)
+{
+    constexpr int kFlight = 4;
+    const int ws = words_per_row(w);
+    const long long threads = (long long)gridDim.x * blockDim.x, first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long row_step = kSigned ? threads / w : 0, row0 = kSigned ? first / w : 0;
+    const int x_step = kSigned ? (int)(threads - row_step * w) : 0;
+    const uint32_t* srow = kSigned ? sign_mask + row0 * ws : nullptr;   // the cell's row of the mask
+    int x = kSigned ? (int)(first - row0 * w) : 0;
+    for (long long i0 = first; i0 < n; i0 += kFlight * threads) {
+        int32_t l[kFlight];
+        uint32_t sign[kFlight];
+#pragma unroll
+        for (int u = 0; u < kFlight; u++) {
+            const long long i = i0 + u * threads;
+            l[u] = 0;
+            sign[u] = 0;
+            if (i < n) {
+                if (kDim == 2) l[u] = len(unpack2(__ldg(static_cast<const uint32_t*>(deltas) + i)));
+                else l[u] = len(load3(static_cast<const int16_t*>(deltas), i));
+                if (kSigned) sign[u] = (__ldg(srow + (x >> 5)) >> (x & 31)) << 31;
+            }
+            if (kSigned) {
+                x += x_step;
+                srow += row_step * ws;
+                if (x >= w) {
+                    x -= w;
+                    srow += ws;
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kFlight; u++) {
+            const long long i = i0 + u * threads;
+            float r = sqrtf((float)l[u]);
+            // half of a square root of an integer is exact: the division by 2 in one multiplication
+            if (kHalve) r = __fmul_rn(r, 0.5f);
+            else if (cw != 1) r = __fdiv_rn(r, (float)cw);
+            if (i < n) out[i] = __uint_as_float(__float_as_uint(r) ^ sign[u]);
+        }
+    }
+}
+
+// Signed images of wide rows: a warp takes 256 cells of a row, eight at a time per
+// lane in flight, the signs of 32 cells being one word (1501 x 4000 13 us, 22 with
+// the cells in order).
+template <bool kHalve>
+__global__ void __launch_bounds__(256) k_deltas_to_dist_rows(const uint32_t* __restrict__ deltas, int cw,
+                                                             const uint32_t* __restrict__ sign_mask,
+                                                             float* __restrict__ out, int w, long long items, int segs)
 {
     const int ws = words_per_row(w), lane = threadIdx.x & 31;
     const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -610,16 +661,14 @@ __global__ void __launch_bounds__(256) k_deltas_to_dist(const void* __restrict__
             l[u] = 0;
             sign[u] = 0;
             if (x0 + x < w) {
-                if (kDim == 2) l[u] = len(unpack2(__ldg(static_cast<const uint32_t*>(deltas) + first + x)));
-                else l[u] = len(load3(static_cast<const int16_t*>(deltas), first + x));
-                if (sign_mask) sign[u] = (__ldg(sign_mask + row * ws + (x0 >> 5) + u) >> lane) << 31;
+                l[u] = len(unpack2(__ldg(deltas + first + x)));
+                sign[u] = (__ldg(sign_mask + row * ws + (x0 >> 5) + u) >> lane) << 31;
             }
         }
 #pragma unroll
         for (int u = 0; u < 8; u++) {
             const int x = 32 * u + lane;
             float r = sqrtf((float)l[u]);
-            // half of a square root of an integer is exact: the division by 2 in one multiplication
             if (kHalve) r = __fmul_rn(r, 0.5f);
             else if (cw != 1) r = __fdiv_rn(r, (float)cw);
             if (x0 + x < w) out[first + x] = __uint_as_float(__float_as_uint(r) ^ sign[u]);
@@ -629,7 +678,7 @@ __global__ void __launch_bounds__(256) k_deltas_to_dist(const void* __restrict__
 
 // The same for volumes of rows of whole fours at 8- and 16-byte aligned arrays: a
 // lane takes four cells as three 8-byte loads and stores them as one float4
-// (256^3: 60 us with 2-byte loads, 35 us).
+// (256^3 with signs: 79 us as above, 35 us).
 template <bool kHalve>
 __global__ void __launch_bounds__(256) k_deltas_to_dist4(const uint2* __restrict__ deltas, int cw,
                                                          const uint32_t* __restrict__ sign_mask,
@@ -663,9 +712,8 @@ __global__ void __launch_bounds__(256) k_deltas_to_dist4(const uint2* __restrict
 void launch_deltas_to_dist(int dim, const void* deltas, int cw, const uint32_t* sign_mask, float* out, int w, int h,
                            int d, cudaStream_t st)
 {
-    const int segs = (w + 255) / 256;
-    const long long items = (long long)h * (dim == 3 ? d : 1) * segs;
-    const long long blocks = (items + 7) / 8, cap = (long long)g_num_sms * 32;
+    const long long n = (long long)w * h * (dim == 3 ? d : 1);
+    const long long blocks = (n + 255) / 256, cap = (long long)g_num_sms * 32;
     const int grid = (int)(blocks < cap ? blocks : cap);
     ProfScope ps("deltas_to_dist", st);
     if (dim == 3 && w % 4 == 0 && ((uintptr_t)deltas & 7) == 0 && ((uintptr_t)out & 15) == 0) {
@@ -677,12 +725,25 @@ void launch_deltas_to_dist(int dim, const void* deltas, int cw, const uint32_t* 
         else k_deltas_to_dist4<false><<<g4, 256, 0, st>>>(in, cw, sign_mask, o, w / 4, n4);
         return;
     }
+    if (dim == 2 && sign_mask && w >= 64) {
+        const int segs = (w + 255) / 256;
+        const long long items = (long long)h * segs, rb = (items + 7) / 8;
+        const int gr = (int)(rb < cap ? rb : cap);
+        const uint32_t* in = static_cast<const uint32_t*>(deltas);
+        if (cw == 2) k_deltas_to_dist_rows<true><<<gr, 256, 0, st>>>(in, cw, sign_mask, out, w, items, segs);
+        else k_deltas_to_dist_rows<false><<<gr, 256, 0, st>>>(in, cw, sign_mask, out, w, items, segs);
+        return;
+    }
+    auto run = [&](auto signed_kern, auto unsigned_kern) {
+        if (sign_mask) signed_kern<<<grid, 256, 0, st>>>(deltas, cw, sign_mask, out, w, n);
+        else unsigned_kern<<<grid, 256, 0, st>>>(deltas, cw, sign_mask, out, w, n);
+    };
     if (dim == 2) {
-        if (cw == 2) k_deltas_to_dist<2, true><<<grid, 256, 0, st>>>(deltas, cw, sign_mask, out, w, items, segs);
-        else k_deltas_to_dist<2, false><<<grid, 256, 0, st>>>(deltas, cw, sign_mask, out, w, items, segs);
+        if (cw == 2) run(k_deltas_to_dist<2, true, true>, k_deltas_to_dist<2, true, false>);
+        else run(k_deltas_to_dist<2, false, true>, k_deltas_to_dist<2, false, false>);
     } else {
-        if (cw == 2) k_deltas_to_dist<3, true><<<grid, 256, 0, st>>>(deltas, cw, sign_mask, out, w, items, segs);
-        else k_deltas_to_dist<3, false><<<grid, 256, 0, st>>>(deltas, cw, sign_mask, out, w, items, segs);
+        if (cw == 2) run(k_deltas_to_dist<3, true, true>, k_deltas_to_dist<3, true, false>);
+        else run(k_deltas_to_dist<3, false, true>, k_deltas_to_dist<3, false, false>);
     }
 }
 
