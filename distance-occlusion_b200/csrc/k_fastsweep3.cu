@@ -594,13 +594,18 @@ bool fastsweep3_by_slices(int w, int h, int d)
     return (h + d - 2.0) * (10.4 + 0.036 * w) < 50.0 * ((w + kTX - 1) / kTX);
 }
 
+// what the columns need, whether or not they are to run
+size_t fastsweep3_columns_most(int w, int h, int d)
+{
+    if (h < 2 || d < 2) return 0;
+    const Fs3Layout l = fs3_layout(w, h, d);
+    return 8 * l.cols > (1 << 28) || l.nch > 65535 ? 0 : l.bytes;
+}
+
 size_t fastsweep3_columns_bytes(int w, int h, int d)
 {
     const int tuned = tune_get(kTuneFs3, w);   // positive: columns, negative: the anti-diagonal wavefront
-    if (h < 2 || d < 2 || tuned < 0 || (tuned == 0 && fastsweep3_by_slices(w, h, d))) return 0;
-    const Fs3Layout l = fs3_layout(w, h, d);
-    if (8 * l.cols > (1 << 28) || l.nch > 65535) return 0;
-    return l.bytes;
+    return tuned < 0 || (tuned == 0 && fastsweep3_by_slices(w, h, d)) ? 0 : fastsweep3_columns_most(w, h, d);
 }
 
 // false: the workspace is too small; nothing has been queued then

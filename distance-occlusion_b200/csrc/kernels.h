@@ -134,6 +134,7 @@ void launch_fastsweep_3d(void* deltas, int w, int h, int d, int cw, void* ws, si
 // or the slices are faster (fastsweep3_by_slices)
 bool fastsweep3_by_slices(int w, int h, int d);
 size_t fastsweep3_columns_bytes(int w, int h, int d);
+size_t fastsweep3_columns_most(int w, int h, int d);
 bool launch_fastsweep_3d_columns(void* deltas, int w, int h, int d, int cw, void* ws, size_t ws_bytes, int* err,
                                  cudaStream_t st);
 

@@ -1,14 +1,15 @@
 // tune.cu -- the launch-configuration table and the autotuner that fills it.
 //
 // Every kernel family here has launch parameters that change speed but never
-// results (all kernels are exact for any of them): cells per thread for the
-// row sweeps (and so threads per row), rows per CTA for the JumpFlood passes,
-// threads per CTA for the EDT line passes, the CTA shape of the batched
-// kernel.  The table maps (family, size bucket = ceil(log2 of the row or line
-// length)) to a value per device; 0 means "not tuned", and launchers then use
-// their built-in heuristic.  dol_autotune measures each candidate on a
-// synthetic problem of the caller's shape (CUDA events, best of two runs) and
-// keeps the fastest; dol_tune_set pins a value by hand.
+// results (all kernels are exact for any of them): cells per lane of the row
+// sweeps, the blocks of Danielsson, the engine of FastSweep 3D, rows per CTA of
+// the JumpFlood passes, threads per CTA of the EDT line passes, the CTA shape of
+// the batched kernel.  The table maps (family, size bucket = ceil(log2 of the row
+// or line length)) to a value per device; 0 means "not tuned", and launchers then
+// use their built-in rules.  dol_autotune measures each candidate on synthetic
+// problems of the caller's shape (CUDA events, best of three runs): the first
+// candidate is what an untuned launch does, and stays unless another is faster by
+// more than kTuneNoise; dol_tune_set pins a value by hand.
 #include <float.h>
 
 #include <algorithm>
@@ -23,6 +24,7 @@ namespace dolk {
 
 constexpr int kTuneDevices = 16;
 constexpr int kTuneBuckets = 16;
+constexpr float kTuneNoise = 0.97f;   // a candidate's time over the best so far, to replace it
 static int g_tune[kTuneDevices][kTuneKinds][kTuneBuckets];
 static std::mutex g_tune_mu;
 
@@ -66,36 +68,32 @@ WaitHooks wait_hooks()
     return g_wait_hooks;
 }
 
-// candidate values per family
-static std::vector<int> candidates(int kind, int w)
+// candidate values per family, the built-in rule first: 0, or the value that means
+// the same (Danielsson and FastSweep 2D 1, FastSweep 3D a positive one where the
+// rule takes the columns, JumpFlood 3D 8, the batch 4, the EDT 512)
+static std::vector<int> candidates(int kind, int w, int h, int d)
 {
     switch (kind) {
         case kTuneDan2:
-        case kTuneFs2:
-        case kTuneDan3: {
-            // CTA engine with 1/2/4/8 cells per thread, or (32) the single-warp engine
-            std::vector<int> c;
-            for (int s : {1, 2, 4, 8})
-                if ((w + s - 1) / s <= 512) c.push_back(s);
-            if (w <= (kind == kTuneDan3 ? 256 : 512)) c.push_back(32);
-            return c;
-        }
+        case kTuneDan3: return {1, 2, 4, 8};   // cells per lane of a block's rows
+        case kTuneFs2: return {1, 4, 8};       // cells per lane
         case kTuneFs3: {   // streaming columns, then the anti-diagonal wavefront (negative)
             std::vector<int> c;
             // (any positive value: the cells per thread of the slices that take over on little scratch)
             for (int most : {128, 256})
                 for (int s : {1, 2, 4, 8})
                     if (c.empty() && (w + s - 1) / s <= most) c.push_back(s);
+            if (fastsweep3_by_slices(w, h, d)) c.insert(c.begin(), 0);
             for (int s : {1, 2, 4, 8})
                 if ((w + s - 1) / s <= 256) c.push_back(-s);
             return c;
         }
-        case kTuneJfa2: return {2, 4, 8, 16};
-        case kTuneJfa3: return {2, 4, 8, 16, -2, -4, -8, -16};   // z walk, then one thread per cell
+        case kTuneJfa2: return {0, 2, 4, 8, 16};   // one launch (up to 2^22 cells), or a launch per pass
+        case kTuneJfa3: return {8, 2, 4, 16, -2, -4, -8, -16};   // z walk, then one thread per cell
         case kTuneBatch: return {4, 8};
-        case kTuneEdt: return {256, 512};
-        case kTuneDanRows: return {4, 8, 16, 32, kDanSerial};
-        case kTuneDanSlices: return {1, 4, 16, 64};
+        case kTuneEdt: return {512, 256};
+        case kTuneDanRows: return {0, 4, 8, 16, kDanSerial};
+        case kTuneDanSlices: return {0, 1, 4, 16, 64};
     }
     return {};
 }
@@ -129,12 +127,12 @@ static dol_status tune_batch(cudaStream_t st)
     cudaEventCreate(&b);
     int best_v = 4;
     float best_t = FLT_MAX;
-    for (int v : candidates(kTuneBatch, 1024)) {
+    for (int v : candidates(kTuneBatch, 1024, 1, 1)) {
         if (s != DOL_OK) break;
         tune_put(kTuneBatch, 1024, v);
         s = dol_batch_run(n, static_cast<uint32_t*>(dm), dd, static_cast<float*>(df), ws, st);
         float t_best = FLT_MAX;
-        for (int rep = 0; rep < 2 && s == DOL_OK; rep++) {
+        for (int rep = 0; rep < 3 && s == DOL_OK; rep++) {
             cudaEventRecord(a, st);
             s = dol_batch_run(n, static_cast<uint32_t*>(dm), dd, static_cast<float*>(df), ws, st);
             cudaEventRecord(b, st);
@@ -143,7 +141,7 @@ static dol_status tune_batch(cudaStream_t st)
             cudaEventElapsedTime(&t, a, b);
             if (t < t_best) t_best = t;
         }
-        if (t_best < best_t) {
+        if (t_best < kTuneNoise * best_t) {
             best_t = t_best;
             best_v = v;
         }
@@ -181,11 +179,9 @@ DOL_API dol_status dol_autotune(int kind, int w, int h, int d, void* stream)
     // a bounded synthetic problem of the caller's row / line shape
     int tw = w, th = h, td = vol ? d : 1;
     if (kind == kTuneFs2) th = h < 256 ? h : 256;
-    if (kind == kTuneFs3) {
-        // both engines are bound by their dependency chains (rows + slices
-        // long) and the slice pipeline by its number of slices, so the ranking
-        // changes with the shape (256 x 64 x 64 ranks 1 cell per thread first,
-        // 256^3 2 cells): the caller's shape up to 2^25 cells, beyond that rows
+    if (kind == kTuneFs3 || kind == kTuneDan3 || ((kind == kTuneDanRows || kind == kTuneDanSlices) && vol)) {
+        // these are bound by their dependency chains, so the ranking changes with
+        // rows and slices: the caller's shape up to 2^25 cells, beyond that rows
         // and slices halved in turn
         while ((long long)tw * th * td > (1LL << 25) && (th > 64 || td > 64)) {
             if (th >= td)
@@ -194,7 +190,6 @@ DOL_API dol_status dol_autotune(int kind, int w, int h, int d, void* stream)
                 td = (td + 1) / 2;
         }
     }
-    if (kind == kTuneDan3) td = d < 32 ? d : 32;   // whole slices: the block schedule's row blocks
     if (kind == kTuneJfa2 && (long long)tw * th > (1LL << 22)) th = (int)((1LL << 22) / tw > 0 ? (1LL << 22) / tw : 1);
     if (kind == kTuneEdt) {
         // the EDT's line kernels are what the value picks, and their cost per
@@ -202,108 +197,111 @@ DOL_API dol_status dol_autotune(int kind, int w, int h, int d, void* stream)
         // (independent column tiles) before shortening the lines
         while ((long long)tw * th * td > (1LL << 26) && tw > 64) tw = ((tw / 2 + 15) / 16) * 16;
     }
-    if (kind == kTuneJfa3 || kind == kTuneEdt || kind == kTuneDanRows || kind == kTuneDanSlices) {
+    if (kind == kTuneJfa3 || kind == kTuneEdt) {
         while ((long long)tw * th * td > (1LL << 26) && td > 1) td = (td + 1) / 2;
     }
     const long long cells = (long long)tw * th * td;
     const size_t mwords = (size_t)((tw + 31) / 32) * th * td;
 
-    // seeds: a sparse LCG scatter (delta methods), solids (FastSweep 3D) or
-    // value noise (EDT)
-    std::vector<uint32_t> hm(mwords, 0u);
-    uint32_t seed = 77;
-    const long long nseeds = cells / 64 + 1;
-    for (long long i = 0; i < nseeds; i++) {
-        seed = lcg_next(seed);
-        int x = lcg_scale(seed, tw);
-        seed = lcg_next(seed);
-        int y = lcg_scale(seed, th);
-        seed = lcg_next(seed);
-        int z = lcg_scale(seed, td);
-        hm[((size_t)z * th + y) * ((tw + 31) / 32) + (x >> 5)] |= 1u << (x & 31);
-    }
     void *dm = nullptr, *dl = nullptr, *tmp = nullptr, *ws = nullptr;
     const size_t cell_bytes = vol ? 6 : 4;
     const bool dan = kind == kTuneDan2 || kind == kTuneDan3 || kind == kTuneDanRows || kind == kTuneDanSlices;
-    size_t ws_bytes = kind == kTuneEdt ? edt_workspace_bytes(3, tw, th, td)
-                      : dan            ? dan_blocks_workspace_bytes(vol ? 3 : 2, tw, th, td, 1)
-                                       : fastsweep3_workspace_bytes(tw, th, td);
-    bool ok = cudaMallocAsync(&dm, mwords * 4, st) == cudaSuccess &&
+    // (sized for every candidate, whatever value is set now)
+    size_t ws_bytes = kind == kTuneEdt   ? edt_workspace_bytes(3, tw, th, td)
+                      : dan              ? dan_blocks_workspace_bytes(vol ? 3 : 2, tw, th, td, 1)
+                      : kind == kTuneFs3 ? std::max(fastsweep3_columns_most(tw, th, td), fastsweep3_workspace_bytes_min(tw, th, td))
+                                         : 0;
+    // an image's cost depends on its content: noise, and points
+    const int contents = vol ? 1 : 2;
+    bool ok = cudaMallocAsync(&dm, contents * mwords * 4, st) == cudaSuccess &&
               cudaMallocAsync(&dl, (size_t)cells * (kind == kTuneEdt ? 4 : cell_bytes), st) == cudaSuccess &&
               cudaMallocAsync(&tmp, jumpflood_workspace_bytes(vol ? 3 : 2, tw, th, td), st) == cudaSuccess &&
-              cudaMallocAsync(&ws, ws_bytes, st) == cudaSuccess;
+              cudaMallocAsync(&ws, ws_bytes + 256, st) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
         for (void* p : {dm, dl, tmp, ws})
             if (p) cudaFreeAsync(p, st);
         return (dol_status)set_error(DOL_ERR_NO_MEMORY, "autotune scratch allocation failed");
     }
+    std::vector<uint32_t> hm(contents > 1 ? mwords : 0, 0u);
     if (kind == kTuneEdt) {
         dol_gen_value_noise_3d(tw, th, td, 16, 3u, static_cast<uint32_t*>(dm), st);
-    } else if (kind == kTuneFs3) {
-        // FastSweep 3D ranks its candidates differently on a scatter of single
-        // seeds (1 cell per thread first) and on solids (2 cells on the 256^3
-        // volume of boxes and spheres): tune it on solids, sized to the volume
+    } else if (vol) {
+        // solids sized to the volume: on a scatter of single seeds candidates rank
+        // differently (FastSweep 3D wavefronts, Danielsson's cells per lane)
         const int m = std::min(tw, std::min(th, td));
         dol_gen_shapes_3d(tw, th, td, 32, 32, std::max(1, 4 * m / 256), std::max(2, 40 * m / 256), 5u,
                           static_cast<uint32_t*>(dm), st);
-    } else
-        cudaMemcpyAsync(dm, hm.data(), mwords * 4, cudaMemcpyHostToDevice, st);
+    } else {
+        dol_gen_value_noise_3d(tw, th, 1, 32, 3u, static_cast<uint32_t*>(dm), st);
+        uint32_t seed = 77;
+        const int points = (int)std::max(8LL, cells / 10000);
+        for (int i = 0; i < points; i++) {
+            seed = lcg_next(seed);
+            const int x = lcg_scale(seed, tw);
+            seed = lcg_next(seed);
+            const int y = lcg_scale(seed, th);
+            hm[(size_t)y * ((tw + 31) / 32) + (x >> 5)] |= 1u << (x & 31);
+        }
+        cudaMemcpyAsync(static_cast<uint32_t*>(dm) + mwords, hm.data(), mwords * 4, cudaMemcpyHostToDevice, st);
+    }
     int* err = nullptr;
     cudaMallocAsync((void**)&err, sizeof(int), st);
 
-    auto run_once = [&]() {
+    auto run_one = [&](const uint32_t* mask) {
         const int dim = vol ? 3 : 2;
         switch (kind) {
             case kTuneDan2:
             case kTuneDan3:   // through the entry path: block schedule or serial engine
-                launch_init_border(dim, static_cast<uint32_t*>(dm), dl, tw, th, td, st);
+                launch_init_border(dim, mask, dl, tw, th, td, st);
                 run_danielsson(dim, dl, tw, th, td, 2, ws, ws_bytes, err, st);
                 break;
             case kTuneFs2:
-                launch_init_border(2, static_cast<uint32_t*>(dm), dl, tw, th, 1, st);
+                launch_init_border(2, mask, dl, tw, th, 1, st);
                 launch_fastsweep_2d(dl, tw, th, 2, st);
                 break;
             case kTuneFs3:
-                launch_init_border(3, static_cast<uint32_t*>(dm), dl, tw, th, td, st);
+                launch_init_border(3, mask, dl, tw, th, td, st);
                 launch_fastsweep_3d(dl, tw, th, td, 2, ws, ws_bytes, err, st);
                 break;
             case kTuneJfa2:
             case kTuneJfa3:
-                launch_init_border(dim, static_cast<uint32_t*>(dm), dl, tw, th, td, st);
+                launch_init_border(dim, mask, dl, tw, th, td, st);
                 launch_jumpflood(dim, dl, tmp, tw, th, td, 2, true, err, st);
                 break;
             case kTuneEdt:
-                launch_edt_mask(3, static_cast<uint32_t*>(dm), static_cast<float*>(dl), tw, th, td, DOL_EDT_SIGNED, ws,
-                                ws_bytes,
-                                err, st);
+                launch_edt_mask(3, mask, static_cast<float*>(dl), tw, th, td, DOL_EDT_SIGNED, ws,
+                                ws_bytes, err, st);
                 break;
             case kTuneDanRows:
             case kTuneDanSlices:
-                launch_init_border(dim, static_cast<uint32_t*>(dm), dl, tw, th, td, st);
+                launch_init_border(dim, mask, dl, tw, th, td, st);
                 run_danielsson(dim, dl, tw, th, td, 2, ws, ws_bytes, err, st);
                 break;
             case kTuneBatch:
                 break;
         }
     };
+    auto run_once = [&]() {
+        for (int c = 0; c < contents; c++) run_one(static_cast<uint32_t*>(dm) + c * mwords);
+    };
 
     cudaEvent_t a, b;
     cudaEventCreate(&a);
     cudaEventCreate(&b);
-    int best_v = 0;
     float best_t = FLT_MAX;
     const int saved = tune_get(kind, w);
+    int best_v = saved;
     // a narrowed synthetic volume looks its value up under its own width:
     // give it each candidate too, and put its entry back afterwards
     const bool other_key = bucket_of(tw) != bucket_of(w);
     const int saved_tw = tune_get(kind, tw);
-    for (int v : candidates(kind, w)) {
+    for (int v : candidates(kind, tw, th, td)) {
         tune_put(kind, w, v);
         if (other_key) tune_put(kind, tw, v);
         run_once();   // warm-up
         float t_best = FLT_MAX;
-        for (int rep = 0; rep < 2; rep++) {
+        for (int rep = 0; rep < 3; rep++) {
             cudaEventRecord(a, st);
             run_once();
             cudaEventRecord(b, st);
@@ -312,12 +310,12 @@ DOL_API dol_status dol_autotune(int kind, int w, int h, int d, void* stream)
             cudaEventElapsedTime(&t, a, b);
             if (t < t_best) t_best = t;
         }
-        if (t_best < best_t) {
+        if (t_best < kTuneNoise * best_t) {
             best_t = t_best;
             best_v = v;
         }
     }
-    tune_put(kind, w, best_v ? best_v : saved);
+    tune_put(kind, w, best_v);
     if (other_key) tune_put(kind, tw, saved_tw);
     cudaEventDestroy(a);
     cudaEventDestroy(b);

@@ -324,14 +324,15 @@ DOL_API dol_status dol_sites_backward(int dim, int w, int h, int d, int n_sites,
    the row sweeps, rows per CTA of the JumpFlood passes, threads per CTA of the
    EDT line passes, the CTA shape of the batched kernel.  They are kept per
    device and per size bucket (ceil(log2(w))); 0 = the built-in heuristic.
-   dol_autotune times every candidate on a synthetic problem of the given shape
-   (blocking; it allocates its own scratch) and keeps the fastest. */
-#define DOL_TUNE_DANIELSSON_2D 0   /* cells per lane of a block's rows: 2, 4, 8 (serial rows: 4, 8); others: by width */
+   dol_autotune times every candidate, the built-in rule among them, on synthetic
+   problems of the given shape (blocking; it allocates its own scratch) and keeps
+   the fastest, the rule unless another is faster by more than 3 %. */
+#define DOL_TUNE_DANIELSSON_2D 0   /* cells per lane of a block's rows: 2, 4, 8 (serial rows: 4, 8); others: the rule */
 #define DOL_TUNE_DANIELSSON_3D 1
-#define DOL_TUNE_FASTSWEEP_2D  2   /* cells per lane: 4, 8; others: by width */
-#define DOL_TUNE_FASTSWEEP_3D  3   /* positive: streaming columns, and 1, 2, 4, 8 cells per thread of the slices
-                                      that run on little scratch; -1, -2, -4, -8: the anti-diagonal wavefront of
-                                      rows */
+#define DOL_TUNE_FASTSWEEP_2D  2   /* cells per lane: 4, 8; others: the rule */
+#define DOL_TUNE_FASTSWEEP_3D  3   /* 0: columns or slices by shape; positive: streaming columns, and 1, 2, 4, 8 cells
+                                      per thread of the slices that run on little scratch; -1, -2, -4, -8: the
+                                      anti-diagonal wavefront of rows */
 #define DOL_TUNE_JUMPFLOOD_2D  4   /* rows per CTA of a launch per pass: 2, 4, 8, 16; 0: up to 2^22 cells one launch */
 #define DOL_TUNE_JUMPFLOOD_3D  5   /* rows per CTA 2, 4, 8, 16 of the z walk; negative: one thread per cell */
 #define DOL_TUNE_BATCH         6   /* 8: 8 warps per CTA; others: 16 */
