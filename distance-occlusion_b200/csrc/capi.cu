@@ -460,7 +460,7 @@ static dol_status danielsson_common(int dim, int w, int h, int d, void* deltas, 
         why = t_err;   // the failed allocation's message
         ws.ptr = nullptr;
     }
-    const bool blocks = run_danielsson(dim, deltas, w, h, dd, cw, ws.ptr, need, ds->err_dev, S(stream));
+    const bool blocks = run_danielsson(dim, deltas, w, h, dd, cw, false, ws.ptr, need, ds->err_dev, S(stream));
     t_engine = blocks ? DOL_ENGINE_BLOCKS : DOL_ENGINE_SERIAL;
     dol_status st = launched(dim == 3 ? "danielsson_3d" : "danielsson_2d");
     if (st == DOL_OK)
@@ -805,8 +805,8 @@ static dol_status sdf_common(int dim, int w, int h, int d, const uint32_t* mask,
     p += align256(cells * cb);
     launch_init_border(dim, mask, dl, w, h, d, st);
     if (method == DOL_DANIELSSON) {
-        run_danielsson(dim, dl, w, h, d, 2, p, danielsson_workspace_bytes(dim, w, h, dim == 3 ? d : 1), ds->err_dev,
-                       st);
+        run_danielsson(dim, dl, w, h, d, 2, true, p, danielsson_workspace_bytes(dim, w, h, dim == 3 ? d : 1),
+                       ds->err_dev, st);
     } else if (method == DOL_FASTSWEEP) {
         if (dim == 2)
             launch_fastsweep_2d(dl, w, h, 2, st);
@@ -890,7 +890,7 @@ static dol_status sdf_two_pass_common(int dim, int w, int h, int d, const uint32
     launch_init_deltas(dim, mask, di, w, rows, 1, st);   // deltas to clear cells
     for (void* dl : {de, di}) {
         if (method == DOL_DANIELSSON) {
-            run_danielsson(dim, dl, w, h, dd, 1, p, danielsson_workspace_bytes(dim, w, h, dd), ds->err_dev, st);
+            run_danielsson(dim, dl, w, h, dd, 1, true, p, danielsson_workspace_bytes(dim, w, h, dd), ds->err_dev, st);
         } else if (method == DOL_FASTSWEEP) {
             if (dim == 2)
                 launch_fastsweep_2d(dl, w, h, 1, st);

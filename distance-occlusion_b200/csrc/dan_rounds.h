@@ -23,4 +23,18 @@ inline int dan_max_rounds(long long nchain, long long h, long long nx)
     return (int)(rows * 4 * nx) + 2;
 }
 
+// Rounds after which the serial walk takes a caller's field over.  A field of
+// seeds settles within about nc + nk + nx rounds (one seed in a corner: 72 of 73 on
+// 1024 x 1024, 501 of 509 on 20 x 20 x 1000); seeds with offsets of part of a cell took
+// up to 172 (of 81, 300 x 200 x 40) and, images, 100 (of 80, 2000 x 500).  Arbitrary
+// components may take as many rounds as the chain is long: 256^3 of components up
+// to 2000 4.9 s, 0.49 with this budget (the walk alone takes 0.3).
+inline int dan_round_budget(int dim, long long nchain, long long h, long long nc, long long nk, long long nx)
+{
+    const long long spread = nc + nk + nx;
+    const long long budget = dim == 3 ? 6 * spread + 64 : spread + spread / 2 + 32;
+    const int most = dan_max_rounds(nchain, h, nx);
+    return budget < most ? (int)budget : most;
+}
+
 }  // namespace dolk

@@ -39,10 +39,11 @@ DOL_DI void x_passes(Cells<DIM, S>& V, int cw, RowShared<NW>& sh, int& par)
 template <int DIM, int S>
 using SerialIO = RowIO<DIM, S, DIM == 3 ? 2 : 1>;
 
-// The whole field; all 32 NW threads of the group call it together.  `strip`:
-// this warp's RowIO strips.
+// The whole field, or one way (0: up, 1: down) through a volume's slices; all 32 NW
+// threads of the group call it together.  `strip`: this warp's RowIO strips.
 template <int DIM, int S, int NW>
-__device__ void dan_serial(void* cells, int w, int h, int d, int cw, unsigned char* strip, RowShared<NW>& sh)
+__device__ void dan_serial(void* cells, int w, int h, int d, int cw, unsigned char* strip, RowShared<NW>& sh,
+                           int way = -1)
 {
     using IO = SerialIO<DIM, S>;
     using Row = Cells<DIM, S>;
@@ -60,8 +61,8 @@ __device__ void dan_serial(void* cells, int w, int h, int d, int cw, unsigned ch
     int par = 0;
     Row P, V;
     constexpr int rc = 0, rq = 1;   // strips: the next row, the row of the slice before
-    const int passes = DIM == 3 ? 2 : 1, first = DIM == 3 ? 1 : 0, last = DIM == 3 ? d : 1;
-    for (int pass = 0; pass < passes; pass++) {
+    const int pass0 = DIM == 3 && way > 0 ? way : 0, pass1 = DIM == 3 && way != 0 ? 2 : 1, first = DIM == 3 ? 1 : 0, last = DIM == 3 ? d : 1;
+    for (int pass = pass0; pass < pass1; pass++) {
         const int dz = pass == 0 ? -cw : cw;
         for (int k = first; k < last; k++) {
             const int z = DIM == 3 ? (pass == 0 ? k : d - 1 - k) : 0;

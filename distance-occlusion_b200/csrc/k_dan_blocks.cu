@@ -64,7 +64,7 @@ struct DanBlk {
     int* stamp;            // many blocks: per block, last round it was queued for
     int* wl[2];            // and the work lists by round parity
     unsigned* ctl;         // by round modulo 3: [0..2] a block changed / work-list size, [3..5] work counter;
-                           // [6] grid barrier, [7] rounds used
+                           // [6] grid barrier, [7] rounds used (0: not done)
     int* err;
     int w, h, d, R, nc, nx, cw;
     int dir;      // +1: slices zfirst, zfirst+1, ...; -1: downwards
@@ -74,6 +74,7 @@ struct DanBlk {
     int nk;       // blocks along the chain: ceil(nchain / Z)
     int nblocks;  // nk * nc * nx, block (k, c, xb) at (k * nc + c) * nx + xb
     int max_rounds;
+    bool rest;    // a field that is not done by then is left to k_dan_rest
 };
 
 // A block's state word: the round it last ran in plus 1, the version that holds
@@ -394,7 +395,7 @@ __global__ void __launch_bounds__(32 * kBlkWarps, 4) k_dan_blocks(DanBlk p)
     for (;; round++) {
         const int cur = round & 1, r3 = round % 3, n3 = (round + 1) % 3;
         if (round >= p.max_rounds) {
-            if (blockIdx.x == 0 && threadIdx.x == 0) atomicExch(p.err, 3);
+            if (!p.rest && blockIdx.x == 0 && threadIdx.x == 0) atomicExch(p.err, 3);
             return;
         }
         const unsigned nwork = own || round == 0 ? (unsigned)p.nblocks : __ldcg(p.ctl + (round + 2) % 3);
@@ -460,6 +461,7 @@ __global__ void k_dan_blocks_init(DanBlk p)
 template <int kCell>
 __global__ void k_dan_blocks_store(DanBlk p, uint16_t* __restrict__ dl, int bx)
 {
+    if (p.ctl[7] == 0) return;   // not done
     const long long row_halves = (long long)p.w * kCell;
     const long long rows = (long long)p.h * p.d;
     for (long long r = blockIdx.x; r < rows; r += gridDim.x) {
@@ -478,6 +480,36 @@ __global__ void k_dan_blocks_store(DanBlk p, uint16_t* __restrict__ dl, int bx)
             for (int i = threadIdx.x; i < row_halves; i += blockDim.x) dst[i] = (state[i / span] >> 2 & 1u ? s1 : s0)[i];
         }
     }
+}
+
+// The phase by the serial walk, on the caller's cells, when its rounds ran out
+template <int DIM, int S, int NW>
+__global__ void __launch_bounds__(32 * NW) k_dan_rest(const unsigned* __restrict__ ctl, void* __restrict__ dl, int w,
+                                                      int h, int d, int cw, int way)
+{
+    extern __shared__ __align__(16) unsigned char strips[];
+    __shared__ RowShared<NW> sh;
+    if (ctl[7] != 0) return;
+    if constexpr (NW > 1) {
+        if (threadIdx.x == 0) sh.bar = 0;
+        __syncthreads();
+    }
+    dan_serial<DIM, S, NW>(dl, w, h, d, cw, strips + (NW > 1 ? threadIdx.x >> 5 : 0) * SerialIO<DIM, S>::kBytes, sh, way);
+}
+
+template <int DIM>
+static void launch_dan_rest(const DanBlk& p, void* dl, cudaStream_t st)
+{
+    auto run = [&](auto kern, int warps, size_t strips) {
+        if (strips > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)strips);
+        kern<<<1, 32 * warps, strips, st>>>(p.ctl, dl, p.w, p.h, p.d, p.cw, p.dir > 0 ? 0 : 1);
+    };
+    if (p.w <= 64) run(k_dan_rest<DIM, 2, 1>, 1, SerialIO<DIM, 2>::kBytes);
+    else if (p.w <= 128) run(k_dan_rest<DIM, 4, 1>, 1, SerialIO<DIM, 4>::kBytes);
+    else if (p.w <= 256) run(k_dan_rest<DIM, 8, 1>, 1, SerialIO<DIM, 8>::kBytes);
+    else if (p.w <= 512) run(k_dan_rest<DIM, 8, 2>, 2, 2 * SerialIO<DIM, 8>::kBytes);
+    else if (p.w <= 1024) run(k_dan_rest<DIM, 8, 4>, 4, 4 * SerialIO<DIM, 8>::kBytes);
+    else run(k_dan_rest<DIM, 8, 8>, 8, 8 * SerialIO<DIM, 8>::kBytes);
 }
 
 static size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
@@ -588,7 +620,7 @@ static bool run_phase(DanBlk& p, void* dl, cudaStream_t st)
     p.Z = Z;
     p.nk = (p.nchain + Z - 1) / Z;
     p.nblocks = p.nk * p.nc * p.nx;
-    p.max_rounds = dan_max_rounds(p.nchain, p.h, p.nx);
+    p.max_rounds = p.rest ? dan_round_budget(kDim, p.nchain, p.h, p.nc, p.nk, p.nx) : dan_max_rounds(p.nchain, p.h, p.nx);
     k_dan_blocks_init<<<min((p.nblocks + 255) / 256, g_num_sms * 8), 256, 0, st>>>(p);
     // a warp per CTA while that spreads the blocks over more SMs
     const int warps = p.nblocks <= 2 * g_num_sms ? 1 : kBlkWarps;
@@ -608,11 +640,12 @@ static bool run_phase(DanBlk& p, void* dl, cudaStream_t st)
     if (gb > (long long)g_num_sms * 32) gb = (long long)g_num_sms * 32;
     k_dan_blocks_store<kDim == 3 ? 3 : 2>
         <<<(int)gb, p.w >= 128 ? 256 : 64, 0, st>>>(p, static_cast<uint16_t*>(dl), 32 * S);
+    if (p.rest) launch_dan_rest<kDim>(p, dl, st);
     return true;
 }
 
 template <int kDim, int S>
-static bool run_all(int w, int h, int d, int cw, int R, void* deltas, void* ws, int* err, cudaStream_t st)
+static bool run_all(int w, int h, int d, int cw, int R, bool initial, void* deltas, void* ws, int* err, cudaStream_t st)
 {
     const DanSizes z = dan_sizes(kDim, w, h, d, R);
     static_assert(8 * sizeof(unsigned) + kWsAlign <= kCtlBytes, "the control words follow the shifted pieces");
@@ -642,6 +675,7 @@ static bool run_all(int w, int h, int d, int cw, int R, void* deltas, void* ws, 
     p.nc = (h + R - 1) / R;
     p.nx = (w + 32 * S - 1) / (32 * S);
     p.cw = cw;
+    p.rest = !initial;
     if (kDim == 2) {
         p.dir = 1;
         p.zfirst = 0;
@@ -666,18 +700,18 @@ size_t danielsson_workspace_bytes(int dim, int w, int h, int d)
     return dan_blocks_workspace_bytes(dim, w, h, d, R);
 }
 
-bool run_danielsson(int dim, void* deltas, int w, int h, int d, int cw, void* ws, size_t ws_bytes, int* err,
-                    cudaStream_t st)
+bool run_danielsson(int dim, void* deltas, int w, int h, int d, int cw, bool initial, void* ws, size_t ws_bytes,
+                    int* err, cudaStream_t st)
 {
     const int R = dan_blocks_rows(dim, w, h, d);
     if (ws && R < kDanSerial && ws_bytes >= dan_blocks_workspace_bytes(dim, w, h, d, R) &&
-        launch_danielsson_blocks(dim, deltas, w, h, d, cw, R, ws, err, st))
+        launch_danielsson_blocks(dim, deltas, w, h, d, cw, R, initial, ws, err, st))
         return true;
     launch_danielsson(dim, deltas, w, h, d, cw, st);
     return false;
 }
 
-bool launch_danielsson_blocks(int dim, void* deltas, int w, int h, int d, int cw, int R, void* ws, int* err,
+bool launch_danielsson_blocks(int dim, void* deltas, int w, int h, int d, int cw, int R, bool initial, void* ws, int* err,
                               cudaStream_t st)
 {
     if (dim == 3 && d < 2) return true;   // the reference's slice loops do not run
@@ -686,14 +720,14 @@ bool launch_danielsson_blocks(int dim, void* deltas, int w, int h, int d, int cw
     ProfScope ps("danielsson_blocks", st);
     switch (dan_blocks_s(dim, w)) {
         case 2:
-            return dim == 2 ? run_all<2, 2>(w, h, 1, cw, R, deltas, ws, err, st)
-                            : run_all<3, 2>(w, h, d, cw, R, deltas, ws, err, st);
+            return dim == 2 ? run_all<2, 2>(w, h, 1, cw, R, initial, deltas, ws, err, st)
+                            : run_all<3, 2>(w, h, d, cw, R, initial, deltas, ws, err, st);
         case 4:
-            return dim == 2 ? run_all<2, 4>(w, h, 1, cw, R, deltas, ws, err, st)
-                            : run_all<3, 4>(w, h, d, cw, R, deltas, ws, err, st);
+            return dim == 2 ? run_all<2, 4>(w, h, 1, cw, R, initial, deltas, ws, err, st)
+                            : run_all<3, 4>(w, h, d, cw, R, initial, deltas, ws, err, st);
         default:
-            return dim == 2 ? run_all<2, 8>(w, h, 1, cw, R, deltas, ws, err, st)
-                            : run_all<3, 8>(w, h, d, cw, R, deltas, ws, err, st);
+            return dim == 2 ? run_all<2, 8>(w, h, 1, cw, R, initial, deltas, ws, err, st)
+                            : run_all<3, 8>(w, h, d, cw, R, initial, deltas, ws, err, st);
     }
 }
 

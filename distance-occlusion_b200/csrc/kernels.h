@@ -110,13 +110,15 @@ void launch_danielsson(int dim, void* deltas, int w, int h, int d, int cw, cudaS
 constexpr int kDanSerial = 65536;   // kTuneDanRows value that selects the serial engine
 int dan_blocks_rows(int dim, int w, int h, int d);
 size_t dan_blocks_workspace_bytes(int dim, int w, int h, int d, int R);
-bool launch_danielsson_blocks(int dim, void* deltas, int w, int h, int d, int cw, int R, void* ws, int* err,
+bool launch_danielsson_blocks(int dim, void* deltas, int w, int h, int d, int cw, int R, bool initial, void* ws, int* err,
                               cudaStream_t st);
 // the Danielsson entry used by the C ABI: the block schedule when its
 // workspace is given and the shape calls for it, else the serial engine
 size_t danielsson_workspace_bytes(int dim, int w, int h, int d);
 // true when the block schedule ran, false for the serial engine
-bool run_danielsson(int dim, void* deltas, int w, int h, int d, int cw, void* ws, size_t ws_bytes, int* err,
+// initial: the deltas come from launch_init_deltas / launch_init_border; a caller's
+// own may need the serial walk after all (dan_rounds.h)
+bool run_danielsson(int dim, void* deltas, int w, int h, int d, int cw, bool initial, void* ws, size_t ws_bytes, int* err,
                     cudaStream_t st);
 void launch_fastsweep_2d(void* deltas, int w, int h, int cw, cudaStream_t st);
 // k_scan.cu -- rows in registers; false: the walk by warps is faster

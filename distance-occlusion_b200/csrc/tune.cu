@@ -254,7 +254,7 @@ DOL_API dol_status dol_autotune(int kind, int w, int h, int d, void* stream)
             case kTuneDan2:
             case kTuneDan3:   // through the entry path: block schedule or serial engine
                 launch_init_border(dim, mask, dl, tw, th, td, st);
-                run_danielsson(dim, dl, tw, th, td, 2, ws, ws_bytes, err, st);
+                run_danielsson(dim, dl, tw, th, td, 2, true, ws, ws_bytes, err, st);
                 break;
             case kTuneFs2:
                 launch_init_border(2, mask, dl, tw, th, 1, st);
@@ -276,7 +276,7 @@ DOL_API dol_status dol_autotune(int kind, int w, int h, int d, void* stream)
             case kTuneDanRows:
             case kTuneDanSlices:
                 launch_init_border(dim, mask, dl, tw, th, td, st);
-                run_danielsson(dim, dl, tw, th, td, 2, ws, ws_bytes, err, st);
+                run_danielsson(dim, dl, tw, th, td, 2, true, ws, ws_bytes, err, st);
                 break;
             case kTuneBatch:
                 break;
