@@ -21,6 +21,7 @@
 #include "dan_scan.cuh"
 #include "dan_serial.cuh"
 #include "dan_slices.cuh"
+#include "diagonals.h"
 #include "kernels.h"
 
 namespace dolk {
@@ -225,7 +226,18 @@ __global__ void __launch_bounds__(256) k_fastsweep3(int16_t* __restrict__ dl, in
     }
 }
 
-// Slice pipeline (the default): a CTA claims a slice kk (in sweep order,
+// diag[c]: the rows of anti-diagonals before c = jj + kk (jj in 1 .. H, kk in 1 .. D),
+// that is, the sum of min(D, c - 1 - jj) over jj in 1 .. min(H, c - 2).  (On the
+// device: a table copied from the host would have to outlive the copy, and a
+// captured graph.)
+__global__ void k_fastsweep3_diagonals(int* __restrict__ diag, int H, int D, int nd)
+{
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= nd) return;
+    diag[c] = rows_before_diagonal(H, D, c);
+}
+
+// Slice pipeline: a CTA claims a slice kk (in sweep order,
 // from an atomic counter) and walks its rows jj = 1 .. H in order, so the
 // row before (y - dy, same slice) is the CTA's own previous result, kept in
 // registers; only the slice before (z - dz, same row) comes from another
@@ -432,25 +444,7 @@ void launch_fastsweep_3d(void* deltas, int w, int h, int d, int cw, void* ws, si
     p += (((size_t)(h + d + 2) * sizeof(int)) + 255) & ~(size_t)255;
     int* counters = reinterpret_cast<int*>(p);   // 8 ints
 
-    // anti-diagonal starts: rows jj in [1, h-1], kk in [1, d-1], c = jj + kk
     const int H = h - 1, Dd = d - 1;
-    static thread_local int* host_diag = nullptr;
-    static thread_local size_t host_diag_n = 0;
-    size_t nd = (size_t)(H + Dd + 2);
-    if (host_diag_n < nd) {
-        if (host_diag) cudaFreeHost(host_diag);
-        cudaMallocHost(&host_diag, nd * sizeof(int));
-        host_diag_n = nd;
-    }
-    long long acc = 0;
-    for (int c = 0; c < (int)nd; c++) {
-        host_diag[c] = (int)acc;
-        if (c >= 2 && c <= H + Dd) {
-            int lo = c - Dd > 1 ? c - Dd : 1, hi = c - 1 < H ? c - 1 : H;
-            if (hi >= lo) acc += hi - lo + 1;
-        }
-    }
-    cudaMemcpyAsync(diag, host_diag, nd * sizeof(int), cudaMemcpyHostToDevice, st);
     cudaMemsetAsync(flags, 0, (size_t)h * d * sizeof(int), st);
     cudaMemsetAsync(counters, 0, 8 * sizeof(int), st);
 
@@ -459,7 +453,11 @@ void launch_fastsweep_3d(void* deltas, int w, int h, int d, int cw, void* ws, si
     // at 256), else at most 256
     int s = tune_get(kTuneFs3, w);
     const bool wavefront = s < 0;   // negative tuned values: the anti-diagonal wavefront with -s cells per thread
-    if (wavefront) s = -s;
+    if (wavefront) {
+        s = -s;
+        const int nd = H + Dd + 2;
+        k_fastsweep3_diagonals<<<(nd + 255) / 256, 256, 0, st>>>(diag, H, Dd, nd);
+    }
     if (!((s == 1 || s == 2 || s == 4 || s == 8) && (w + s - 1) / s <= 256)) {
         s = pick_s(w, 128);
         if (!s) s = pick_s(w, 256);
