@@ -540,8 +540,11 @@ int dan_blocks_rows(int dim, int w, int h, int d)
     if (dim == 2 && ((w <= 256 && h <= 32) || (w <= 128 && h <= 64) || (w <= 64 && h <= 200) || (w <= 32 && h <= 512) ||
                      h < 24))
         return kDanSerial;
-    // 8 rows; tall images of several x blocks 16 (1024^2, 100 points: 0.51
-    // against 0.62 ms; 501 x 700 noise: 0.53 against 0.43); volumes whose
+    // 8 rows; tall images of several x blocks 16.  8 | 16 rows on 1024 columns,
+    // noise of lattice 20, of lattice 51, 100 points, us: 700 high 240 | 286, 394 |
+    // 446, 469 | 414; 1000 high 305 | 291, 410 | 453, 572 | 522; 1600 high 0.88, 0.95, 0.77
+    // of the time (on 300 columns 1.14, 1.0, 0.85): even somewhere between 850 and
+    // 1100 rows, by content.  Volumes whose
     // blocks of 4 rows do not outnumber the resident warps by much 4 (101 x 77
     // x 90: 1.6 against 2.0 ms; 256^3: 9.3 against 8.8)
     if (dim == 2) return w > 256 && h >= 1024 ? 16 : 8;

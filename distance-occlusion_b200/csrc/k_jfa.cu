@@ -678,7 +678,7 @@ __global__ void __launch_bounds__(256) k_deltas_to_dist_rows(const uint32_t* __r
 
 // The same for volumes of rows of whole fours at 8- and 16-byte aligned arrays: a
 // lane takes four cells as three 8-byte loads and stores them as one float4
-// (256^3 with signs: 79 us as above, 35 us).
+// (256^3 with signs: 79 us a cell at a time, 35 us).
 template <bool kHalve>
 __global__ void __launch_bounds__(256) k_deltas_to_dist4(const uint2* __restrict__ deltas, int cw,
                                                          const uint32_t* __restrict__ sign_mask,

@@ -152,7 +152,7 @@ DOL_API dol_status dol_fastsweep_3d(int w, int h, int d, dol_delta3* deltas, int
 /* JumpFlood (DistanceOcclusionLib.cpp:887-908, :2450-2472); the workspace
    stands for the reference's internal ping-pong buffer: one 4-byte cell per
    cell in 2D; in 3D room for two buffers of 8-byte cells, of which sites packed
-   into 4 bytes take half (sides up to about 1000 cells), the caller's 6-byte
+   into 4 bytes take half (sides of up to 599 cells at cw 1, 300 at cw 2), the caller's 6-byte
    cells being read by the first pass and written by the last */
 DOL_API size_t     dol_jumpflood_2d_workspace_size(int w, int h);
 DOL_API size_t     dol_jumpflood_3d_workspace_size(int w, int h, int d);
