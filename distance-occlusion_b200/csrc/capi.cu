@@ -548,7 +548,7 @@ dol_status dol_jumpflood_2d(int w, int h, dol_delta2* deltas, int cw, void* work
     DOL_TRY(check_dev_ptr(deltas, "deltas"));
     Workspace ws;
     DOL_TRY(get_workspace(ws, workspace, workspace_bytes, dol_jumpflood_2d_workspace_size(w, h), S(stream)));
-    launch_jumpflood(2, deltas, ws.ptr, w, h, 1, cw, false, ds->err_dev, S(stream));
+    launch_jumpflood(2, deltas, ws.ptr, w, h, 1, cw, false, ds->err_dev, g_workspace_limit.load(), S(stream));
     return launched("jumpflood_2d");
 }
 
@@ -563,7 +563,7 @@ dol_status dol_jumpflood_3d(int w, int h, int d, dol_delta3* deltas, int cw, voi
     DOL_TRY(check_dev_ptr(deltas, "deltas"));
     Workspace ws;
     DOL_TRY(get_workspace(ws, workspace, workspace_bytes, dol_jumpflood_3d_workspace_size(w, h, d), S(stream)));
-    launch_jumpflood(3, deltas, ws.ptr, w, h, d, cw, false, ds->err_dev, S(stream));
+    launch_jumpflood(3, deltas, ws.ptr, w, h, d, cw, false, ds->err_dev, g_workspace_limit.load(), S(stream));
     return launched("jumpflood_3d");
 }
 
@@ -813,7 +813,7 @@ static dol_status sdf_common(int dim, int w, int h, int d, const uint32_t* mask,
         else
             launch_fastsweep_3d(dl, w, h, d, 2, p, fs3_bytes, ds->err_dev, st);
     } else {
-        launch_jumpflood(dim, dl, p, w, h, d, 2, true, ds->err_dev, st);
+        launch_jumpflood(dim, dl, p, w, h, d, 2, true, ds->err_dev, g_workspace_limit.load(), st);
     }
     if (dist) launch_deltas_to_dist(dim, dl, 2, mask, dist, w, h, d, st);
     return launched("sdf");
@@ -897,7 +897,7 @@ static dol_status sdf_two_pass_common(int dim, int w, int h, int d, const uint32
             else
                 launch_fastsweep_3d(dl, w, h, d, 1, p, fs3_bytes, ds->err_dev, st);
         } else {
-            launch_jumpflood(dim, dl, p, w, h, dd, 1, true, ds->err_dev, st);
+            launch_jumpflood(dim, dl, p, w, h, dd, 1, true, ds->err_dev, g_workspace_limit.load(), st);
         }
     }
     if (dist) launch_two_pass_dist(dim, de, di, dist, (long long)cells, st);

@@ -517,7 +517,7 @@ static bool run_packed(void* deltas, void* temp, size_t half, int w, int h, int 
 }
 
 void launch_jumpflood(int dim, void* deltas, void* temp, int w, int h, int d, int cw, bool initial, int* err,
-                      cudaStream_t st)
+                      size_t scratch_cap, cudaStream_t st)
 {
     int m = w > h ? w : h;
     if (dim == 3 && d > m) m = d;
@@ -535,6 +535,7 @@ void launch_jumpflood(int dim, void* deltas, void* temp, int w, int h, int d, in
         void* a = deltas;
         void* b = temp;
         if (tune_get(kTuneJfa2, w) == 0 && (long long)w * h <= kJfaOneLaunch && np > 1 &&
+            (!scratch_cap || scratch_cap >= sizeof(unsigned)) &&
             jfa2_one_launch(static_cast<uint32_t*>(deltas), static_cast<uint32_t*>(temp), w, h, cw, steps, np, err, st))
             return;
         const dim3 grid((w + 31) / 32, (h + ry - 1) / ry);

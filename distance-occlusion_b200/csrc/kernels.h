@@ -95,8 +95,9 @@ void launch_felz_float_2d(float* dist, int w, int h, void* ws, cudaStream_t st);
 // temp: jumpflood_workspace_bytes (3D: two 8-byte-cell ping-pong buffers)
 size_t jumpflood_workspace_bytes(int dim, int w, int h, int d);
 // initial: the deltas come from launch_init_deltas / launch_init_border (with cw 1 / 2)
+// scratch_cap: of the library's own allocations (0: none)
 void launch_jumpflood(int dim, void* deltas, void* temp, int w, int h, int d, int cw, bool initial, int* err,
-                      cudaStream_t st);
+                      size_t scratch_cap, cudaStream_t st);
 void launch_deltas_to_dist(int dim, const void* deltas, int cw, const uint32_t* sign_mask, float* out, int w, int h,
                            int d, cudaStream_t st);
 void launch_two_pass_dist(int dim, const void* ext, const void* intr, float* out, long long cells, cudaStream_t st);

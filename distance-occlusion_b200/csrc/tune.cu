@@ -267,7 +267,7 @@ DOL_API dol_status dol_autotune(int kind, int w, int h, int d, void* stream)
             case kTuneJfa2:
             case kTuneJfa3:
                 launch_init_border(dim, mask, dl, tw, th, td, st);
-                launch_jumpflood(dim, dl, tmp, tw, th, td, 2, true, err, st);
+                launch_jumpflood(dim, dl, tmp, tw, th, td, 2, true, err, 0, st);
                 break;
             case kTuneEdt:
                 launch_edt_mask(3, mask, static_cast<float*>(dl), tw, th, td, DOL_EDT_SIGNED, ws,

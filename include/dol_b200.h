@@ -84,7 +84,9 @@ DOL_API const char* dol_last_error(void);            /* detail of the last failu
 DOL_API dol_status  dol_sync(void* stream);          /* wait for the stream, report device errors */
 /* Caps the scratch the library allocates by itself (0: no cap, the default);
    process-wide.  Entry points needing more return DOL_ERR_NO_MEMORY, except
-   Danielsson, which then runs its serial engine (see dol_last_engine).
+   Danielsson, which then runs its serial engine (see dol_last_engine), and
+   those with a slower form that needs less or none (FastSweep 3D, the mask EDT
+   of odd widths, Chamfer, occlusion, JumpFlood 2D).
    No reference counterpart. */
 DOL_API void        dol_set_workspace_limit(size_t bytes);
 
