@@ -360,25 +360,25 @@ static int threads_for(int w, int s)
     return ((n + 31) / 32) * 32;
 }
 
-// Cells per lane and warps of a row: 256 cells per warp, fewer per lane for
-// rows that one warp holds with fewer (one for an image's rows of up to 32).
-// Tuning values 4 and 8 set the cells
-// per lane (any other: this rule).
+// Cells per lane and warps of a row: 256 cells per warp, fewer per lane for rows
+// that one warp holds with fewer.  Tuning values 4 and 8 set the cells per lane
+// (any other: this rule).
 static void row_shape(int kind, int w, int* s, int* nw)
 {
     const int tv = tune_get(kind, w);
     *s = tv == 4 || tv == 8 ? tv : (w <= 64 ? 2 : (w <= 128 ? 4 : 8));
     if (*s < 8 && w > 32 * *s * 16) *s = 8;
-    if (w <= 32 && tv != 4 && tv != 8 && kind != kTuneDan3) *s = 1;
+    if (w <= 32 && tv != 4 && tv != 8) *s = 1;
     const int need = (w + 32 * *s - 1) / (32 * *s);
     *nw = 1;
     while (*nw < need) *nw *= 2;
 }
 
-// every shape row_shape gives for images and volumes, up to 4096 cells: f(S, NW);
-// (1, 1) is an image's alone
+// every shape row_shape gives up to 4096 cells, f(S, NW), but for the narrow rows
+// (1, 1) and (2, 1): images' alone, of 32 and 64 cells (Danielsson) and 33 to 64
+// (FastSweep); k_scan.cu has the others
 #define DOL_ROW_SHAPES(f) \
-    f(2, 1) f(4, 1) f(4, 2) f(4, 4) f(4, 8) f(4, 16) f(8, 1) f(8, 2) f(8, 4) f(8, 8) f(8, 16)
+    f(4, 1) f(4, 2) f(4, 4) f(4, 8) f(4, 16) f(8, 1) f(8, 2) f(8, 4) f(8, 8) f(8, 16)
 
 void launch_danielsson(int dim, void* deltas, int w, int h, int d, int cw, cudaStream_t st)
 {
@@ -400,6 +400,7 @@ void launch_danielsson(int dim, void* deltas, int w, int h, int d, int cw, cudaS
     }
     DOL_ROW_SHAPES(DOL_DAN_CASE)
 #undef DOL_DAN_CASE
+    if (s == 2) run(k_dan_serial<2, 2, 1>, 1, SerialIO<2, 2>::kBytes);
     if (s == 1) run(k_dan_serial<2, 1, 1>, 1, SerialIO<2, 1>::kBytes);
 }
 
@@ -414,6 +415,7 @@ void launch_fastsweep_2d(void* deltas, int w, int h, int cw, cudaStream_t st)
     if (s == SV && nw == NWV)  \
         k_fastsweep2<SV, NWV><<<1, 32 * NWV, NWV * SerialIO<2, SV>::kBytes, st>>>(deltas, w, h, cw);
     DOL_ROW_SHAPES(DOL_FS_CASE)
+    DOL_FS_CASE(2, 1)
 #undef DOL_FS_CASE
 }
 
